@@ -105,27 +105,65 @@ __global__ void __launch_bounds__(ROT_COLS * ROT_SLICES) k_rotation_columns(cons
 // of those columns, give the core vorticity (sum of w zeta hz / sum of w hz, FP64 sums in a fixed order), the UH
 // peak of the most rotating one and the strongest anticyclonic one; then the rotation state from the step's keys, the
 // time the rotation has held (unless `refresh`, which keeps it and the model time), and the keys cleared.
-__global__ void k_rotation_summary(const RunDesc* __restrict__ runs, const int4* items, int nitems, int refresh) {
-  __shared__ int roots[256];
-  __shared__ int nroots;
-  __shared__ double red[3][32];
+// Bound by the latency of one block's dependent passes, so only the scan for core columns touches every column: it
+// compacts them (column order; each warp its own stretch, counted and then written) into a list in the run's face
+// potential, free after the step, and the label passes and the component sums walk that list, a component a warp. The
+// first version walked every column in every pass and for every component, one component at a time, with 256 threads:
+// 742 us a step on the 320 x 256 grid, now 55.
+constexpr int SUM_THREADS = 1024, SUM_WARPS = SUM_THREADS / 32;
+__global__ void __launch_bounds__(SUM_THREADS) k_rotation_summary(const RunDesc* __restrict__ runs, const int4* items, int nitems, int refresh) {
+  __shared__ int count[SUM_WARPS + 1];
+  __shared__ double best[SUM_WARPS][3];  // a warp's most rotating component: vorticity, its UH peak; the strongest anticyclonic
+  __shared__ int bestRoot[SUM_WARPS];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED] || !(R.flags & RF_ROTATION)) continue;
-    const int layer = R.layer, nx = R.nx, ny = R.ny, t = threadIdx.x, NT = blockDim.x;
-    const float* coreW = R.diag + DG_COREW * layer;
-    const float* coreWZ = R.diag + DG_COREWZ * layer;
-    const float* col = R.diag + DG_UH * layer;
+    const int layer = R.layer, nx = R.nx, ny = R.ny;
+    const float* __restrict__ coreW = R.diag + DG_COREW * layer;
+    const float* __restrict__ coreWZ = R.diag + DG_COREWZ * layer;
+    const float* __restrict__ col = R.diag + DG_UH * layer;
     int* label = reinterpret_cast<int*>(R.diag + DG_LABEL * layer);
-    int any = 0;
-    for (int c = t; c < layer; c += NT) { const bool core = coreW[c] > 0.f; label[c] = core ? c : -1; any |= core; }
-    const bool hasCores = __syncthreads_or(any);  // (no core column: no labels, no components)
-    // labels only decrease, so the passes end (at most one per column)
-    for (int pass = 0; pass < layer && hasCores && __syncthreads_or(any); pass++) {
-      int changed = 0;
-      for (int c = t; c < layer; c += NT) {
-        const int l0 = label[c];
-        if (l0 < 0) continue;
+    int* list = reinterpret_cast<int*>(R.phi);  // the core columns, then (from list + layer) the roots
+    // Compacts the indices k < m with flag(k) into out in order (value(k) written); returns their count.
+    auto compact = [&](int m, auto flag, auto value, int* out) {
+      const int seg = ((m + SUM_WARPS - 1) / SUM_WARPS + 31) / 32 * 32, k0 = min(m, warp * seg), k1 = min(m, k0 + seg);
+      int mine = 0;
+#pragma unroll 4
+      for (int k = k0 + lane; k < k1; k += 32) mine += flag(k) ? 1 : 0;
+      for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+      __syncthreads();  // (the last compaction's counts are read)
+      if (lane == 0) count[warp] = mine;
+      __syncthreads();
+      if (warp == 0) {  // exclusive prefix over the warps
+        const int own = count[lane];
+        int sum = own;
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+        count[lane] = sum - own;
+        if (lane == 31) count[SUM_WARPS] = sum;
+      }
+      __syncthreads();
+      const int total = count[SUM_WARPS];
+      if (total && mine) {
+        int at = count[warp];
+        for (int k = k0; k < k1; k += 32) {
+          const bool f = k + lane < k1 && flag(k + lane);
+          const unsigned ballot = __ballot_sync(0xffffffffu, f);
+          if (f) out[at + __popc(ballot & ((1u << lane) - 1u))] = value(k + lane);
+          at += __popc(ballot);
+        }
+      }
+      __syncthreads();
+      return total;
+    };
+    const int cores = compact(layer, [&](int c) { const bool core = coreW[c] > 0.f; label[c] = core ? c : -1; return core; },
+                              [](int c) { return c; }, list);
+    // labels only decrease, so the passes end (at most one per core column)
+    int changed = cores > 0;
+    for (int pass = 0; pass < cores && __syncthreads_or(changed); pass++) {
+      changed = 0;
+      for (int k = t; k < cores; k += SUM_THREADS) {
+        const int c = list[k], l0 = label[c];
         int m = min(l0, label[l0]);
         const int x = c % nx, y = c / nx;
         for (int oy = -1; oy <= 1; oy++) {
@@ -137,49 +175,39 @@ __global__ void k_rotation_summary(const RunDesc* __restrict__ runs, const int4*
         }
         if (m < l0) { label[c] = m; changed = 1; }
       }
-      any = changed;
     }
     __syncthreads();
     double coreZeta = 0, coreUH = 0, coreAnti = 0;  // meaningful in thread 0
-    // the components in the order of their smallest columns (the roots), a block of columns at a time: the block's
-    // roots are compacted in column order by warp ballots
-    for (int start = 0; start < layer && hasCores; start += NT) {
-      const int c = start + t;
-      const bool isRoot = c < layer && label[c] == c;
-      const unsigned ballot = __ballot_sync(0xffffffffu, isRoot);
-      if ((t & 31) == 0) red[0][t >> 5] = (double)__popc(ballot);
-      __syncthreads();
-      if (t == 0) {
-        int acc = 0;
-        for (int wi = 0; wi < (NT + 31) / 32; wi++) { const int k = (int)red[0][wi]; red[1][wi] = (double)acc; acc += k; }
-        nroots = acc;
-      }
-      __syncthreads();
-      if (isRoot) roots[(int)red[1][t >> 5] + __popc(ballot & ((1u << (t & 31)) - 1u))] = c;
-      __syncthreads();
-      const int nr = nroots;
-      for (int k = 0; k < nr; k++) {
+    if (cores) {
+      int* roots = list + layer;
+      const int nroots = compact(cores, [&](int k) { return label[list[k]] == list[k]; }, [&](int k) { return list[k]; }, roots);
+      double zeta = 0, uh = 0, anti = 0;
+      int first = 0x7fffffff;
+      for (int k = warp; k < nroots; k += SUM_WARPS) {
         const int r = roots[k];
         double sw = 0, swz = 0, peak = 0;
-        for (int c = t; c < layer; c += NT)
+        for (int j = lane; j < cores; j += 32) {
+          const int c = list[j];
           if (label[c] == r) { sw += coreW[c]; swz += coreWZ[c]; peak = fmax(peak, (double)col[c]); }
+        }
         for (int o = 16; o > 0; o >>= 1) {
           sw += __shfl_xor_sync(0xffffffffu, sw, o);
           swz += __shfl_xor_sync(0xffffffffu, swz, o);
           peak = fmax(peak, __shfl_xor_sync(0xffffffffu, peak, o));
         }
-        if ((t & 31) == 0) { red[0][t >> 5] = sw; red[1][t >> 5] = swz; red[2][t >> 5] = peak; }
-        __syncthreads();
-        if (t == 0) {
-          double a = 0, b = 0, p = 0;
-          for (int wi = 0; wi < (NT + 31) / 32; wi++) { a += red[0][wi]; b += red[1][wi]; p = fmax(p, red[2][wi]); }
-          const double ratio = b / a;
-          if (ratio > coreZeta) { coreZeta = ratio; coreUH = p; }
-          coreAnti = fmax(coreAnti, -ratio);
-        }
-        __syncthreads();
+        const double ratio = swz / sw;
+        if (ratio > zeta) { zeta = ratio; uh = peak; first = k; }
+        anti = fmax(anti, -ratio);
       }
+      if (lane == 0) { best[warp][0] = zeta; best[warp][1] = uh; best[warp][2] = anti; bestRoot[warp] = first; }
       __syncthreads();
+      if (t == 0) {  // the first of the components with the largest vorticity, as the reference's scan keeps it
+        int at = 0x7fffffff;
+        for (int w = 0; w < SUM_WARPS; w++) {
+          if (best[w][0] > coreZeta || (best[w][0] == coreZeta && bestRoot[w] < at)) { coreZeta = best[w][0]; coreUH = best[w][1]; at = bestRoot[w]; }
+          coreAnti = fmax(coreAnti, best[w][2]);
+        }
+      }
     }
     if (t == 0) {
       const unsigned long long kuh = *key(R, K_UH), k01 = *key(R, K_01), kmin = *key(R, K_MIN), k03 = *key(R, K_03);
@@ -258,7 +286,7 @@ void launch_rotation_columns(const Launch& cols, int refresh) {
   if (cols.n) k_rotation_columns<<<GRID(cols.n, cols.cap), ROT_COLS * ROT_SLICES, 0, cols.stream>>>(cols.runs, cols.items, cols.n, refresh);
 }
 void launch_rotation_summary(const Launch& runs, int refresh) {
-  if (runs.n) k_rotation_summary<<<GRID(runs.n, runs.cap), 256, 0, runs.stream>>>(runs.runs, runs.items, runs.n, refresh);
+  if (runs.n) k_rotation_summary<<<GRID(runs.n, runs.cap), SUM_THREADS, 0, runs.stream>>>(runs.runs, runs.items, runs.n, refresh);
 }
 void launch_diag_sample(const Launch& L) { k_diag_sample<<<GRID(L.n, L.cap), 256, 0, L.stream>>>(L.runs, L.items, L.n); }
 

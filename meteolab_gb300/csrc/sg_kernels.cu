@@ -1363,24 +1363,28 @@ __global__ void k_fill_partial(const RunDesc* __restrict__ runs, const int4* ite
     blockSumsDF<NCONS * 3>(hi, lo, R.part + (size_t)chunk * NCONS * 3, sh);
   }
 }
-// Per run: the scale of each conserve field, kept as delta = scale - 1 so a * scale rounds once (fma). Thread k sums
-// field k's block partials (FP64, in chunk order).
-__global__ void k_fill_final(const RunDesc* __restrict__ runs, const int4* items, int nitems) {
+// Per run: the scale of each conserve field, kept as delta = scale - 1 so a * scale rounds once (fma). Warp k sums
+// field k's block partials (FP64; a lane every 32nd chunk in order, then the lanes by halves: a fixed order). One block's
+// chain of loads bounds it: with a thread a field it took 323 us a step on the 320 x 256 x 80 grid (1600 chunks), now 25.
+constexpr int FINAL_THREADS = 32 * 8;
+__global__ void __launch_bounds__(FINAL_THREADS) k_fill_final(const RunDesc* __restrict__ runs, const int4* items, int nitems) {
+  static_assert(NCONS <= FINAL_THREADS / 32, "a warp a field");
   __shared__ double negs[NCONS];
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    const int nch = (R.n + CHUNK - 1) / CHUNK, k = threadIdx.x;
+    const int nch = (R.n + CHUNK - 1) / CHUNK, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (k < NCONS) {
       double removed = 0, kept = 0, negative = 0;
-      for (int c = 0; c < nch; c++) {
+#pragma unroll 4
+      for (int c = lane; c < nch; c += 32) {
         const double* p = R.part + ((size_t)c * NCONS + k) * 3;
         removed += p[0]; kept += p[1]; negative += p[2];
       }
+      removed = warpSum(removed); kept = warpSum(kept); negative = warpSum(negative);
       double delta = 0;
       if (!(removed == 0 && negative == 0)) delta = kept > 0 ? fmax(-1.0, removed / kept) : -1.0;
-      R.scr[S_FILL + k] = (float)delta;
-      negs[k] = negative;
+      if (lane == 0) { R.scr[S_FILL + k] = (float)delta; negs[k] = negative; }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1694,24 +1698,33 @@ __global__ void __launch_bounds__(320, 2) k_mix_tile(const RunDesc* __restrict__
 }
 
 // Per run, once a step: the water budget and negative mass of this step added in a fixed order, the step count,
-// the scratch reset for the next step.
-__global__ void k_step_end(const RunDesc* __restrict__ runs, const int4* items, int nitems) {
+// the scratch reset for the next step. The chunks' partial sums are added by the whole block (a thread every 256th
+// chunk, then blockSums): by one thread, its chain of dependent loads and FP64 additions took 483 us a step on the
+// 320 x 256 x 80 grid (1600 chunks), now 12.
+constexpr int END_THREADS = 256;
+__global__ void __launch_bounds__(END_THREADS) k_step_end(const RunDesc* __restrict__ runs, const int4* items, int nitems) {
+  __shared__ double sh[32 * 5], sums[5];
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
-    if (threadIdx.x == 0 && !R.cnt[C_FAILED]) {
+    const bool live = !R.cnt[C_FAILED], elec = R.flags & RF_ELEC;
+    if (live) {  // (the same for the whole block)
       const size_t nch = (R.n + CHUNK - 1) / CHUNK;
-      double w[3] = {0, 0, 0};
-      for (size_t c = 0; c < nch; c++) for (int j = 0; j < 3; j++) w[j] += R.part[nch * NCONS * 3 + c * 4 + j];
-      for (int j = 0; j < 3; j++) R.acc[A_WATER + j] += w[j];
-      if (R.flags & RF_ELEC) {
-        // the charge separated this step (:1126), and the sedimentation's charge reaching the ground (:590)
-        double sep = 0, ground = 0;
-        for (size_t c = 0; c < nch; c++) sep += R.part[nch * NCONS * 3 + c * 4 + 3];
-        const int sedItems = (R.layer + SED_COLS - 1) / SED_COLS;
-        for (int c = 0; c < sedItems; c++) ground += R.cpart[c];
-        R.acc[A_CHG_SEPARATED] += sep; R.acc[A_CHG_GROUND] += ground; R.acc[A_CHG_PRECIP] += ground;
+      const double* part = R.part + nch * NCONS * 3;
+      double w[5] = {0, 0, 0, 0, 0};  // the water budget's three sums; the charge separated (:1126) and fallen to the ground (:590)
+      for (size_t c = threadIdx.x; c < nch; c += END_THREADS) {
+        w[0] += part[c * 4]; w[1] += part[c * 4 + 1]; w[2] += part[c * 4 + 2];
+        if (elec) w[3] += part[c * 4 + 3];
       }
-      R.cnt[C_STEPS] += 1;
+      if (elec) {
+        const int sedItems = (R.layer + SED_COLS - 1) / SED_COLS;
+        for (int c = threadIdx.x; c < sedItems; c += END_THREADS) w[4] += R.cpart[c];
+      }
+      blockSums<5>(w, sums, sh);
+      if (threadIdx.x == 0) {
+        for (int j = 0; j < 3; j++) R.acc[A_WATER + j] += sums[j];
+        if (elec) { R.acc[A_CHG_SEPARATED] += sums[3]; R.acc[A_CHG_GROUND] += sums[4]; R.acc[A_CHG_PRECIP] += sums[4]; }
+        R.cnt[C_STEPS] += 1;
+      }
     }
     __syncthreads();
     if (threadIdx.x < S_COUNT + 16) R.scr[threadIdx.x] = 0.f;
@@ -1825,7 +1838,7 @@ void launch_pres_correct(const Launch& L, int set, int final_) {
 }
 
 void launch_fill_partial(const Launch& L, int set) { k_fill_partial<<<GRID(L.n, L.cap), 128, 0, L.stream>>>(L.runs, L.items, L.n, set); }
-void launch_fill_final(const Launch& L) { k_fill_final<<<GRID(L.n, L.cap), 32, 0, L.stream>>>(L.runs, L.items, L.n); }
+void launch_fill_final(const Launch& L) { k_fill_final<<<GRID(L.n, L.cap), FINAL_THREADS, 0, L.stream>>>(L.runs, L.items, L.n); }
 void launch_sediment_2m(const Launch& L, int maxnz) {
   const int K = (maxnz + 31) / 32;  // level slots a lane (nz <= 128)
   if (K <= 1) k_sediment_2m<1><<<GRID(L.n, L.cap), SED2_WARPS * 32, 0, L.stream>>>(L.runs, L.items, L.n);
@@ -1849,7 +1862,7 @@ size_t mix_smem(int TX, int TY) { return (size_t)2 * (NMIX + 1) * (TX + 2) * (TY
 void launch_mix(const Launch& L, int in, int TX, int TY) {
   k_mix_tile<<<GRID(L.n, L.cap), TX * TY, mix_smem(TX, TY), L.stream>>>(L.runs, L.items, L.n, in, TX, TY);
 }
-void launch_step_end(const Launch& L) { k_step_end<<<GRID(L.n, L.cap), 64, 0, L.stream>>>(L.runs, L.items, L.n); }
+void launch_step_end(const Launch& L) { k_step_end<<<GRID(L.n, L.cap), END_THREADS, 0, L.stream>>>(L.runs, L.items, L.n); }
 void launch_divergence_max(const Launch& L, int set, double* out) { k_divergence_max<<<GRID(L.n, L.cap), 256, 0, L.stream>>>(L.runs, L.items, L.n, set, out); }
 
 // The constant tables the kernels read that are made on the host: the Seifert-Beheng sweep coefficients of two-moment
