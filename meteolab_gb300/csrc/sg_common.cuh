@@ -76,6 +76,7 @@ struct RunDesc {
   int nx, ny, nz, layer, n, nm, mh, ncells;
   int fx_nf, fy_nf, fx_rad[8], fy_rad[8];  // FFT radix plans of nx and ny
   int slot, flags, nf, breakup;  // nf: the run's field ids (NF, or NFE with the extra fields); breakup: two-moment rain's
+  int chunk, pad1;               // nodes per summed chunk
   float dx, dy, inv_dx, inv_dy, dt, height;
   float inv_dx_lo, inv_dy_lo, inv_dt, inv_dt_lo;      // FP32 rounding errors of 1/dx, 1/dy; 1/dt as a pair
   float coriolis, keep, sponge_start, cs, drag, frame_u, frame_v, ue0, ve0, env_speed, lenH2, capH, rho0;
@@ -95,7 +96,7 @@ struct RunDesc {
   const float2* twx;       // exp(-2 pi i t / nx), t < nx
   const float2* twy;       // exp(-2 pi i t / ny)
   float* scr;              // per-step scratch: courant[4], fill delta[7], ...
-  double* part;            // FP64 partial sums (positivity fix, water budget)
+  double* part;            // FP64 partial sums per chunk (water budget; the positivity fix's are in kmkh, see fill_part)
   double* acc;             // FP64 running totals: negativeFilled, water[4]
   unsigned long long* cnt; // counters: clipped, steps, failed flag
   // per-run diagnostics (RF_ROTATION): columns [DG_COUNT][layer] and the rotation state and accumulators
@@ -137,9 +138,25 @@ enum Counter { C_CLIPPED = 0, C_STEPS = 1, C_FAILED = 2, C_TIMEOUT = 3, C_COUNT 
 // A_CHG_*: the charge budget (AtmosphereModel.chargeGround and .charge, src/core/model.ts:218-224), C; A_FLASH_*: counts
 enum Acc { A_NEG = 0, A_WATER = 1, A_CHG_GROUND = 8, A_CHG_SEPARATED, A_CHG_IC, A_CHG_CG_NEG, A_CHG_CG_POS, A_CHG_PRECIP, A_CHG_CONDUCTION,
            A_FLASH_IC, A_FLASH_CG, A_COUNT = 24 };
-// partial-sum layout (per run): fill partials [chunk][7][3], then water partials [chunk][4].
-constexpr int CHUNK = 4096;   // nodes per pointwise work item
+// partial-sum layout (per run): water partials [chunk][4] in part; fill partials [chunk][7][3] in the viscosities' memory
+// (they live between the end of the dynamics and the physics, the viscosities from the physics to the mixing).
+constexpr int CHUNK = 4096;   // nodes per packed-transfer item, and at most per pointwise one
+// Nodes per summed chunk of a run of n nodes (RunDesc.chunk: the items of the positivity fix and the physics, whose
+// partial sums are per chunk). A function of the run alone, so that a run's bits do not depend on its batch. Small runs
+// take small chunks, or one of them alone keeps few SMs busy: a standard run's physics takes 90 us in 16 chunks of 4096,
+// 33 in 63 of 1024 and 23 in 125 of 512, its sums 31, 14 and 10; on the 64-run batch the physics takes 381, 344 and 352
+// us, the sums 70, 72 and 88 (a block's sums cost it as much as four nodes a thread).
+SG_HD int chunk_nodes(size_t n) { return n <= (1u << 20) ? 1024 : CHUNK; }
+// Nodes per item of the pointwise kernels without sums (node items: slot, first node, end), free to follow the batch:
+// the largest power of two that still gives `blocks` items, within 512..4096. A single standard run's step (658 us) is
+// 125 us faster with 512-node items than with 4096; the 64-run batch's corrections are 15% faster with 2048 than 1024.
+inline int node_chunk(size_t nodes, size_t blocks) {
+  int c = CHUNK;
+  while (c > 512 && nodes / c < blocks) c /= 2;
+  return c;
+}
 
+SG_HD double* fill_part(const RunDesc& R) { return reinterpret_cast<double*>(R.kmkh); }
 SG_HD float lvl(const RunDesc& R, int which, int z) { return R.lv[which * R.nz + z]; }
 // Set s of the 13 base fields is fld[s * 13 n ...]; an electrified run's charge carriers follow the three sets,
 // four fields a set, so the base fields keep their offsets (and the hot kernels their constant strides).

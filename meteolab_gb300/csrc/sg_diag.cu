@@ -239,7 +239,7 @@ __global__ void k_diag_sample(const RunDesc* __restrict__ runs, const int4* item
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (!(R.flags & RF_ROTATION)) continue;
-    const int layer = R.layer, i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int layer = R.layer, i0 = items[it].y, i1 = items[it].z;
     const float* __restrict__ w = field(R, 0, W);
     const float* __restrict__ cl = field(R, 0, CLOUD);
     const float* __restrict__ ic = field(R, 0, ICE);

@@ -134,7 +134,7 @@ __device__ void blockSumsDF(float (&hi)[COUNT], float (&lo)[COUNT], double* out,
 __global__ void k_theta_in(const RunDesc* __restrict__ runs, const int4* items, int nitems, const float* src) {
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
-    int i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int i0 = items[it].y, i1 = items[it].z;
     float* th = field(R, 0, THETA);
     const float* s = src ? src : field(R, 1, THETA);  // null: each run's own staging slot (set B)
     for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) th[i] = (float)((double)s[i] - R.lv64[D_THB * R.nz + i / R.layer]);
@@ -143,7 +143,7 @@ __global__ void k_theta_in(const RunDesc* __restrict__ runs, const int4* items, 
 __global__ void k_theta_out(const RunDesc* __restrict__ runs, const int4* items, int nitems, float* dst) {
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
-    int i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int i0 = items[it].y, i1 = items[it].z;
     const float* th = field(R, 0, THETA);
     float* d = dst ? dst : field(R, 1, THETA);
     for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) d[i] = (float)((double)th[i] + R.lv64[D_THB * R.nz + i / R.layer]);
@@ -157,7 +157,7 @@ __global__ void k_fall_courant(const RunDesc* __restrict__ runs, const int4* ite
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    int i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int i0 = items[it].y, i1 = items[it].z;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
     const float *rain = field(R, 0, RAIN), *snow = field(R, 0, SNOW), *graupel = field(R, 0, GRAUPEL), *hail = field(R, 0, HAIL);
     for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
@@ -1006,7 +1006,7 @@ __global__ void k_face_correct(const RunDesc* __restrict__ runs, const int4* ite
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    const int nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer, i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer, i0 = items[it].y, i1 = items[it].z;
     const float* __restrict__ u = field(R, set, U);
     const float* __restrict__ v = field(R, set, V);
     const float* __restrict__ w = field(R, set, W);
@@ -1063,7 +1063,7 @@ __global__ void k_pres_correct(const RunDesc* __restrict__ runs, const int4* ite
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
     if (final_ && (bool)(R.flags & RF_REFINE) != two) continue;
-    const int nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer, i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer, i0 = items[it].y, i1 = items[it].z;
     float *u = field(R, set, U), *v = field(R, set, V), *w = field(R, set, W);
     const float* __restrict__ p = R.pres;
     const float* __restrict__ p2 = R.pres2;
@@ -1322,7 +1322,7 @@ __global__ void k_fill_partial(const RunDesc* __restrict__ runs, const int4* ite
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    const int chunk = items[it].y, i0 = chunk * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int chunk = items[it].y, i0 = chunk * R.chunk, i1 = min(R.n, i0 + R.chunk);
     // per conserve field: removed (the tiny values the fix zeroes), kept (the rest), negative (-sum of the negatives)
     float hi[NCONS * 3], lo[NCONS * 3];
 #pragma unroll
@@ -1360,7 +1360,7 @@ __global__ void k_fill_partial(const RunDesc* __restrict__ runs, const int4* ite
         }
       }
     }
-    blockSumsDF<NCONS * 3>(hi, lo, R.part + (size_t)chunk * NCONS * 3, sh);
+    blockSumsDF<NCONS * 3>(hi, lo, fill_part(R) + (size_t)chunk * NCONS * 3, sh);
   }
 }
 // Per run: the scale of each conserve field, kept as delta = scale - 1 so a * scale rounds once (fma). Warp k sums
@@ -1373,12 +1373,12 @@ __global__ void __launch_bounds__(FINAL_THREADS) k_fill_final(const RunDesc* __r
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    const int nch = (R.n + CHUNK - 1) / CHUNK, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nch = (R.n + R.chunk - 1) / R.chunk, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (k < NCONS) {
       double removed = 0, kept = 0, negative = 0;
 #pragma unroll 4
       for (int c = lane; c < nch; c += 32) {
-        const double* p = R.part + ((size_t)c * NCONS + k) * 3;
+        const double* p = fill_part(R) + ((size_t)c * NCONS + k) * 3;
         removed += p[0]; kept += p[1]; negative += p[2];
       }
       removed = warpSum(removed); kept = warpSum(kept); negative = warpSum(negative);
@@ -1408,7 +1408,7 @@ __global__ void __launch_bounds__(256, (ELEC || MOM == 3) ? 2 : 3) k_physics(con
   __shared__ double sh[32 * 4];
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
-    const int chunk = items[it].y, i0 = chunk * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int chunk = items[it].y, i0 = chunk * R.chunk, i1 = min(R.n, i0 + R.chunk);
     const float dt = R.dt, keepCold = __powf(.9992f, dt);
     float fill[NCONS];
 #pragma unroll
@@ -1501,8 +1501,7 @@ __global__ void __launch_bounds__(256, (ELEC || MOM == 3) ? 2 : 3) k_physics(con
       }
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicExch(&R.cnt[C_FAILED], 1ull);
-    size_t nch = (R.n + CHUNK - 1) / CHUNK;
-    blockSumsDF<NW>(whi, wlo, R.part + nch * NCONS * 3 + (size_t)chunk * 4, sh);
+    blockSumsDF<NW>(whi, wlo, R.part + (size_t)chunk * 4, sh);
   }
 }
 
@@ -1513,7 +1512,7 @@ __global__ void k_viscosity(const RunDesc* __restrict__ runs, const int4* items,
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    const int nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer, i0 = items[it].y * CHUNK, i1 = min(R.n, i0 + CHUNK);
+    const int nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer, i0 = items[it].y, i1 = items[it].z;
     const float* __restrict__ u = field(R, set, U);
     const float* __restrict__ v = field(R, set, V);
     const float* __restrict__ w = field(R, set, W);
@@ -1708,8 +1707,8 @@ __global__ void __launch_bounds__(END_THREADS) k_step_end(const RunDesc* __restr
     const RunDesc& R = runs[items[it].x];
     const bool live = !R.cnt[C_FAILED], elec = R.flags & RF_ELEC;
     if (live) {  // (the same for the whole block)
-      const size_t nch = (R.n + CHUNK - 1) / CHUNK;
-      const double* part = R.part + nch * NCONS * 3;
+      const size_t nch = (R.n + R.chunk - 1) / R.chunk;
+      const double* part = R.part;
       double w[5] = {0, 0, 0, 0, 0};  // the water budget's three sums; the charge separated (:1126) and fallen to the ground (:590)
       for (size_t c = threadIdx.x; c < nch; c += END_THREADS) {
         w[0] += part[c * 4]; w[1] += part[c * 4 + 1]; w[2] += part[c * 4 + 2];
@@ -1736,7 +1735,7 @@ __global__ void __launch_bounds__(END_THREADS) k_step_end(const RunDesc* __restr
 __global__ void k_divergence_max(const RunDesc* __restrict__ runs, const int4* items, int nitems, int set, double* out) {
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
-    const int nx = R.nx, ny = R.ny, layer = R.layer, i0 = items[it].y * CHUNK, i1 = min(R.ncells, i0 + CHUNK);
+    const int nx = R.nx, ny = R.ny, layer = R.layer, i0 = items[it].y, i1 = items[it].z;
     const float *u = field(R, set, U), *v = field(R, set, V), *w = field(R, set, W);
     double m = 0;
     for (int cidx = i0 + threadIdx.x; cidx < i1; cidx += blockDim.x) {

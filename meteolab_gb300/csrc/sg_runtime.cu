@@ -41,15 +41,15 @@ struct Layout {
 // fall speeds and the vertical field after the rest, an electrified one also the lightning's buffers (sg_lightning.cu).
 Layout layout(int nx, int ny, int nz, int flags = 0) {
   const bool extra = flags & RF_EXTRA, elec = flags & RF_ELEC;
-  Layout L; size_t n = (size_t)nx * ny * nz, layer = (size_t)nx * ny, nm = nx / 2 + 1, nch = (n + CHUNK - 1) / CHUNK, o = 0;
+  Layout L; size_t n = (size_t)nx * ny * nz, layer = (size_t)nx * ny, nm = nx / 2 + 1, nch = (n + chunk_nodes(n) - 1) / chunk_nodes(n), o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += align(bytes); return at; };
-  L.fld = take(3 * (size_t)(extra ? NFE : NF) * n * 4); L.faces = take(4 * n * 4); L.kmkh = take(2 * n * 4); L.phi = take(n * 4);
+  L.fld = take(3 * (size_t)(extra ? NFE : NF) * n * 4); L.faces = take(4 * n * 4); L.kmkh = take(std::max(2 * n * 4, nch * NCONS * 3 * 8)); L.phi = take(n * 4);
   L.pres = take(layer * (nz - 1) * 4); L.pres2 = take(layer * (nz - 1) * 4); L.spec = take(nm * nz * ny * 8); L.cols = take(3 * layer * 4);
   L.lv = take((size_t)L_COUNT * nz * 4); L.lv64 = take((size_t)D_COUNT * nz * 8);
   L.triF = take(nm * nz * ny * 24); L.triP = take(nm * (nz - 1) * ny * 24); L.ab = take(nm * ny * 16);
-  L.twx = take(nx * 8); L.twy = take(ny * 8); L.scr = take(64 * 4); L.part = take((nch * NCONS * 3 + nch * 4) * 8);
+  L.twx = take(nx * 8); L.twy = take(ny * 8); L.scr = take(64 * 4); L.part = take(nch * 4 * 8);
   L.acc = take(A_COUNT * 8); L.cnt = take(C_COUNT * 8);
-  L.items = take(nch * 16);  // the run's own per-node work items (field conversions outside a batch plan)
+  L.items = take((n + CHUNK - 1) / CHUNK * 16);  // the run's own per-node work items (field conversions outside a batch plan)
   L.diag = take((size_t)DG_COUNT * layer * 4); L.rot = take(R_COUNT * 8);
   if (extra) { L.vfall = take(((flags & RF_ICE2M) ? 12 : 6) * n * 4); L.ez = take(n * 4); L.cpart = take(((layer + 63) / 64) * 8); }
   if (elec) L.lgt = take(lightning_bytes(nx, ny, nz));
@@ -106,7 +106,7 @@ struct Plan {
   }
 };
 enum Family { FAM_NODE, FAM_COLS, FAM_ROWS_FACE, FAM_ROWS_PRES, FAM_MODES, FAM_RUNS, FAM_CELLS, FAM_T_WENO, FAM_T_DYN, FAM_MIX,
-              FAM_REFINE, FAM_T_CHG, FAM_T_CHG3, FAM_PHYS, FAM_PHYS_LAST = FAM_PHYS + 5, FAM_LROWS_FACE, FAM_LROWS_PRES, FAM_LMODES, FAM_COUNT };
+              FAM_REFINE, FAM_T_CHG, FAM_T_CHG3, FAM_PHYS, FAM_PHYS_LAST = FAM_PHYS + 5, FAM_FILL, FAM_LROWS_FACE, FAM_LROWS_PRES, FAM_LMODES, FAM_COUNT };
 
 }  // namespace
 
@@ -417,14 +417,17 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, Plan& P) {
     else { P.rowAny = true; P.rowMaxnx = std::max(P.rowMaxnx, r.nx); P.rowMaxny = std::max(P.rowMaxny, r.ny); }
   }
   P.yc = P.rowAny ? std::min(P.rowMaxnx > 128 ? 16 : 32, (P.rowMaxny + 1) / 2 * 2) : 32;
+  size_t nodes = 0;
+  for (int s : slots) nodes += (size_t)ctx->runs[s].desc.n;
+  const int step = node_chunk(nodes, (size_t)ctx->sms * 8);
   for (int s : slots) {
     const Run& r = ctx->runs[s];
-    int n = r.nx * r.ny * r.nz, nch = (n + CHUNK - 1) / CHUNK, layer = r.nx * r.ny;
-    for (int c = 0; c < nch; c++) all[FAM_NODE].push_back(make_int4(s, c, 0, 0));
+    int n = r.nx * r.ny * r.nz, chunk = r.desc.chunk, nch = (n + chunk - 1) / chunk, layer = r.nx * r.ny, cells = layer * (r.nz - 1);
+    for (int i = 0; i < n; i += step) all[FAM_NODE].push_back(make_int4(s, i, std::min(n, i + step), 0));
     // the physics' node chunks by kernel variant: a run takes the same physics code whatever batch it is in
     for (int c = 0; c < nch; c++) all[FAM_PHYS + physics_variant(r.desc.flags)].push_back(make_int4(s, c, 0, 0));
-    int ncc = (r.nx * r.ny * (r.nz - 1) + CHUNK - 1) / CHUNK;
-    for (int c = 0; c < ncc; c++) all[FAM_CELLS].push_back(make_int4(s, c, 0, 0));
+    for (int c = 0; c < nch; c++) all[FAM_FILL].push_back(make_int4(s, c, 0, 0));
+    for (int i = 0; i < cells; i += step) all[FAM_CELLS].push_back(make_int4(s, i, std::min(cells, i + step), 0));
     for (int c = 0; c < (layer + 63) / 64; c++) all[FAM_COLS].push_back(make_int4(s, c, 0, 0));
     if (layerPath(r)) {  // a layer an item
       for (int k = 0; k < r.nz; k++) all[FAM_LROWS_FACE].push_back(make_int4(s, k, 0, 0));
@@ -641,7 +644,7 @@ void enqueue_part(sg_context* ctx, const Plan& P, int part, Hook hook) {
       if (s < 2) enqueue_project(ctx, P, out[s], 0, st, hook);
     }
   } else if (part == 3) {
-    launch_fill_partial(node, B); hook(11);
+    launch_fill_partial(lx(ctx, P, FAM_FILL), B); hook(11);
     launch_fill_final(runs); hook(12);
     for (int v = 0; v < 6; v++) launch_physics(lx(ctx, P, FAM_PHYS + v), B, C, v);
     hook(13);
@@ -955,6 +958,7 @@ int sg_run_create(sg_context* ctx, const sg_grid* g, const sg_base_state* b, con
   HostTables T; RunDesc& d = r.desc; d = RunDesc{};
   build_tables(g, b, sw, T, d);
   d.slot = slot;
+  d.chunk = chunk_nodes((size_t)d.n);
   d.nf = elec || two ? NFE : NF;
   d.flags |= xflags;
   d.breakup = sw->rain_breakup;
@@ -991,7 +995,7 @@ int sg_run_create(sg_context* ctx, const sg_grid* g, const sg_base_state* b, con
     const size_t n = (size_t)g->nx * g->ny * g->nz;
     r.nNode = (int)((n + CHUNK - 1) / CHUNK);
     std::vector<int4> items(r.nNode);
-    for (int c = 0; c < r.nNode; c++) items[c] = make_int4(slot, c, 0, 0);
+    for (int c = 0; c < r.nNode; c++) items[c] = make_int4(slot, c * CHUNK, std::min(d.n, (c + 1) * CHUNK), 0);
     r.nodeItems = (int4*)(mem + Lo.items);
     CK(H2D(Lo.items, items.data(), items.size() * sizeof(int4)));
   }
