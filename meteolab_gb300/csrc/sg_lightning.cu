@@ -434,12 +434,13 @@ inline int blocks(int n, int t) { return (n + t - 1) / t; }
 size_t lightning_bytes(int nx, int ny, int nz) {
   const size_t n = (size_t)nx * ny * nz, mh = nx / 2, spec = (size_t)(nz - 2) * (mh + 1) * ny;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  return al(sizeof(LgtState)) + 6 * al(n * 8) + al(n * 4) + 5 * al(n * 4) + 4 * al((size_t)MAX_CHANNEL * 8) +
-         al((size_t)LT_COUNT * nz * 8) + al(((n + 255) / 256 + 1) * 8) + 2 * al(spec * 16) + 2 * al(spec * 8) + al((size_t)nz * 8) +
+  return al(sizeof(LgtState)) + 5 * al(n * 8) + al(n * 4) + 5 * al(n * 4) + 4 * al((size_t)MAX_CHANNEL * 8) +
+         al((size_t)LT_COUNT * nz * 8) + al(((n + 255) / 256 + 1) * 8) + al(spec * 16) + 3 * al(spec * 8) +
          al((size_t)nx * 16) + al((size_t)ny * 16);
 }
 
-void lightning_bind(char* base, int nx, int ny, int nz, LgtDev& L) {
+void lightning_bind(char* base, int nx, int ny, int nz, LgtHost& H) {
+  LgtDev& L = H.dev;
   const size_t n = (size_t)nx * ny * nz, mh = nx / 2, spec = (size_t)(nz - 2) * (mh + 1) * ny;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
   size_t o = 0;
@@ -447,17 +448,17 @@ void lightning_bind(char* base, int nx, int ny, int nz, LgtDev& L) {
   L.nz = nz;
   L.st = (LgtState*)take(sizeof(LgtState));
   L.rho = (double*)take(n * 8); L.phi = (double*)take(n * 8); L.sigma = (double*)take(n * 8);
-  L.weight = (double*)take(n * 8); L.scale = (double*)take(n * 8); double* spare = (double*)take(n * 8); (void)spare;
+  L.weight = (double*)take(n * 8); L.scale = (double*)take(n * 8);
   L.cloudy = (float*)take(n * 4);
   L.mark = (int*)take(n * 4); L.seen = (int*)take(n * 4); L.link = (int*)take(n * 4); L.failed = (int*)take(n * 4); L.frontier = (int*)take(n * 4);
   L.nodes = (int*)take(MAX_CHANNEL * 8); L.parent = (int*)take(MAX_CHANNEL * 8); L.polarity = (int*)take(MAX_CHANNEL * 8);
   L.dep = (double*)take(MAX_CHANNEL * 8);
   L.lv = (double*)take((size_t)LT_COUNT * nz * 8);
   L.part = (double*)take(((n + 255) / 256 + 1) * 8);
-  L.es.nx = nx; L.es.ny = ny; L.es.nz = nz; L.es.mh = (int)mh;
-  L.es.S1 = (double2*)take(spec * 16); L.es.S2 = (double2*)take(spec * 16);
-  L.es.cp = (double*)take(spec * 8); L.es.ipiv = (double*)take(spec * 8); L.es.lo = (double*)take((size_t)nz * 8);
-  L.es.twx = (double2*)take((size_t)nx * 16); L.es.twy = (double2*)take((size_t)ny * 16);
+  H.es.shape(nx, ny, nz - 2);
+  H.es.S = (double2*)take(spec * 16);
+  H.es.a = (double*)take(spec * 8); H.es.b = (double*)take(spec * 8); H.es.c = (double*)take(spec * 8);
+  H.es.twx = (double2*)take((size_t)nx * 16); H.es.twy = (double2*)take((size_t)ny * 16);
 }
 
 int lightning_init(cudaStream_t st, const sg_grid* g, const double* rho, LgtHost& H) {
@@ -480,16 +481,16 @@ int lightning_init(cudaStream_t st, const sg_grid* g, const double* rho, LgtHost
   }
   H.conductDt = 0;
   H.tables = lv;
-  std::vector<double> lo, cpv, ipv;
+  std::vector<double> a, b, c;
   std::vector<double2> tx, ty;
-  elec_host_tables(nx, ny, nz, dx, dy, g->dzs, g->hz, lo, cpv, ipv, tx, ty);
+  elec_host_tables(H.es, dx, dy, g->dzs, g->hz, a, b, c, tx, ty);
   cudaError_t e;
-  if ((e = cudaMemcpyAsync(L.lv, lv.data(), lv.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(L.es.cp, cpv.data(), cpv.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(L.es.ipiv, ipv.data(), ipv.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(L.es.lo, lo.data(), lo.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(L.es.twx, tx.data(), tx.size() * 16, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(L.es.twy, ty.data(), ty.size() * 16, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+  if ((e = spectral64_limits()) != cudaSuccess || (e = cudaMemcpyAsync(L.lv, lv.data(), lv.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(H.es.a, a.data(), a.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(H.es.b, b.data(), b.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(H.es.c, c.data(), c.size() * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(H.es.twx, tx.data(), tx.size() * 16, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(H.es.twy, ty.data(), ty.size() * 16, cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return (int)e;
   H.dxy = dx * dy;
   return 0;
@@ -529,7 +530,7 @@ int lightning_probe(cudaStream_t st, const RunDesc& R, LgtHost& H, double* phi, 
   const int nb = blocks(R.n, 256), ni = blocks(R.n - 2 * R.layer, 256);
   k_lgt_cloudy<<<nb, 256, 0, st>>>(R, L);
   k_lgt_rho<<<nb, 256, 0, st>>>(R, L);
-  elec_solve_launch(L.es, L.rho, L.phi, st);
+  elec_solve_launch(H.es, L.rho, L.phi, st);
   k_lgt_search_reset<<<1, 32, 0, st>>>(L);
   k_lgt_strongest<<<ni, 256, 0, st>>>(R, L, -1);
   k_lgt_pick<<<ni, 256, 0, st>>>(R, L, -1);
@@ -576,7 +577,7 @@ void launch_search(LgtJob& J) {
   const int nb = blocks(J.R.n, 256), ni = blocks(J.R.n - 2 * J.R.layer, 256);
   cudaStream_t st = J.H->st;
   k_lgt_rho<<<nb, 256, 0, st>>>(J.R, L);
-  elec_solve_launch(L.es, L.rho, L.phi, st);
+  elec_solve_launch(J.H->es, L.rho, L.phi, st);
   if (J.k == J.limit) { launch_finish(J); J.phase = LgtJob::FINISHING; return; }
   k_lgt_search_reset<<<1, 32, 0, st>>>(L);
   k_lgt_strongest<<<ni, 256, 0, st>>>(J.R, L, J.stamp);
@@ -624,7 +625,7 @@ cudaError_t advance(LgtJob& J) {
       if (!end) {
         // the field of the charge as it now stands; before the contact the channel stays neutral on it
         k_lgt_rho<<<blocks(J.R.n, 256), 256, 0, H.st>>>(J.R, H.dev);
-        elec_solve_launch(H.dev.es, H.dev.rho, H.dev.phi, H.st);
+        elec_solve_launch(H.es, H.dev.rho, H.dev.phi, H.st);
         launch_stage(J);
         break;
       }

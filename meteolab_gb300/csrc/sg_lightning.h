@@ -40,7 +40,6 @@ struct LgtDev {
   double *rho = nullptr, *phi = nullptr, *sigma = nullptr, *weight = nullptr, *scale = nullptr, *dep = nullptr, *lv = nullptr, *part = nullptr;
   float* cloudy = nullptr;
   int *mark = nullptr, *seen = nullptr, *link = nullptr, *failed = nullptr, *frontier = nullptr, *nodes = nullptr, *parent = nullptr, *polarity = nullptr;
-  ElecSolve es;
 };
 
 // One flash (the reference's Flash record, src/core/lightning.ts:69-106, without the drawing and the TLE).
@@ -54,6 +53,7 @@ struct FlashRecord {
 
 struct LgtHost {
   LgtDev dev;
+  Spectral64 es;         // the potential's solve
   int flashId = 0;
   uint32_t seed = 0;     // config.seed + 1 (src/core/model.ts:1538)
   bool corona = true;    // over land (:1539)
@@ -81,7 +81,7 @@ struct LgtJob {
 };
 
 size_t lightning_bytes(int nx, int ny, int nz);
-void lightning_bind(char* base, int nx, int ny, int nz, LgtDev& L);
+void lightning_bind(char* base, int nx, int ny, int nz, LgtHost& H);
 int lightning_init(cudaStream_t st, const sg_grid* g, const double* rho, LgtHost& H);
 // The run's lightning stream and pinned host buffers (once).
 int lightning_host_buffers(LgtHost& H);

@@ -8,15 +8,16 @@
 // as the preconditioner (sg_faces_*).
 //
 // Layout: velocities FP32 [n] (node x + nx (y + ny z)); the cells' vectors FP64 [nc * nx * ny], nc = nz - 1 (cell
-// x + nx (y + ny k) between node levels k and k + 1); spectra FP64 complex [nc][nx/2 + 1][ny]. One CG iteration is
-// twelve launches: the cut cells' gradient of the search direction (a thread per node), its divergence fused with the
-// d.Sd partial sums (a thread per cell), the q/r update fused with the r.r partials, the preconditioner (x-DFT per row,
-// y-DFT per column, a Thomas sweep per mode over the levels, y- and x-inverse, the last fused with the r.z partials),
-// the direction update, and one-block reductions that finish each dot product in a fixed order (the result does not
-// depend on scheduling) and keep alpha, beta and the stopping test on the device. Eight iterations are one CUDA graph,
+// x + nx (y + ny k) between node levels k and k + 1); spectra FP64 complex [nc][nx/2 + 1][ny]. One CG iteration is seven
+// launches (the faces' six): the new direction with the column fluxes of its gradient, their divergence with d.Sd (the
+// faces: one kernel for both), the q/r update with r.r and the preconditioner's x-transform, its y-transform, vertical
+// sweeps and y-inverse (sg_spectral64.cuh), and its x-inverse with r.z. Each dot product is finished, and acted on, by
+// the block that ends last, from the partials in a fixed order (the result does not depend on scheduling); alpha, beta
+// and the stopping test stay on the device. Eight iterations are one CUDA graph,
 // replayed until the device's stop flag is set: the host reads one int per eight iterations; every kernel of an
-// iteration after the stop returns at once, so the iterations done, the residual and the result are exactly those
-// of the reference's loop (:313-329), which stops at the first top-of-loop test it passes.
+// iteration after the stop returns at once, so the iterations done, the residual and the result are those
+// of the reference's loop (:313-329), which stops at the first top-of-loop test it passes. The FP64 pipe bounds the
+// kernels (two operations a clock and SM), so their FP64 instructions are counted: see k_mp_flux and sg_spectral64.cuh.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -24,7 +25,10 @@
 #include <string>
 #include <vector>
 #include "sg_kernels.h"
+#include "sg_spectral64.cuh"
 #include "stormgpu.h"
+
+using namespace sg;
 
 namespace {
 
@@ -150,14 +154,16 @@ void slope_area(const HostGrid& g, const float* h, float* area) {
 // 2 a zero right-hand side (nothing to project).
 struct MpState {
   double bb, tol2bb, rz, rr, alpha, beta, tolerance;
-  int k, done, maxIt, keepBB;
+  int k, done, maxIt, keepRR;
 };
 enum { STOP = 1, ZERO = 2, ANY = 3 };
-enum { R_BB, R_RZ0, R_RR, R_DSD, R_RZN, R_RR_KEEP, R_TEST };
+enum { R_BB, R_RR0, R_RZ0, R_DSD, R_RR, R_RZN };
 
 struct Geo {
   const uint8_t *solid, *wall, *dropped;
-  const double *invMass, *low, *high, *rho, *dzs, *hz;
+  // A, B: a column's shares of each cell layer's fluxes (see k_mp_flux); invMass 1 / (rho0 h), wMass rho0 / 4 of it, zero
+  // where w is; rho4 rho0 / 4; idz 1 / dzs
+  const double *A, *B, *invMass, *wMass, *rho, *rho4, *dzs, *idz, *hz;
   int nx, ny, nz, layer, nc;
   size_t n, cells;
   double dx, dy;
@@ -187,12 +193,129 @@ __global__ void k_mp_mask(float* __restrict__ u, float* __restrict__ v, float* _
   else if (g.wall[i] || i < (size_t)g.layer || i >= g.n - g.layer) w[i] = 0;
 }
 
-// divergencePart (:240-264) of every cell; DOT 1 adds the partial sums of out . with, DOT 2 of out . out.
-template <class S, int DOT>
-__global__ void __launch_bounds__(TPB) k_mp_div(const S* __restrict__ u, const S* __restrict__ v, const S* __restrict__ w,
-                                                double* __restrict__ out, const double* __restrict__ with, double* __restrict__ part,
-                                                Geo g, const MpState* __restrict__ st, int skip) {
+// Adds a dot product's block sums and acts on it in the block that finishes last (a counter; no block waits): the
+// partials in a fixed order, so the result does not depend on which block that is (the scalars of :306-329).
+template <int OP>
+__device__ __forceinline__ void finish_dot(double dot, double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st) {
   __shared__ double sh[32];
+  __shared__ bool last;
+  const int id = blockIdx.y * gridDim.x + blockIdx.x, nparts = gridDim.x * gridDim.y;
+  const double mine = block_sum(dot, sh);
+  if (threadIdx.x == 0) {
+    part[id] = mine;
+    __threadfence();
+    last = atomicAdd(arrived, 1u) == (unsigned)nparts - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double v = 0;
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += __ldcg(part + i);
+  __syncthreads();  // (sh is read by the first sum's warp)
+  const double s = block_sum(v, sh);
+  if (threadIdx.x != 0) return;
+  *arrived = 0;
+  if (OP == R_BB) {
+    st->bb = s; st->tol2bb = st->tolerance * st->tolerance * s; st->rr = st->keepRR ? s : 0; st->k = 0;
+    if (!(s > 0)) st->done = ZERO;
+  } else if (OP == R_RR0) {  // the first guess's residual: the first top-of-loop test
+    if (st->maxIt > 0) { st->rr = s; if (s <= st->tol2bb) st->done = STOP; }
+  } else if (OP == R_RZ0) {
+    st->rz = s;
+    if (st->maxIt <= 0 || (st->keepRR && !(st->rr > st->tol2bb))) st->done |= STOP;
+  } else if (OP == R_DSD) {
+    if (!(s > 0)) st->done = STOP;
+    else st->alpha = st->rz / s;
+  } else if (OP == R_RR) {
+    // The update's residual and the next iteration's top-of-loop test: what follows the update in this iteration changes
+    // no result, so a solve that passes stops here and counts it. The faces keep the last update's residual (:137), the
+    // projection the last one tested (:314).
+    if (st->keepRR) {
+      st->rr = s;
+      if (!(s > st->tol2bb)) { st->k++; st->done = STOP; }
+    } else if (st->k + 1 < st->maxIt) {
+      st->rr = s;
+      if (s <= st->tol2bb) { st->k++; st->done = STOP; }
+    }
+  } else {
+    st->beta = s / st->rz; st->rz = s; st->k++;
+    if (st->k >= st->maxIt) st->done = STOP;
+  }
+}
+
+// The operator works on column fluxes: for every column and cell layer k, with the shares A = rho0 low / 4 of the node
+// below (0 when solid) and B = rho0 (high + low of a solid node) / 4 of the one above, fu = A u_k + B u_(k+1), fv alike,
+// fw = rho0 w / 4 at k + 1 less that at k; a cell's divergence is the difference of its four columns' fluxes. The
+// gradient of a cell vector, over the node masses, is formed a column at a time from the same shares (the operator's
+// adjoint), so one march up the column makes S d's fluxes without a pass over node velocities: 26 FP64 instructions a
+// layer here and 13 a cell in k_mp_div, against 59 with the nodes between and some 340 with the divides they replace.
+// Each thread marches `seg` layers of one column. DIR: of the new direction z + beta d, which it also writes.
+template <bool DIR>
+__global__ void __launch_bounds__(TPB) k_mp_flux(const double* __restrict__ d, const double* __restrict__ z, double* __restrict__ dn,
+                                                 double* __restrict__ fu, double* __restrict__ fv, double* __restrict__ fw, Geo g, int seg,
+                                                 const MpState* __restrict__ st, int skip) {
+  if (st->done & skip) return;
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= g.layer) return;
+  const int j = col / g.nx, x = col - j * g.nx, j0 = j * g.nx, jm = (j == 0 ? g.ny - 1 : j - 1) * g.nx, xm = x == 0 ? g.nx - 1 : x - 1;
+  const int k0 = blockIdx.y * seg, k1 = min(g.nc, k0 + seg);
+  const double beta = DIR ? st->beta : 0;
+  struct Layer { double u, v, w; };  // of one cell layer: the x and y differences and the sum over h of the node's four cells
+  auto layer_of = [&](int k) {
+    Layer L{0, 0, 0};
+    if (k < 0 || k >= g.nc) return L;
+    const size_t l = (size_t)k * g.layer;
+    double a = d[xm + jm + l], b = d[x + jm + l], c = d[xm + j0 + l], e = d[col + l];
+    if (DIR) {
+      a = fma(beta, a, z[xm + jm + l]); b = fma(beta, b, z[x + jm + l]); c = fma(beta, c, z[xm + j0 + l]); e = fma(beta, e, z[col + l]);
+      if (k >= k0 && k < k1) dn[col + l] = e;
+    }
+    const double ab = a + b, ce = c + e;
+    L.u = (a + c) - (b + e); L.v = ab - ce; L.w = (ab + ce) * g.idz[k];
+    return L;
+  };
+  auto share_a = [&](int k) { return k >= 0 && k < g.nc ? g.A[col + (size_t)k * g.layer] : 0.0; };
+  auto share_b = [&](int k) { return k >= 0 && k < g.nc ? g.B[col + (size_t)k * g.layer] : 0.0; };
+  struct Vel { double u, v, w; };
+  auto node = [&](int k, const Layer& below, const Layer& here, double b, double a) {
+    const size_t i = col + (size_t)k * g.layer;
+    const double m = g.invMass[i];
+    return Vel{fma(a, here.u, b * below.u) * m, fma(a, here.v, b * below.v) * m, (below.w - here.w) * g.wMass[i]};
+  };
+  Layer L0 = layer_of(k0 - 1), L1 = layer_of(k0);
+  double a = share_a(k0);
+  Vel lo = node(k0, L0, L1, share_b(k0 - 1), a);
+  for (int k = k0; k < k1; k++) {
+    const Layer L2 = layer_of(k + 1);
+    const double b = share_b(k), an = share_a(k + 1);
+    const Vel hi = node(k + 1, L1, L2, b, an);
+    const size_t c = col + (size_t)k * g.layer;
+    fu[c] = fma(a, lo.u, b * hi.u);
+    fv[c] = fma(a, lo.v, b * hi.v);
+    fw[c] = fma(g.rho4[k + 1], hi.w, -(g.rho4[k] * lo.w));
+    lo = hi; a = an; L1 = L2;
+  }
+}
+
+// The column fluxes of the node winds (divergencePart, :240-264).
+__global__ void __launch_bounds__(TPB) k_mp_wind_flux(const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
+                                                      double* __restrict__ fu, double* __restrict__ fv, double* __restrict__ fw, Geo g) {
+  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= g.cells) return;
+  const int k = (int)(c / g.layer);
+  const size_t up = c + g.layer;
+  const double a = g.A[c], b = g.B[c];
+  fu[c] = a * (double)u[c] + b * (double)u[up];
+  fv[c] = a * (double)v[c] + b * (double)v[up];
+  fw[c] = g.rho4[k + 1] * (double)w[up] - g.rho4[k] * (double)w[c];
+}
+
+// Every cell's divergence from its four columns' fluxes, with sx and sy for 1 / dx and 1 / dy (their squares for S d: the
+// gradient's own is applied here). DOT 1: with the sum of out . with; 2: of out . out.
+template <int DOT>
+__global__ void __launch_bounds__(TPB) k_mp_div(const double* __restrict__ fu, const double* __restrict__ fv, const double* __restrict__ fw,
+                                                double* __restrict__ out, const double* __restrict__ with, double sx, double sy,
+                                                double* __restrict__ part, unsigned* __restrict__ arrived, Geo g, MpState* __restrict__ st, int skip) {
   if (st && (st->done & skip)) return;
   const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double dot = 0;
@@ -201,62 +324,16 @@ __global__ void __launch_bounds__(TPB) k_mp_div(const S* __restrict__ u, const S
     if (!g.dropped[c]) {
       const int k = (int)(c / g.layer), rem = (int)(c - (size_t)k * g.layer), j = rem / g.nx, i = rem - j * g.nx;
       const int i1 = i + 1 == g.nx ? 0 : i + 1, j0 = j * g.nx, j1 = (j + 1 == g.ny ? 0 : j + 1) * g.nx;
-      const size_t l = (size_t)k * g.layer;
-      const double r0 = g.rho[k] / 4, r1 = g.rho[k + 1] / 4;
-      double ddx = 0, ddy = 0, ddz = 0;
-#pragma unroll
-      for (int corner = 0; corner < 4; corner++) {
-        const size_t lo = (size_t)((corner & 1 ? i1 : i) + (corner & 2 ? j1 : j0)) + l, up = lo + g.layer;
-        const double hi = g.high[lo];
-        if (hi > 0) {
-          const bool s = g.solid[lo] != 0;
-          const double lw = g.low[lo], a = s ? 0 : r0 * lw, b = r1 * (hi + (s ? lw : 0));
-          const double fu = a * (double)u[lo] + b * (double)u[up], fv = a * (double)v[lo] + b * (double)v[up];
-          ddx += corner & 1 ? fu : -fu;
-          ddy += corner & 2 ? fv : -fv;
-        }
-        ddz += r1 * (double)w[up] - r0 * (double)w[lo];
-      }
-      val = ddx / g.dx + ddy / g.dy + ddz / g.dzs[k];
+      const size_t l = (size_t)k * g.layer, p = i + j0 + l, q = i1 + j0 + l, r = i + j1 + l, s = i1 + j1 + l;
+      const double ddx = (fu[q] + fu[s]) - (fu[p] + fu[r]), ddy = (fv[r] + fv[s]) - (fv[p] + fv[q]), ddz = (fw[p] + fw[q]) + (fw[r] + fw[s]);
+      val = fma(ddx, sx, fma(ddy, sy, ddz * g.idz[k]));
     }
     out[c] = val;
     if (DOT == 1) dot = val * with[c];
     if (DOT == 2) dot = val * val;
   }
-  if (DOT) {
-    const double s = block_sum(dot, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-  }
-}
-
-// gradientPart (:270-300) of every node: the operator's adjoint over the node's mass of phi = q / dzs (zero in the
-// dropped cells), times the cells' heights.
-__global__ void __launch_bounds__(TPB) k_mp_grad(const double* __restrict__ q, double* __restrict__ tu, double* __restrict__ tv,
-                                                 double* __restrict__ tw, Geo g, const MpState* __restrict__ st, int skip) {
-  if (st->done & skip) return;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.n) return;
-  if (g.solid[i]) { tu[i] = 0; tv[i] = 0; tw[i] = 0; return; }
-  const int k = (int)(i / g.layer), rem = (int)(i - (size_t)k * g.layer), j = rem / g.nx, x = rem - j * g.nx;
-  const int xm = x == 0 ? g.nx - 1 : x - 1, jm = (j == 0 ? g.ny - 1 : j - 1) * g.nx, j0 = j * g.nx, col = x + j0;
-  const bool below = k > 0, above = k < g.nz - 1;
-  const double r = g.rho[k] / 4;
-  auto phi = [&](size_t cell, double dz) { return g.dropped[cell] ? 0.0 : q[cell] / dz; };
-  double gu = 0, gv = 0, gw = 0;
-  if (above) {
-    const size_t l = (size_t)k * g.layer;
-    const double f = g.low[col + l] * r, h = g.dzs[k];
-    const double a = h * phi(xm + jm + l, h), b = h * phi(x + jm + l, h), c = h * phi(xm + j0 + l, h), d = h * phi(x + j0 + l, h);
-    gu += f * (a - b + c - d) / g.dx; gv += f * (a + b - c - d) / g.dy; gw -= r * (a + b + c + d) / h;
-  }
-  if (below) {
-    const size_t l = (size_t)(k - 1) * g.layer;
-    const double f = r * (g.high[col + l] + (g.solid[col + l] ? g.low[col + l] : 0)), h = g.dzs[k - 1];
-    const double a = h * phi(xm + jm + l, h), b = h * phi(x + jm + l, h), c = h * phi(xm + j0 + l, h), d = h * phi(x + j0 + l, h);
-    gu += f * (a - b + c - d) / g.dx; gv += f * (a + b - c - d) / g.dy; gw += r * (a + b + c + d) / h;
-  }
-  const double m = g.invMass[i];
-  tu[i] = gu * m; tv[i] = gv * m; tw[i] = g.wall[i] || !below || !above ? 0 : gw * m;
+  if (DOT == 1) finish_dot<R_DSD>(dot, part, arrived, st);
+  if (DOT == 2) finish_dot<R_BB>(dot, part, arrived, st);
 }
 
 // The first guess q = V phi from the last pressure (:311).
@@ -266,196 +343,68 @@ __global__ void k_mp_start(const double* __restrict__ p, double* __restrict__ q,
   if (c < g.cells) q[c] = g.dropped[c] ? 0 : p[c] * dt * g.dzs[c / g.layer];
 }
 
-// r = -b - S q with the r.r partials (:313).
+// r = -b - S q with its square (:313).
 __global__ void __launch_bounds__(TPB) k_mp_resid(const double* __restrict__ b, const double* __restrict__ sq, double* __restrict__ r,
-                                                  double* __restrict__ part, Geo g, const MpState* __restrict__ st) {
-  __shared__ double sh[32];
+                                                  double* __restrict__ part, unsigned* __restrict__ arrived, Geo g, MpState* __restrict__ st) {
   if (st->done & ZERO) return;
   const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double v = 0;
   if (c < g.cells) { v = -b[c] - sq[c]; r[c] = v; }
-  const double s = block_sum(v * v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  finish_dot<R_RR0>(v * v, part, arrived, st);
 }
 
-// q += alpha d, r -= alpha S d, with the r.r partials of the next top-of-loop test (:324).
-__global__ void __launch_bounds__(TPB) k_mp_update(double* __restrict__ q, double* __restrict__ r, const double* __restrict__ d,
-                                                   const double* __restrict__ sd, double* __restrict__ part, Geo g, const MpState* __restrict__ st) {
-  __shared__ double sh[32];
+// q += alpha d, r -= alpha S d and the new residual's square (:324), with the preconditioner's x-transform of the new r:
+// the rows of a block's group are updated on their way into shared memory.
+__global__ void k_mp_update_xfwd(double* __restrict__ q, double* __restrict__ r, const double* __restrict__ d, const double* __restrict__ sd,
+                                 double2* __restrict__ S, int nx, int ny, int pairs, Fft64 P, const double2* __restrict__ tw,
+                                 double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st) {
+  extern __shared__ double2 z64[];
   if (st->done) return;
   const double alpha = st->alpha;
-  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double v = 0;
-  if (c < g.cells) { q[c] += alpha * d[c]; v = r[c] - alpha * sd[c]; r[c] = v; }
-  const double s = block_sum(v * v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  const int k = blockIdx.y, y0 = blockIdx.x * 2 * pairs, rows = min(2 * pairs, ny - y0);
+  const size_t base = (size_t)k * nx * ny + (size_t)y0 * nx;
+  double rr = 0;
+  for (int e = threadIdx.x; e < (rows + (rows & 1)) * nx; e += blockDim.x) {
+    const int row = e / nx, x = e - row * nx;
+    double v = 0;
+    if (row < rows) {
+      q[base + e] = fma(alpha, d[base + e], q[base + e]);
+      v = fma(-alpha, sd[base + e], r[base + e]);
+      r[base + e] = v;
+      rr = fma(v, v, rr);
+    }
+    reinterpret_cast<double*>(&z64[(row >> 1) * nx + x])[row & 1] = v;
+  }
+  __syncthreads();
+  const double2* Z = fft64_rows(z64, z64 + pairs * nx, (rows + 1) / 2, P, tw);
+  fft64_unpack(Z, S, nx, ny, y0, rows, k);
+  finish_dot<R_RR>(rr, part, arrived, st);
 }
 
-// d = z (first) or d = z + beta d (:331, :328).
-__global__ void k_mp_dir(double* __restrict__ d, const double* __restrict__ z, Geo g, const MpState* __restrict__ st, int first) {
-  if (st->done & (first ? ZERO : ANY)) return;
-  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < g.cells) d[c] = first ? z[c] : z[c] + st->beta * d[c];
-}
-
-// One block finishes a dot product from the partials in a fixed order and acts on it (the scalars of :306-329).
+// The preconditioner's x inverse: z = the plain solution (the face solve's), or with dzs V phi, zero in the dropped cells
+// (:355), and the sum r . z (OP: what it is for).
 template <int OP>
-__global__ void __launch_bounds__(TPB) k_mp_reduce(MpState* __restrict__ st, const double* __restrict__ part, int nparts, int skip) {
-  __shared__ double sh[32];
+__global__ void k_mp_xinv(const double2* __restrict__ S, double* __restrict__ out, const double* __restrict__ r, int nx, int ny, int pairs, Fft64 P,
+                          const double2* __restrict__ tw, const double* __restrict__ dzs, const uint8_t* __restrict__ dropped,
+                          double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st, int skip) {
+  extern __shared__ double2 z64[];
   if (st->done & skip) return;
-  double v = 0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += part[i];
-  const double s = block_sum(v, sh);
-  if (threadIdx.x != 0) return;
-  if (OP == R_BB) {
-    st->bb = s; st->tol2bb = st->tolerance * st->tolerance * s; st->rr = st->keepBB ? s : 0; st->k = 0;
-    if (!(s > 0)) st->done = ZERO;
-  } else if (OP == R_RZ0) {
-    st->rz = s;
-    if (st->maxIt <= 0) st->done = STOP;
-  } else if (OP == R_RR) {
-    st->rr = s;
-    if (s <= st->tol2bb) st->done = STOP;
-  } else if (OP == R_RR_KEEP) {
-    st->rr = s;
-  } else if (OP == R_TEST) {
-    if (!(st->rr > st->tol2bb)) st->done = STOP;
-  } else if (OP == R_DSD) {
-    if (!(s > 0)) st->done = STOP;
-    else st->alpha = st->rz / s;
-  } else {
-    st->beta = s / st->rz; st->rz = s; st->k++;
-    if (st->k >= st->maxIt) st->done = STOP;
-  }
-}
-
-// Forward x-DFT of each cell row of scale * src: S1[k][m][y], m <= nx / 2.
-// With `per` (the face solve): row = scale * src / per[k], the right-hand side over each level's height.
-__global__ void k_mp_xdft(const double* __restrict__ src, double scale, const double* __restrict__ per, double2* __restrict__ S1,
-                          const double2* __restrict__ twx, Geo g, int mh, const MpState* __restrict__ st, int skip) {
-  extern __shared__ double row[];
-  if (st && (st->done & skip)) return;
-  const int y = blockIdx.x, k = blockIdx.y, nx = g.nx;
-  const double* s = src + (size_t)k * g.layer + (size_t)y * nx;
-  for (int x = threadIdx.x; x < nx; x += blockDim.x) row[x] = per ? scale * s[x] / per[k] : scale * s[x];
+  const int k = blockIdx.y, y0 = blockIdx.x * 2 * pairs, rows = min(2 * pairs, ny - y0);
+  fft64_pack(S, z64, nx, ny, y0, rows, k);
   __syncthreads();
-  for (int m = threadIdx.x; m <= mh; m += blockDim.x) {
-    double re = 0, im = 0;
-    int t = 0;
-    for (int x = 0; x < nx; x++) {
-      const double2 tw = twx[t];
-      re = fma(row[x], tw.x, re);
-      im = fma(-row[x], tw.y, im);
-      t += m;
-      if (t >= nx) t -= nx;
-    }
-    S1[((size_t)k * (mh + 1) + m) * g.ny + y] = make_double2(re, im);
-  }
-}
-
-// y-DFT of each (cell layer, x-mode) column, sign -1 forward and +1 inverse (unnormalised).
-__global__ void k_mp_ydft(const double2* __restrict__ in, double2* __restrict__ out, const double2* __restrict__ twy, int ny, int mh, double sign,
-                          const MpState* __restrict__ st, int skip) {
-  extern __shared__ double2 colv[];
-  if (st && (st->done & skip)) return;
-  const size_t base = ((size_t)blockIdx.y * (mh + 1) + blockIdx.x) * ny;
-  for (int y = threadIdx.x; y < ny; y += blockDim.x) colv[y] = in[base + y];
-  __syncthreads();
-  for (int nn = threadIdx.x; nn < ny; nn += blockDim.x) {
-    double re = 0, im = 0;
-    int t = 0;
-    for (int y = 0; y < ny; y++) {
-      const double2 tw = twy[t], v = colv[y];
-      const double s = sign * tw.y;
-      re = fma(v.x, tw.x, fma(-v.y, s, re));
-      im = fma(v.y, tw.x, fma(v.x, s, im));
-      t += nn;
-      if (t >= ny) t -= ny;
-    }
-    out[base + nn] = make_double2(re, im);
-  }
-}
-
-// One mode a thread, the reference's Thomas sweep over the cell layers (pressure.ts:118-140) with the rows' lower
-// coefficients and pivots from the host (the face solve's right-hand sides times each level's height, rs); the forward
-// values kept in place for the back substitution. A mode the
-// reference zeroes, and the pinned lowest cell of the uniform mode, have an infinite pivot. The recurrence is a
-// dependent chain of FP64 divides: each eight layers' coefficients and right-hand sides are loaded before their eight
-// steps, so a step waits on the divide, not on memory.
-constexpr int THOMAS_AHEAD = 8;
-__global__ void k_mp_thomas(double2* __restrict__ S2, const double* __restrict__ lo, const double* __restrict__ cp,
-                            const double* __restrict__ piv, const double* __restrict__ rs, int nc, int modes, const MpState* __restrict__ st,
-                            int skip) {
-  if (st && (st->done & skip)) return;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= modes) return;
-  double2 d = make_double2(0, 0);
-  for (int k0 = 0; k0 < nc; k0 += THOMAS_AHEAD) {
-    double2 r[THOMAS_AHEAD];
-    double a[THOMAS_AHEAD], m[THOMAS_AHEAD];
-#pragma unroll
-    for (int q = 0; q < THOMAS_AHEAD; q++) {
-      const size_t at = (size_t)min(k0 + q, nc - 1) * modes + g;
-      r[q] = S2[at]; a[q] = lo[at]; m[q] = piv[at];
-      if (rs) { const double h = rs[min(k0 + q, nc - 1)]; r[q] = make_double2(h * r[q].x, h * r[q].y); }
-    }
-#pragma unroll
-    for (int q = 0; q < THOMAS_AHEAD; q++)
-      if (k0 + q < nc) {
-        d = make_double2((r[q].x - a[q] * d.x) / m[q], (r[q].y - a[q] * d.y) / m[q]);
-        S2[(size_t)(k0 + q) * modes + g] = d;
-      }
-  }
-  for (int k1 = nc - 2; k1 >= 0; k1 -= THOMAS_AHEAD) {
-    double2 v[THOMAS_AHEAD];
-    double c[THOMAS_AHEAD];
-#pragma unroll
-    for (int q = 0; q < THOMAS_AHEAD; q++) {
-      const size_t at = (size_t)max(k1 - q, 0) * modes + g;
-      v[q] = S2[at]; c[q] = cp[at];
-    }
-#pragma unroll
-    for (int q = 0; q < THOMAS_AHEAD; q++)
-      if (k1 - q >= 0) {
-        d = make_double2(v[q].x - c[q] * d.x, v[q].y - c[q] * d.y);
-        S2[(size_t)(k1 - q) * modes + g] = d;
-      }
-  }
-}
-
-// Inverse x-DFT of each cell row from its half spectrum, / (nx ny). MODE 1: the preconditioner's z = V phi, zero in the
-// dropped cells (:355), with the r.z partials; 2: the plain solution with the r.z partials (the face solve's); 0: the
-// plain solution (the flat solve's pressure).
-template <int MODE>
-__global__ void k_mp_xidft(const double2* __restrict__ S1, double* __restrict__ out, const double* __restrict__ r, double* __restrict__ part,
-                           const double2* __restrict__ twx, Geo g, int mh, const MpState* __restrict__ st, int skip) {
-  extern __shared__ double2 zs[];
-  __shared__ double sh[32];
-  if (st && (st->done & skip)) return;
-  const int y = blockIdx.x, k = blockIdx.y, nx = g.nx;
-  for (int m = threadIdx.x; m <= mh; m += blockDim.x) zs[m] = S1[((size_t)k * (mh + 1) + m) * g.ny + y];
-  __syncthreads();
-  const double scale = 1.0 / ((double)nx * g.ny);
+  const double2* Z = fft64_rows(z64, z64 + pairs * nx, (rows + 1) / 2, P, tw);
+  const size_t base = (size_t)k * nx * ny + (size_t)y0 * nx;
+  const double h = dzs ? dzs[k] : 1;
   double dot = 0;
-  for (int x = threadIdx.x; x < nx; x += blockDim.x) {
-    double v = zs[0].x;
-    int t = 0;
-    for (int m = 1; m <= mh; m++) {
-      t += x;
-      if (t >= nx) t -= nx;
-      const double2 tw = twx[t];
-      v = 2 * m == nx ? fma(zs[m].x, tw.x, v) : fma(2.0, fma(zs[m].x, tw.x, -zs[m].y * tw.y), v);
-    }
-    const size_t c = (size_t)k * g.layer + (size_t)y * nx + x;
-    double val = v * scale;
-    if (MODE == 1) val = g.dropped[c] ? 0 : val * g.dzs[k];
-    if (MODE) dot += r[c] * val;
-    out[c] = val;
+  for (int e = threadIdx.x; e < rows * nx; e += blockDim.x) {
+    const int row = e / nx, x = e - row * nx;
+    const double2 v = Z[(row >> 1) * nx + x];
+    double val = row & 1 ? -v.y : v.x;
+    if (dzs) val = dropped[base + e] ? 0 : val * h;
+    dot = fma(r[base + e], val, dot);
+    out[base + e] = val;
   }
-  if (MODE) {
-    const double s = block_sum(dot, sh);
-    if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
-  }
+  finish_dot<OP>(dot, part, arrived, st);
 }
 
 // The potential phi = q / V and the pressure kept, phi / dt (:332).
@@ -465,16 +414,29 @@ __global__ void k_mp_finish(const double* __restrict__ q, double* __restrict__ p
   if (c < g.cells) p[c] = q[c] / g.dzs[c / g.layer] / dt;
 }
 
-// u = M (u* - G phi): the correction added in FP32 stores, then masked (:334-336).
-__global__ void k_mp_correct(float* __restrict__ u, float* __restrict__ v, float* __restrict__ w, const double* __restrict__ tu,
-                             const double* __restrict__ tv, const double* __restrict__ tw, Geo g, const MpState* __restrict__ st) {
+// u = M (u* - G phi) (gradientPart :270-300 of q = V phi at each node): the correction added in FP32 stores, then masked
+// (:334-336).
+__global__ void __launch_bounds__(TPB) k_mp_correct(float* __restrict__ u, float* __restrict__ v, float* __restrict__ w, const double* __restrict__ q,
+                                                    Geo g, const MpState* __restrict__ st) {
   if (st->done & ZERO) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.n) return;
   if (g.solid[i]) { u[i] = 0; v[i] = 0; w[i] = 0; return; }
-  u[i] = (float)((double)u[i] + tu[i]);
-  v[i] = (float)((double)v[i] + tv[i]);
-  const float wn = (float)((double)w[i] + tw[i]);
+  const int k = (int)(i / g.layer), col = (int)(i - (size_t)k * g.layer), j = col / g.nx, x = col - j * g.nx;
+  const int xm = x == 0 ? g.nx - 1 : x - 1, jm = (j == 0 ? g.ny - 1 : j - 1) * g.nx, j0 = j * g.nx;
+  double gu = 0, gv = 0, gw = 0;
+  for (int side = 0; side < 2; side++) {  // the layer above the node, then the one below
+    const int kc = k - side;
+    if (kc < 0 || kc >= g.nc) continue;
+    const size_t l = (size_t)kc * g.layer;
+    const double a = q[xm + jm + l], b = q[x + jm + l], c = q[xm + j0 + l], d = q[x + j0 + l];
+    const double f = side ? g.B[col + l] : g.A[col + l], ab = a + b, cd = c + d, s = (ab + cd) * g.idz[kc];
+    gu = fma(f, (a + c) - (b + d), gu); gv = fma(f, ab - cd, gv); gw += side ? s : -s;
+  }
+  const double m = g.invMass[i];
+  u[i] = (float)((double)u[i] + gu * m / g.dx);
+  v[i] = (float)((double)v[i] + gv * m / g.dy);
+  const float wn = (float)((double)w[i] + gw * g.wMass[i]);
   w[i] = g.wall[i] || i < (size_t)g.layer || i >= g.n - g.layer ? 0.0f : wn;
 }
 
@@ -521,7 +483,7 @@ __global__ void k_mp_flat_correct(const double* __restrict__ p, float* __restric
 
 struct FaceGeo {
   const uint8_t* open;  // bit 1 the face to x + 1, 2 to y + 1, 4 to z + 1: both nodes fluid
-  const double *ax, *ay, *hn, *rho, *dzs;
+  const double *ax, *ay, *hn, *rho, *dzs, *cx, *cy, *cz;
   int nx, ny, nz, layer;
   size_t n;
   double dx, dy;
@@ -557,11 +519,11 @@ __global__ void k_tm_faces(const float* __restrict__ u, const float* __restrict_
   mz[i] = o & 4 ? (g.rho[a.z] + g.rho[a.z + 1]) / 2 * ((double)w[i] + (double)w[i + g.layer]) / 2 : 0;
 }
 
-// The apertures' divergence of the face fluxes (:96-105): MODE 0 b = -(h div) with the b.b partials, 1 div = h div / hn.
+// The apertures' divergence of the face fluxes (:96-105): MODE 0 b = -(h div) with its square, 1 div = h div / hn.
 template <int MODE>
 __global__ void __launch_bounds__(TPB) k_tm_tdiv(const double* __restrict__ mx, const double* __restrict__ my, const double* __restrict__ mz,
-                                                 double* __restrict__ out, double* __restrict__ part, FaceGeo g) {
-  __shared__ double sh[32];
+                                                 double* __restrict__ out, double* __restrict__ part, unsigned* __restrict__ arrived, FaceGeo g,
+                                                 MpState* __restrict__ st) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double dot = 0;
   if (i < g.n) {
@@ -572,34 +534,33 @@ __global__ void __launch_bounds__(TPB) k_tm_tdiv(const double* __restrict__ mx, 
     else v = v / g.hn[i];
     out[i] = v;
   }
-  if (MODE == 0) {
-    const double s = block_sum(dot, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-  }
+  if (MODE == 0) finish_dot<R_BB>(dot, part, arrived, st);
 }
 
-// S d = -h div(M rho0 grad d) (:170-176) at each node from d at it and its six neighbours (each face flux as the
-// reference forms it), with the d.Sd partials.
-__global__ void __launch_bounds__(TPB) k_tm_apply(const double* __restrict__ d, double* __restrict__ out, double* __restrict__ part, FaceGeo g,
-                                                  const MpState* __restrict__ st) {
-  __shared__ double sh[32];
+// S d = -h div(M rho0 grad d) (:170-176) at each node, d the new direction z + beta d formed at the node and its six
+// neighbours, with the sum d . S d: six differences times the faces' coefficients (cx = rho0 ax / dx^2 of an open face to
+// x + 1, cy alike, cz = rho0 / dzs to z + 1, zero when shut).
+__global__ void __launch_bounds__(TPB) k_tm_apply(const double* __restrict__ d, const double* __restrict__ z, double* __restrict__ dn, double* __restrict__ out,
+                                                  double* __restrict__ part, unsigned* __restrict__ arrived, FaceGeo g, MpState* __restrict__ st) {
   if (st->done) return;
+  const double beta = st->beta;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double dot = 0;
   if (i < g.n) {
     const Node a = node_of(i, g);
-    const double r = g.rho[a.z], di = d[i];
-    const uint8_t oi = g.open[i];
-    const double fxi = oi & 1 ? r * (d[a.e] - di) / g.dx : 0, fxw = g.open[a.w] & 1 ? r * (di - d[a.w]) / g.dx : 0;
-    const double fyi = oi & 2 ? r * (d[a.no] - di) / g.dy : 0, fys = g.open[a.so] & 2 ? r * (di - d[a.so]) / g.dy : 0;
-    const double fzi = oi & 4 ? (g.rho[a.z] + g.rho[a.z + 1]) / 2 * (d[i + g.layer] - di) / g.dzs[a.z] : 0;
-    const double fzb = a.z > 0 && (g.open[i - g.layer] & 4) ? (g.rho[a.z - 1] + g.rho[a.z]) / 2 * (di - d[i - g.layer]) / g.dzs[a.z - 1] : 0;
-    const double v = -((g.ax[i] * fxi - g.ax[a.w] * fxw) / g.dx + (g.ay[i] * fyi - g.ay[a.so] * fys) / g.dy + (fzi - fzb));
+    auto dir = [&](size_t at) { return fma(beta, d[at], z[at]); };
+    const double di = dir(i);
+    dn[i] = di;
+    double v = g.cx[i] * (di - dir(a.e));
+    v = fma(g.cx[a.w], di - dir(a.w), v);
+    v = fma(g.cy[i], di - dir(a.no), v);
+    v = fma(g.cy[a.so], di - dir(a.so), v);
+    if (a.z + 1 < g.nz) v = fma(g.cz[i], di - dir(i + g.layer), v);
+    if (a.z > 0) v = fma(g.cz[i - g.layer], di - dir(i - g.layer), v);
     out[i] = v;
     dot = di * v;
   }
-  const double s = block_sum(dot, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  finish_dot<R_DSD>(dot, part, arrived, st);
 }
 
 // The fluxes lose M rho0 grad(q) (:150).
@@ -617,7 +578,16 @@ __global__ void k_tm_correct(const double* __restrict__ q, double* __restrict__ 
 }
 
 int blocks(size_t count) { return (int)((count + TPB - 1) / TPB); }
-int threads_for(int count) { return std::min(256, std::max(32, (count + 31) / 32 * 32)); }
+// Shared memory beyond 48 KB for rows of more than 1536 points.
+cudaError_t solve_limits() {
+  cudaError_t e = spectral64_limits();
+  for (const void* k : {(const void*)k_mp_update_xfwd, (const void*)k_mp_xinv<R_RZ0>, (const void*)k_mp_xinv<R_RZN>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SPECTRAL64_SMEM);
+  return e;
+}
+// Layers a thread of k_mp_flux marches: two layers' work is its start, so as many as leave 152 SMs a block each of 256
+// columns, within 4..16.
+int flux_seg(int layer, int nc) { return std::min(16, std::max(4, (int)((size_t)layer * nc / (152 * (size_t)TPB)))); }
 
 }  // namespace
 
@@ -625,14 +595,15 @@ struct sg_masked {
   sg_context* ctx = nullptr;
   HostGrid hg{};
   Geo geo{};
-  int mh = 0, modes = 0, maxIt = 200;
+  int maxIt = 200;
   double tolerance = 1e-6;
   bool any = false;
   char* mem = nullptr;
   float *u = nullptr, *v = nullptr, *w = nullptr;
-  double *p = nullptr, *b = nullptr, *q = nullptr, *r = nullptr, *z = nullptr, *d = nullptr, *sd = nullptr, *tu = nullptr, *tv = nullptr,
-         *tw = nullptr, *pDot = nullptr, *pRR = nullptr, *lo = nullptr, *cp = nullptr, *piv = nullptr;
-  double2 *S1 = nullptr, *S2 = nullptr, *twx = nullptr, *twy = nullptr;
+  double *p = nullptr, *b = nullptr, *q = nullptr, *r = nullptr, *z = nullptr, *d[2] = {}, *sd = nullptr, *fu = nullptr, *fv = nullptr,
+         *fw = nullptr, *part = nullptr;
+  unsigned* arrived = nullptr;
+  Spectral64 sp;
   MpState* st = nullptr;
   std::vector<uint8_t> dropped;
   cudaGraphExec_t chunk = nullptr;
@@ -643,14 +614,14 @@ struct sg_masked {
 struct sg_faces {
   sg_context* ctx = nullptr;
   FaceGeo fg{};
-  Geo geo{};  // the node vectors as the shared kernels see them: cells = n, nc = nz
-  int mh = 0, modes = 0, maxIt = 400;
+  int maxIt = 400;
   double tolerance = 1e-10;
   char* mem = nullptr;
   float *u = nullptr, *v = nullptr, *w = nullptr;
-  double *mx = nullptr, *my = nullptr, *mz = nullptr, *div = nullptr, *b = nullptr, *q = nullptr, *r = nullptr, *z = nullptr, *d = nullptr,
-         *sd = nullptr, *pDot = nullptr, *pRR = nullptr, *lo = nullptr, *cp = nullptr, *piv = nullptr, *hz = nullptr;
-  double2 *S1 = nullptr, *S2 = nullptr, *twx = nullptr, *twy = nullptr;
+  double *mx = nullptr, *my = nullptr, *mz = nullptr, *div = nullptr, *q = nullptr, *r = nullptr, *z = nullptr, *d[2] = {},
+         *sd = nullptr, *part = nullptr;
+  unsigned* arrived = nullptr;
+  Spectral64 sp;
   MpState* st = nullptr;
   cudaGraphExec_t chunk = nullptr;
   int iterations = 0;
@@ -659,58 +630,60 @@ struct sg_faces {
 
 namespace {
 
-constexpr int CHUNK = 8;
+constexpr int REPLAY = 8;
 
-// The face solve's preconditioner (flatSolve, advection.ts:179-184): div = -r / h, the flat face solve (forward,
-// modes with the right-hand sides times h, inverse) into z, with the r.z partials.
-void enqueue_face_precondition(sg_faces* f, cudaStream_t s, int skip) {
-  const Geo& g = f->geo;
-  const int nx = g.nx, ny = g.ny, nz = g.nc, mh = f->mh;
-  k_mp_xdft<<<dim3(ny, nz), threads_for(mh + 1), (size_t)nx * 8, s>>>(f->r, -1.0, f->hz, f->S1, f->twx, g, mh, f->st, skip);
-  k_mp_ydft<<<dim3(mh + 1, nz), threads_for(ny), (size_t)ny * 16, s>>>(f->S1, f->S2, f->twy, ny, mh, -1.0, f->st, skip);
-  k_mp_thomas<<<(f->modes + 63) / 64, 64, 0, s>>>(f->S2, f->lo, f->cp, f->piv, f->hz, nz, f->modes, f->st, skip);
-  k_mp_ydft<<<dim3(mh + 1, nz), threads_for(ny), (size_t)ny * 16, s>>>(f->S2, f->S1, f->twy, ny, mh, 1.0, f->st, skip);
-  k_mp_xidft<2><<<dim3(ny, nz), threads_for(nx), (size_t)(mh + 1) * 16, s>>>(f->S1, f->z, f->r, f->pDot, f->twx, g, mh, f->st, skip);
+// The preconditioner's x-inverse into z with r . z, on the shape of a solve.
+template <int OP>
+void enqueue_xinv(const Spectral64& S, double* z, const double* r, const double* dzs, const uint8_t* dropped, double* part, unsigned* arrived,
+                  MpState* st, int skip, cudaStream_t s) {
+  k_mp_xinv<OP><<<dim3(S.x.groups, S.levels), S.x.threads, S.x.smem, s>>>(S.S, z, r, S.nx, S.ny, S.x.pairs, S.px, S.twx, dzs, dropped, part, arrived, st, skip);
+}
+// The preconditioner after the x-transform of r: the flat solve of -r (:351-356; the face solve's flatSolve,
+// advection.ts:179-184, whose right-hand side over and back times each level's height is -r too).
+template <int OP>
+void enqueue_precondition(const Spectral64& S, double* z, const double* r, const double* dzs, const uint8_t* dropped, double* part, unsigned* arrived,
+                          MpState* st, int skip, cudaStream_t s) {
+  S.forward_y(s, &st->done, skip);
+  S.sweep(s, 1, &st->done, skip);
+  S.inverse_y(s, &st->done, skip);
+  enqueue_xinv<OP>(S, z, r, dzs, dropped, part, arrived, st, skip, s);
+}
+// The start's: the x-transform of r as it stands, then the same.
+void enqueue_first_precondition(const Spectral64& S, double* z, const double* r, const double* dzs, const uint8_t* dropped, double* part,
+                                unsigned* arrived, MpState* st, cudaStream_t s) {
+  S.forward_x(r, s, &st->done, ANY);
+  enqueue_precondition<R_RZ0>(S, z, r, dzs, dropped, part, arrived, st, ANY, s);
+}
+// The end of an iteration from S d on: the update with its x-transform, the preconditioner.
+void enqueue_descent(const Spectral64& S, double* q, double* r, double* z, const double* d, const double* sd, const double* dzs, const uint8_t* dropped,
+                     double* part, unsigned* arrived, MpState* st, cudaStream_t s) {
+  k_mp_update_xfwd<<<dim3(S.x.groups, S.levels), S.x.threads, S.x.smem, s>>>(q, r, d, sd, S.S, S.nx, S.ny, S.x.pairs, S.px, S.twx, part, arrived, st);
+  enqueue_precondition<R_RZN>(S, z, r, dzs, dropped, part, arrived, st, ANY, s);
 }
 
-// One iteration of setVelocityMasked's loop (:127-145): the test on the last update's r.r, S d and d.Sd, alpha, the
-// update with its r.r kept, the preconditioner, beta, the new direction.
-void enqueue_face_iteration(sg_faces* f, cudaStream_t s) {
-  const Geo& g = f->geo;
-  const int nb = blocks(g.cells);
-  k_mp_reduce<R_TEST><<<1, TPB, 0, s>>>(f->st, f->pRR, 0, ANY);
-  k_tm_apply<<<nb, TPB, 0, s>>>(f->d, f->sd, f->pDot, f->fg, f->st);
-  k_mp_reduce<R_DSD><<<1, TPB, 0, s>>>(f->st, f->pDot, nb, ANY);
-  k_mp_update<<<nb, TPB, 0, s>>>(f->q, f->r, f->d, f->sd, f->pRR, g, f->st);
-  k_mp_reduce<R_RR_KEEP><<<1, TPB, 0, s>>>(f->st, f->pRR, nb, ANY);
-  enqueue_face_precondition(f, s, ANY);
-  k_mp_reduce<R_RZN><<<1, TPB, 0, s>>>(f->st, f->pDot, g.ny * g.nc, ANY);
-  k_mp_dir<<<nb, TPB, 0, s>>>(f->d, f->z, g, f->st, 0);
+// One iteration of setVelocityMasked's loop (:127-145); `odd`: which of the two direction buffers is the last one's.
+void enqueue_face_iteration(sg_faces* f, int odd, cudaStream_t s) {
+  double *last = f->d[odd], *next = f->d[odd ^ 1];
+  k_tm_apply<<<blocks(f->fg.n), TPB, 0, s>>>(last, f->z, next, f->sd, f->part, f->arrived, f->fg, f->st);
+  enqueue_descent(f->sp, f->q, f->r, f->z, next, f->sd, nullptr, nullptr, f->part, f->arrived, f->st, s);
 }
 
-// The preconditioner z = P S0^-1 P r (:351-356): the flat solve of -r, z = V phi, with the r.z partials.
-void enqueue_precondition(sg_masked* m, cudaStream_t s, int skip) {
+// The fluxes of a cell vector's gradient (of z + beta d where dn is given).
+void enqueue_flux(sg_masked* m, const double* d, const double* z, double* dn, int skip, cudaStream_t s) {
   const Geo& g = m->geo;
-  const int nx = g.nx, ny = g.ny, nc = g.nc, mh = m->mh;
-  k_mp_xdft<<<dim3(ny, nc), threads_for(mh + 1), (size_t)nx * 8, s>>>(m->r, -1.0, nullptr, m->S1, m->twx, g, mh, m->st, skip);
-  k_mp_ydft<<<dim3(mh + 1, nc), threads_for(ny), (size_t)ny * 16, s>>>(m->S1, m->S2, m->twy, ny, mh, -1.0, m->st, skip);
-  k_mp_thomas<<<(m->modes + 63) / 64, 64, 0, s>>>(m->S2, m->lo, m->cp, m->piv, nullptr, nc, m->modes, m->st, skip);
-  k_mp_ydft<<<dim3(mh + 1, nc), threads_for(ny), (size_t)ny * 16, s>>>(m->S2, m->S1, m->twy, ny, mh, 1.0, m->st, skip);
-  k_mp_xidft<1><<<dim3(ny, nc), threads_for(nx), (size_t)(mh + 1) * 16, s>>>(m->S1, m->z, m->r, m->pDot, m->twx, g, mh, m->st, skip);
+  const int seg = flux_seg(g.layer, g.nc), tpb = 64;
+  const dim3 grid((g.layer + tpb - 1) / tpb, (g.nc + seg - 1) / seg);
+  if (dn) k_mp_flux<true><<<grid, tpb, 0, s>>>(d, z, dn, m->fu, m->fv, m->fw, g, seg, m->st, skip);
+  else k_mp_flux<false><<<grid, tpb, 0, s>>>(d, nullptr, nullptr, m->fu, m->fv, m->fw, g, seg, m->st, skip);
 }
 
 // One iteration of the loop (:314-329).
-void enqueue_iteration(sg_masked* m, cudaStream_t s) {
+void enqueue_iteration(sg_masked* m, int odd, cudaStream_t s) {
   const Geo& g = m->geo;
-  const int cb = blocks(g.cells), nb = blocks(g.n);
-  k_mp_reduce<R_RR><<<1, TPB, 0, s>>>(m->st, m->pRR, cb, ANY);
-  k_mp_grad<<<nb, TPB, 0, s>>>(m->d, m->tu, m->tv, m->tw, g, m->st, ANY);
-  k_mp_div<double, 1><<<cb, TPB, 0, s>>>(m->tu, m->tv, m->tw, m->sd, m->d, m->pDot, g, m->st, ANY);
-  k_mp_reduce<R_DSD><<<1, TPB, 0, s>>>(m->st, m->pDot, cb, ANY);
-  k_mp_update<<<cb, TPB, 0, s>>>(m->q, m->r, m->d, m->sd, m->pRR, g, m->st);
-  enqueue_precondition(m, s, ANY);
-  k_mp_reduce<R_RZN><<<1, TPB, 0, s>>>(m->st, m->pDot, g.ny * g.nc, ANY);
-  k_mp_dir<<<cb, TPB, 0, s>>>(m->d, m->z, g, m->st, 0);
+  double *last = m->d[odd], *next = m->d[odd ^ 1];
+  enqueue_flux(m, last, m->z, next, ANY, s);
+  k_mp_div<1><<<blocks(g.cells), TPB, 0, s>>>(m->fu, m->fv, m->fw, m->sd, next, 1 / (g.dx * g.dx), 1 / (g.dy * g.dy), m->part, m->arrived, g, m->st, ANY);
+  enqueue_descent(m->sp, m->q, m->r, m->z, next, m->sd, g.dzs, g.dropped, m->part, m->arrived, m->st, s);
 }
 
 int fail(sg_masked* m, const char* what, cudaError_t e) {
@@ -768,41 +741,55 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
   if (cudaSetDevice(sg_context_device(ctx)) != cudaSuccess) return sg_context_fail(ctx, SG_ERR_DEVICE, "masked projection: cudaSetDevice");
   const int nx = g.nx, ny = g.ny, nz = g.nz, nc = nz - 1, layer = g.layer, mh = nx / 2, modes = (mh + 1) * ny;
   const size_t n = g.n, cells = (size_t)layer * nc, spec = (size_t)nc * modes;
+  Spectral64 sp;
+  sp.shape(nx, ny, nc);
 
-  // The constructor (:190-218): solid and wall nodes, 1 / (rho0 hn), the columns' shares of each cell layer, dropped cells.
-  std::vector<uint8_t> solid(n), wall(n, 0), dropped(cells, 0);
+  // The constructor (:190-218): solid and wall nodes, 1 / (rho0 hn), dropped cells, and as k_mp_flux takes them the
+  // columns' shares of each cell layer's fluxes (of the layer's half below its middle and above it that are above the
+  // ground) and the nodes' weights.
+  std::vector<uint8_t> solid(n), wall(n, 0), blocked(cells), dropped(cells);
   std::vector<int32_t> levels(layer);
-  std::vector<double> heights(n), inv(n, 0.0), low(cells), high(cells);
+  std::vector<double> heights(n), inv(n, 0.0), wm(n, 0.0), sa(cells), sb(cells), rho4(nz), idz(nz, 0.0);
   solid_levels(g, ground, solid.data(), levels.data());
   node_heights(g, solid.data(), levels.data(), ground, heights.data());
   bool any = false;
   for (size_t i = 0; i < n; i++) any = any || solid[i];
   for (int c = 0; c < layer; c++) any = any || ground[c] > 0;
-  for (int k = 0; k < nz; k++)
+  for (int k = 0; k < nz; k++) rho4[k] = rho[k] / 4;
+  for (int k = 0; k < nc; k++) idz[k] = 1 / g.dzs[k];
+  for (int k = 0; k < nz; k++) {
+    const double r = rho[k], r4 = k > 0 && k < nz - 1 ? rho4[k] : 0;
     for (int c = 0; c < layer; c++) {
       const size_t i = c + (size_t)k * layer;
       if (solid[i]) continue;
-      if (g.zs[k] <= (double)ground[c]) wall[i] = 1;
-      inv[i] = 1 / (rho[k] * heights[i]);
+      inv[i] = 1 / (r * heights[i]);
+      if (g.zs[k] <= (double)ground[c]) wall[i] = 1; else wm[i] = r4 * inv[i];
     }
-  for (int k = 0; k < nc; k++)
+  }
+  for (int k = 0; k < nc; k++) {
+    const double half = g.dzs[k] / 2, middle = g.zs[k] + half, per = 1 / half;
     for (int c = 0; c < layer; c++) {
-      const double half = g.dzs[k] / 2, middle = g.zs[k] + half, h = (double)ground[c];
-      low[c + (size_t)k * layer] = std::min(1.0, std::max(0.0, (middle - std::max(h, g.zs[k])) / half));
-      high[c + (size_t)k * layer] = std::min(1.0, std::max(0.0, (g.zs[k + 1] - std::max(h, middle)) / half));
+      const size_t at = c + (size_t)k * layer;
+      const double h = (double)ground[c];
+      const double low = std::min(1.0, std::max(0.0, (middle - std::max(h, g.zs[k])) * per));
+      const double high = std::min(1.0, std::max(0.0, (g.zs[k + 1] - std::max(h, middle)) * per));
+      blocked[at] = high == 0;
+      sa[at] = high > 0 && !solid[at] ? rho4[k] * low : 0;
+      sb[at] = high > 0 ? rho4[k + 1] * (high + (solid[at] ? low : 0)) : 0;
     }
+  }
   for (int k = 0; k < nc; k++)
-    for (int j = 0; j < ny; j++)
-      for (int i = 0; i < nx; i++) {
-        const size_t l = (size_t)k * layer;
-        const int i1 = (i + 1) % nx, j0 = j * nx, j1 = ((j + 1) % ny) * nx;
-        if (high[i + j0 + l] == 0 && high[i1 + j0 + l] == 0 && high[i + j1 + l] == 0 && high[i1 + j1 + l] == 0) dropped[i + j0 + l] = 1;
-      }
+    for (int j = 0; j < ny; j++) {
+      const uint8_t *b0 = blocked.data() + (size_t)k * layer + (size_t)j * nx, *b1 = blocked.data() + (size_t)k * layer + (size_t)((j + 1) % ny) * nx;
+      uint8_t* out = dropped.data() + (size_t)k * layer + (size_t)j * nx;
+      for (int i = 0; i < nx; i++) { const int i1 = i + 1 == nx ? 0 : i + 1; out[i] = b0[i] & b0[i1] & b1[i] & b1[i1]; }
+    }
 
-  // The flat solve's rows per mode (pressure.ts:36-44, :118-140): lower coefficient, pivot and cp = up / pivot of each
-  // cell layer in the reference's elimination order. Modes it zeroes and the uniform mode's pinned lowest cell get an
-  // infinite pivot (their values come out zero).
-  std::vector<double> tlo(spec, 0.0), tcp(spec, 0.0), tpiv(spec, 0.0);
+  // The flat solve's rows per mode (pressure.ts:36-44, :118-140) as the sweep takes them: a = 1 / pivot (with the
+  // transforms' factor), b = lower / pivot and c = upper / pivot of each cell layer in the reference's elimination order.
+  // Modes it zeroes and the uniform mode's pinned lowest cell have a and b zero (their values come out zero).
+  const double factor = sp.factor();
+  std::vector<double> ta(spec, 0.0), tb(spec, 0.0), tcp(spec, 0.0);
   auto exact = [](double x) { return x < 1e-12 ? 0 : x > 1 - 1e-12 ? 1 : x; };
   for (int m = 0; m <= mh; m++)
     for (int q = 0; q < ny; q++) {
@@ -810,10 +797,7 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
       const double sy = exact(std::pow(std::sin(PI_ * q / ny), 2)), cy = exact(std::pow(std::cos(PI_ * q / ny), 2));
       const double a = 4 * (sx * cy / (g.dx * g.dx) + cx * sy / (g.dy * g.dy)), b = cx * cy;
       const size_t mode = (size_t)m * ny + q;
-      if ((a == 0 && b == 0) || (nc == 1 && a == 0)) {
-        for (int k = 0; k < nc; k++) tpiv[(size_t)k * modes + mode] = INFINITY;
-        continue;
-      }
+      if ((a == 0 && b == 0) || (nc == 1 && a == 0)) continue;
       const bool pinned = a == 0;
       double cprev = 0;
       for (int k = 0; k < nc; k++) {
@@ -823,10 +807,10 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
         bool zero = false;
         if (pinned && k == 0) { lo = 0; di = 1; up = 0; zero = true; }
         if (pinned && k == 1) lo = 0;
-        const double piv = k == 0 ? di : di - lo * cprev;
-        cprev = up / piv;
+        const double ip = 1 / (k == 0 ? di : di - lo * cprev);
+        cprev = up * ip;
         const size_t at = (size_t)k * modes + mode;
-        tlo[at] = lo; tcp[at] = cprev; tpiv[at] = zero ? INFINITY : piv;
+        ta[at] = zero ? 0 : factor * ip; tb[at] = zero ? 0 : lo * ip; tcp[at] = cprev;
       }
     }
   std::vector<double2> tx(nx), ty(ny);
@@ -835,42 +819,49 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
 
   // One allocation, 256-byte aligned parts.
   auto al = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-  const size_t nparts = std::max((size_t)blocks(cells), (size_t)ny * nc);
+  const size_t nparts = std::max((size_t)blocks(cells), (size_t)sp.x.groups * nc);
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += al(bytes); return o; };
   const size_t oU = take(n * 4), oV = take(n * 4), oW = take(n * 4), oP = take(cells * 8), oB = take(cells * 8), oQ = take(cells * 8), oR = take(cells * 8),
-               oZ = take(cells * 8), oD = take(cells * 8), oSd = take(cells * 8), oTu = take(n * 8), oTv = take(n * 8), oTw = take(n * 8),
-               oPd = take(nparts * 8), oPr = take(nparts * 8), oLo = take(spec * 8), oCp = take(spec * 8), oPv = take(spec * 8),
-               oS1 = take(spec * 16), oS2 = take(spec * 16), oTx = take((size_t)nx * 16), oTy = take((size_t)ny * 16), oSt = take(sizeof(MpState)),
-               oSol = take(n), oWal = take(n), oDr = take(cells), oInv = take(n * 8), oLow = take(cells * 8), oHigh = take(cells * 8),
-               oRho = take((size_t)nz * 8), oDz = take((size_t)nz * 8), oHz = take((size_t)nz * 8), total = off;
+               oZ = take(cells * 8), oD = take(cells * 8), oD2 = take(cells * 8), oSd = take(cells * 8), oFu = take(cells * 8), oFv = take(cells * 8),
+               oFw = take(cells * 8), oPart = take(nparts * 8), oA = take(spec * 8), oBb = take(spec * 8), oC = take(spec * 8), oS = take(spec * 16),
+               oTx = take((size_t)nx * 16), oTy = take((size_t)ny * 16), oSt = take(sizeof(MpState)), oArr = take(sizeof(unsigned)), oSol = take(n),
+               oWal = take(n), oDr = take(cells), oInv = take(n * 8), oWm = take(n * 8), oSa = take(cells * 8), oSb = take(cells * 8),
+               oRho = take((size_t)nz * 8), oR4 = take((size_t)nz * 8), oDz = take((size_t)nz * 8), oIdz = take((size_t)nz * 8), oHz = take((size_t)nz * 8),
+               total = off;
   auto* s = new sg_masked;
-  s->ctx = ctx; s->hg = g; s->mh = mh; s->modes = modes; s->maxIt = max_iterations; s->tolerance = tolerance; s->any = any;
+  s->ctx = ctx; s->hg = g; s->maxIt = max_iterations; s->tolerance = tolerance; s->any = any;
   s->dropped = dropped;
-  cudaError_t e = cudaMalloc(&s->mem, total);
+  cudaError_t e = solve_limits();
+  if (e != cudaSuccess) { delete s; return sg_context_fail(ctx, SG_ERR_DEVICE, "masked projection: shared memory"); }
+  e = cudaMalloc(&s->mem, total);
   if (e != cudaSuccess) { delete s; cudaGetLastError(); return sg_context_fail(ctx, SG_ERR_BUDGET, "masked projection: device memory"); }
   char* M = s->mem;
   s->u = (float*)(M + oU); s->v = (float*)(M + oV); s->w = (float*)(M + oW);
   s->p = (double*)(M + oP); s->b = (double*)(M + oB); s->q = (double*)(M + oQ); s->r = (double*)(M + oR); s->z = (double*)(M + oZ);
-  s->d = (double*)(M + oD); s->sd = (double*)(M + oSd); s->tu = (double*)(M + oTu); s->tv = (double*)(M + oTv); s->tw = (double*)(M + oTw);
-  s->pDot = (double*)(M + oPd); s->pRR = (double*)(M + oPr); s->lo = (double*)(M + oLo); s->cp = (double*)(M + oCp); s->piv = (double*)(M + oPv);
-  s->S1 = (double2*)(M + oS1); s->S2 = (double2*)(M + oS2); s->twx = (double2*)(M + oTx); s->twy = (double2*)(M + oTy); s->st = (MpState*)(M + oSt);
+  s->d[0] = (double*)(M + oD); s->d[1] = (double*)(M + oD2); s->sd = (double*)(M + oSd); s->fu = (double*)(M + oFu); s->fv = (double*)(M + oFv);
+  s->fw = (double*)(M + oFw); s->part = (double*)(M + oPart); s->arrived = (unsigned*)(M + oArr); s->st = (MpState*)(M + oSt);
+  sp.a = (double*)(M + oA); sp.b = (double*)(M + oBb); sp.c = (double*)(M + oC); sp.S = (double2*)(M + oS);
+  sp.twx = (double2*)(M + oTx); sp.twy = (double2*)(M + oTy);
+  s->sp = sp;
   Geo& G = s->geo;
   G.solid = (const uint8_t*)(M + oSol); G.wall = (const uint8_t*)(M + oWal); G.dropped = (const uint8_t*)(M + oDr);
-  G.invMass = (const double*)(M + oInv); G.low = (const double*)(M + oLow); G.high = (const double*)(M + oHigh);
-  G.rho = (const double*)(M + oRho); G.dzs = (const double*)(M + oDz); G.hz = (const double*)(M + oHz);
+  G.A = (const double*)(M + oSa); G.B = (const double*)(M + oSb); G.invMass = (const double*)(M + oInv); G.wMass = (const double*)(M + oWm);
+  G.rho = (const double*)(M + oRho); G.rho4 = (const double*)(M + oR4); G.dzs = (const double*)(M + oDz); G.idz = (const double*)(M + oIdz);
+  G.hz = (const double*)(M + oHz);
   G.nx = nx; G.ny = ny; G.nz = nz; G.layer = layer; G.nc = nc; G.n = n; G.cells = cells; G.dx = g.dx; G.dy = g.dy;
   cudaStream_t st = sg_context_stream(ctx);
   std::vector<double> dz(nz, 0.0);
   std::copy(g.dzs, g.dzs + nz - 1, dz.begin());
   struct Up { size_t off; const void* src; size_t bytes; };
-  const Up ups[] = {{oLo, tlo.data(), spec * 8}, {oCp, tcp.data(), spec * 8}, {oPv, tpiv.data(), spec * 8}, {oTx, tx.data(), (size_t)nx * 16},
+  const Up ups[] = {{oA, ta.data(), spec * 8}, {oBb, tb.data(), spec * 8}, {oC, tcp.data(), spec * 8}, {oTx, tx.data(), (size_t)nx * 16},
                     {oTy, ty.data(), (size_t)ny * 16}, {oSol, solid.data(), n}, {oWal, wall.data(), n}, {oDr, dropped.data(), cells},
-                    {oInv, inv.data(), n * 8}, {oLow, low.data(), cells * 8}, {oHigh, high.data(), cells * 8}, {oRho, rho, (size_t)nz * 8},
-                    {oDz, dz.data(), (size_t)nz * 8}, {oHz, g.hz, (size_t)nz * 8}};
+                    {oInv, inv.data(), n * 8}, {oWm, wm.data(), n * 8}, {oSa, sa.data(), cells * 8}, {oSb, sb.data(), cells * 8},
+                    {oRho, rho, (size_t)nz * 8}, {oR4, rho4.data(), (size_t)nz * 8}, {oDz, dz.data(), (size_t)nz * 8},
+                    {oIdz, idz.data(), (size_t)nz * 8}, {oHz, g.hz, (size_t)nz * 8}};
   for (const Up& up : ups)
     if ((e = cudaMemcpyAsync(M + up.off, up.src, up.bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-  if (e == cudaSuccess) e = cudaMemsetAsync(s->d, 0, cells * 8, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s->arrived, 0, sizeof(unsigned), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     cudaFree(s->mem); delete s;
@@ -909,7 +900,8 @@ int sg_masked_divergence(sg_masked* m, const float* u, const float* v, const flo
   float* dev[3] = {m->u, m->v, m->w};
   for (int f = 0; f < 3; f++)
     if ((e = cudaMemcpyAsync(dev[f], host[f], n * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail(m, "copy in", e);
-  k_mp_div<float, 0><<<blocks(cells), TPB, 0, s>>>(m->u, m->v, m->w, m->b, nullptr, nullptr, m->geo, nullptr, 0);
+  k_mp_wind_flux<<<blocks(cells), TPB, 0, s>>>(m->u, m->v, m->w, m->fu, m->fv, m->fw, m->geo);
+  k_mp_div<0><<<blocks(cells), TPB, 0, s>>>(m->fu, m->fv, m->fw, m->b, nullptr, 1 / m->geo.dx, 1 / m->geo.dy, nullptr, nullptr, m->geo, nullptr, 0);
   if ((e = cudaMemcpyAsync(out, m->b, cells * 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess ||
       (e = cudaGetLastError()) != cudaSuccess)
     return fail(m, "divergence", e);
@@ -924,7 +916,7 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
   cudaStream_t s = sg_context_stream(m->ctx);
   const Geo& g = m->geo;
   const size_t n = g.n, cells = g.cells;
-  const int nb = blocks(n), cb = blocks(cells), nx = g.nx, ny = g.ny, nc = g.nc, mh = m->mh;
+  const int nb = blocks(n), cb = blocks(cells);
   cudaError_t e;
   float* host[3] = {u, v, w};
   float* dev[3] = {m->u, m->v, m->w};
@@ -936,50 +928,44 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
   if (!m->any) {
     // No terrain at all: the flat projection exactly (:336-339); the pressure is the flat solve's, not a first guess.
     k_mp_flat_div<<<cb, TPB, 0, s>>>(m->u, m->v, m->w, m->b, dt, g);
-    k_mp_xdft<<<dim3(ny, nc), threads_for(mh + 1), (size_t)nx * 8, s>>>(m->b, 1.0, nullptr, m->S1, m->twx, g, mh, nullptr, 0);
-    k_mp_ydft<<<dim3(mh + 1, nc), threads_for(ny), (size_t)ny * 16, s>>>(m->S1, m->S2, m->twy, ny, mh, -1.0, nullptr, 0);
-    k_mp_thomas<<<(m->modes + 63) / 64, 64, 0, s>>>(m->S2, m->lo, m->cp, m->piv, nullptr, nc, m->modes, nullptr, 0);
-    k_mp_ydft<<<dim3(mh + 1, nc), threads_for(ny), (size_t)ny * 16, s>>>(m->S2, m->S1, m->twy, ny, mh, 1.0, nullptr, 0);
-    k_mp_xidft<0><<<dim3(ny, nc), threads_for(nx), (size_t)(mh + 1) * 16, s>>>(m->S1, m->p, nullptr, nullptr, m->twx, g, mh, nullptr, 0);
+    m->sp.solve(m->b, m->p, 0, s);
     k_mp_flat_correct<<<nb, TPB, 0, s>>>(m->p, m->u, m->v, m->w, dt, g);
   } else {
     MpState init{};
     init.tolerance = m->tolerance; init.maxIt = m->maxIt;
     if ((e = cudaMemcpyAsync(m->st, &init, sizeof(MpState), cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail(m, "state", e);
-    // b = D R M u*, bb; q from the first guess, r = -b - S q, z = P S0^-1 P r, d = z, rz (:306-312).
-    k_mp_div<float, 2><<<cb, TPB, 0, s>>>(m->u, m->v, m->w, m->b, nullptr, m->pDot, g, m->st, 0);
-    k_mp_reduce<R_BB><<<1, TPB, 0, s>>>(m->st, m->pDot, cb, 0);
+    if ((e = cudaMemsetAsync(m->d[0], 0, cells * 8, s)) != cudaSuccess) return fail(m, "direction", e);  // (the first direction: z + 0 d)
+    // b = D R M u*, bb; q from the first guess, r = -b - S q and its first test, z = P S0^-1 P r, rz (:306-312).
+    k_mp_wind_flux<<<cb, TPB, 0, s>>>(m->u, m->v, m->w, m->fu, m->fv, m->fw, g);
+    k_mp_div<2><<<cb, TPB, 0, s>>>(m->fu, m->fv, m->fw, m->b, nullptr, 1 / g.dx, 1 / g.dy, m->part, m->arrived, g, m->st, 0);
     k_mp_start<<<cb, TPB, 0, s>>>(m->p, m->q, dt, g, m->st);
-    k_mp_grad<<<nb, TPB, 0, s>>>(m->q, m->tu, m->tv, m->tw, g, m->st, ZERO);
-    k_mp_div<double, 0><<<cb, TPB, 0, s>>>(m->tu, m->tv, m->tw, m->sd, nullptr, nullptr, g, m->st, ZERO);
-    k_mp_resid<<<cb, TPB, 0, s>>>(m->b, m->sd, m->r, m->pRR, g, m->st);
-    enqueue_precondition(m, s, ZERO);
-    k_mp_reduce<R_RZ0><<<1, TPB, 0, s>>>(m->st, m->pDot, ny * nc, ZERO);
-    k_mp_dir<<<cb, TPB, 0, s>>>(m->d, m->z, g, m->st, 1);
+    enqueue_flux(m, m->q, nullptr, nullptr, ZERO, s);
+    k_mp_div<0><<<cb, TPB, 0, s>>>(m->fu, m->fv, m->fw, m->sd, nullptr, 1 / (g.dx * g.dx), 1 / (g.dy * g.dy), nullptr, nullptr, g, m->st, ZERO);
+    k_mp_resid<<<cb, TPB, 0, s>>>(m->b, m->sd, m->r, m->part, m->arrived, g, m->st);
+    enqueue_first_precondition(m->sp, m->z, m->r, g.dzs, g.dropped, m->part, m->arrived, m->st, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(m, "launch", e);
     if (!m->chunk) {
       // Eight iterations as one graph (the buffers are the object's own, so one capture serves every call).
       cudaGraph_t graph = nullptr;
       if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return fail(m, "capture", e);
-      for (int it = 0; it < CHUNK; it++) enqueue_iteration(m, s);
+      for (int it = 0; it < REPLAY; it++) enqueue_iteration(m, it & 1, s);
       e = cudaStreamEndCapture(s, &graph);
       if (e == cudaSuccess) e = cudaGraphInstantiate(&m->chunk, graph, 0);
       if (graph) cudaGraphDestroy(graph);
       if (e != cudaSuccess) { m->chunk = nullptr; return fail(m, "graph", e); }
     }
-    // Every iteration either counts or stops, so maxIt / CHUNK + 1 replays always reach the stop.
+    // Every iteration either counts or stops, so maxIt / REPLAY + 1 replays always reach the stop.
     int done = 0;
     for (int c = 0;; c++) {
       if ((e = cudaMemcpyAsync(&done, &m->st->done, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return fail(m, "solve", e);
-      if (done || c > m->maxIt / CHUNK + 1) break;
+      if (done || c > m->maxIt / REPLAY + 1) break;
       if ((e = cudaGraphLaunch(m->chunk, s)) != cudaSuccess) return fail(m, "graph launch", e);
     }
     if (!done) return sg_context_fail(m->ctx, SG_ERR_DEVICE, "masked projection: the iterations did not stop");
     // u = M (u* - G phi); the pressure kept is phi / dt (:332-336).
     k_mp_finish<<<cb, TPB, 0, s>>>(m->q, m->p, dt, g, m->st);
-    k_mp_grad<<<nb, TPB, 0, s>>>(m->q, m->tu, m->tv, m->tw, g, m->st, ZERO);
-    k_mp_correct<<<nb, TPB, 0, s>>>(m->u, m->v, m->w, m->tu, m->tv, m->tw, g, m->st);
+    k_mp_correct<<<nb, TPB, 0, s>>>(m->u, m->v, m->w, m->q, g, m->st);
     MpState fin{};
     if ((e = cudaMemcpyAsync(&fin, m->st, sizeof(MpState), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return fail(m, "state", e);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(m, "solve", e);
@@ -1023,6 +1009,8 @@ int sg_faces_create(sg_context* ctx, const sg_grid* grid, const double* rho, con
   if (cudaSetDevice(sg_context_device(ctx)) != cudaSuccess) return sg_context_fail(ctx, SG_ERR_DEVICE, "masked faces: cudaSetDevice");
   const int nx = g.nx, ny = g.ny, nz = g.nz, layer = g.layer, mh = nx / 2, modes = (mh + 1) * ny;
   const size_t n = g.n, spec = (size_t)nz * modes;
+  Spectral64 sp;
+  sp.shape(nx, ny, nz);
 
   // setTerrain (advection.ts:78-90) with the model's geometry (model.ts:366-377): open faces, node heights (1 in the
   // ground), the faces' open heights.
@@ -1043,9 +1031,21 @@ int sg_faces_create(sg_context* ctx, const sg_grid* grid, const double* rho, con
         if (z < nz - 1 && !solid[i + layer]) open[i] |= 4;
       }
 
-  // The flat face solve's rows per mode (advection.ts:222-241): each level's lower coefficient, pivot and cp in the
-  // reference's order; the uniform mode's pinned lowest level with an infinite pivot.
-  std::vector<double> tlo(spec, 0.0), tcp(spec, 0.0), tpiv(spec, 0.0);
+  // The faces' coefficients of S (k_tm_apply).
+  std::vector<double> cx(n, 0.0), cy(n, 0.0), cz(n, 0.0);
+  for (int z = 0; z < nz; z++) {
+    const double rx = rho[z] / (g.dx * g.dx), ry = rho[z] / (g.dy * g.dy), rz = z < nz - 1 ? (rho[z] + rho[z + 1]) / 2 / g.dzs[z] : 0;
+    for (size_t i = (size_t)z * layer; i < (size_t)(z + 1) * layer; i++) {
+      if (open[i] & 1) cx[i] = rx * ax[i];
+      if (open[i] & 2) cy[i] = ry * ay[i];
+      if (open[i] & 4) cz[i] = rz;
+    }
+  }
+
+  // The flat face solve's rows per mode (advection.ts:222-241) as the sweep takes them, each level's in the reference's
+  // order (see the projection's above); the uniform mode's lowest level is pinned to zero.
+  const double factor = sp.factor();
+  std::vector<double> ta(spec, 0.0), tb(spec, 0.0), tcp(spec, 0.0);
   auto face = [&](int k) { return k < 0 || k >= nz - 1 ? 0.0 : (rho[k] + rho[k + 1]) / 2; };
   for (int m = 0; m <= mh; m++)
     for (int q = 0; q < ny; q++) {
@@ -1059,10 +1059,10 @@ int sg_faces_create(sg_context* ctx, const sg_grid* grid, const double* rho, con
         bool zero = false;
         if (pinned && k == 0) { lo = 0; di = 1; up = 0; zero = true; }
         if (pinned && k == 1) lo = 0;
-        const double piv = k == 0 ? di : di - lo * cprev;
-        cprev = up / piv;
+        const double ip = 1 / (k == 0 ? di : di - lo * cprev);
+        cprev = up * ip;
         const size_t at = (size_t)k * modes + mode;
-        tlo[at] = lo; tcp[at] = cprev; tpiv[at] = zero ? INFINITY : piv;
+        ta[at] = zero ? 0 : factor * ip; tb[at] = zero ? 0 : lo * ip; tcp[at] = cprev;
       }
     }
   std::vector<double2> tx(nx), ty(ny);
@@ -1070,41 +1070,45 @@ int sg_faces_create(sg_context* ctx, const sg_grid* grid, const double* rho, con
   for (int t = 0; t < ny; t++) ty[t] = make_double2(std::cos(2 * PI_ * t / ny), std::sin(2 * PI_ * t / ny));
 
   auto al = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-  const size_t nparts = std::max((size_t)blocks(n), (size_t)ny * nz);
+  const size_t nparts = std::max((size_t)blocks(n), (size_t)sp.x.groups * nz);
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += al(bytes); return o; };
   const size_t oU = take(n * 4), oV = take(n * 4), oW = take(n * 4), oMx = take(n * 8), oMy = take(n * 8), oMz = take(n * 8), oDiv = take(n * 8),
-               oB = take(n * 8), oQ = take(n * 8), oR = take(n * 8), oZ = take(n * 8), oD = take(n * 8), oSd = take(n * 8), oPd = take(nparts * 8),
-               oPr = take(nparts * 8), oLo = take(spec * 8), oCp = take(spec * 8), oPv = take(spec * 8), oS1 = take(spec * 16), oS2 = take(spec * 16),
-               oTx = take((size_t)nx * 16), oTy = take((size_t)ny * 16), oSt = take(sizeof(MpState)), oOpen = take(n), oAx = take(n * 8),
-               oAy = take(n * 8), oHn = take(n * 8), oRho = take((size_t)nz * 8), oDz = take((size_t)nz * 8), oHz = take((size_t)nz * 8), total = off;
+               oQ = take(n * 8), oR = take(n * 8), oZ = take(n * 8), oD = take(n * 8), oD2 = take(n * 8), oSd = take(n * 8), oPart = take(nparts * 8),
+               oA = take(spec * 8), oBb = take(spec * 8), oC = take(spec * 8), oS = take(spec * 16), oTx = take((size_t)nx * 16),
+               oTy = take((size_t)ny * 16), oSt = take(sizeof(MpState)), oArr = take(sizeof(unsigned)), oOpen = take(n), oAx = take(n * 8),
+               oAy = take(n * 8), oHn = take(n * 8), oCx = take(n * 8), oCy = take(n * 8), oCz = take(n * 8), oRho = take((size_t)nz * 8),
+               oDz = take((size_t)nz * 8), total = off;
   auto* f = new sg_faces;
-  f->ctx = ctx; f->mh = mh; f->modes = modes; f->maxIt = max_iterations; f->tolerance = tolerance;
-  cudaError_t e = cudaMalloc(&f->mem, total);
+  f->ctx = ctx; f->maxIt = max_iterations; f->tolerance = tolerance;
+  cudaError_t e = solve_limits();
+  if (e != cudaSuccess) { delete f; return sg_context_fail(ctx, SG_ERR_DEVICE, "masked faces: shared memory"); }
+  e = cudaMalloc(&f->mem, total);
   if (e != cudaSuccess) { delete f; cudaGetLastError(); return sg_context_fail(ctx, SG_ERR_BUDGET, "masked faces: device memory"); }
   char* M = f->mem;
   f->u = (float*)(M + oU); f->v = (float*)(M + oV); f->w = (float*)(M + oW);
-  f->mx = (double*)(M + oMx); f->my = (double*)(M + oMy); f->mz = (double*)(M + oMz); f->div = (double*)(M + oDiv); f->b = (double*)(M + oB);
-  f->q = (double*)(M + oQ); f->r = (double*)(M + oR); f->z = (double*)(M + oZ); f->d = (double*)(M + oD); f->sd = (double*)(M + oSd);
-  f->pDot = (double*)(M + oPd); f->pRR = (double*)(M + oPr); f->lo = (double*)(M + oLo); f->cp = (double*)(M + oCp); f->piv = (double*)(M + oPv);
-  f->S1 = (double2*)(M + oS1); f->S2 = (double2*)(M + oS2); f->twx = (double2*)(M + oTx); f->twy = (double2*)(M + oTy); f->st = (MpState*)(M + oSt);
-  f->hz = (double*)(M + oHz);
+  f->mx = (double*)(M + oMx); f->my = (double*)(M + oMy); f->mz = (double*)(M + oMz); f->div = (double*)(M + oDiv);
+  f->q = (double*)(M + oQ); f->r = (double*)(M + oR); f->z = (double*)(M + oZ); f->d[0] = (double*)(M + oD); f->d[1] = (double*)(M + oD2);
+  f->sd = (double*)(M + oSd); f->part = (double*)(M + oPart); f->arrived = (unsigned*)(M + oArr); f->st = (MpState*)(M + oSt);
+  sp.a = (double*)(M + oA); sp.b = (double*)(M + oBb); sp.c = (double*)(M + oC); sp.S = (double2*)(M + oS);
+  sp.twx = (double2*)(M + oTx); sp.twy = (double2*)(M + oTy);
+  f->sp = sp;
   FaceGeo& F = f->fg;
   F.open = (const uint8_t*)(M + oOpen); F.ax = (const double*)(M + oAx); F.ay = (const double*)(M + oAy); F.hn = (const double*)(M + oHn);
+  F.cx = (const double*)(M + oCx); F.cy = (const double*)(M + oCy); F.cz = (const double*)(M + oCz);
   F.rho = (const double*)(M + oRho); F.dzs = (const double*)(M + oDz);
   F.nx = nx; F.ny = ny; F.nz = nz; F.layer = layer; F.n = n; F.dx = g.dx; F.dy = g.dy;
-  Geo& G = f->geo;
-  G.nx = nx; G.ny = ny; G.nz = nz; G.layer = layer; G.nc = nz; G.n = n; G.cells = n; G.dx = g.dx; G.dy = g.dy;
   cudaStream_t st = sg_context_stream(ctx);
   std::vector<double> dz(nz, 0.0);
   std::copy(g.dzs, g.dzs + nz - 1, dz.begin());
   struct Up { size_t off; const void* src; size_t bytes; };
-  const Up ups[] = {{oLo, tlo.data(), spec * 8}, {oCp, tcp.data(), spec * 8}, {oPv, tpiv.data(), spec * 8}, {oTx, tx.data(), (size_t)nx * 16},
+  const Up ups[] = {{oA, ta.data(), spec * 8}, {oBb, tb.data(), spec * 8}, {oC, tcp.data(), spec * 8}, {oTx, tx.data(), (size_t)nx * 16},
                     {oTy, ty.data(), (size_t)ny * 16}, {oOpen, open.data(), n}, {oAx, ax.data(), n * 8}, {oAy, ay.data(), n * 8},
-                    {oHn, hn.data(), n * 8}, {oRho, rho, (size_t)nz * 8}, {oDz, dz.data(), (size_t)nz * 8}, {oHz, g.hz, (size_t)nz * 8}};
+                    {oHn, hn.data(), n * 8}, {oCx, cx.data(), n * 8}, {oCy, cy.data(), n * 8}, {oCz, cz.data(), n * 8},
+                    {oRho, rho, (size_t)nz * 8}, {oDz, dz.data(), (size_t)nz * 8}};
   for (const Up& up : ups)
     if ((e = cudaMemcpyAsync(M + up.off, up.src, up.bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-  if (e == cudaSuccess) e = cudaMemsetAsync(f->d, 0, n * 8, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(f->arrived, 0, sizeof(unsigned), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     cudaFree(f->mem); delete f;
@@ -1119,8 +1123,7 @@ int sg_faces_set_velocity(sg_faces* f, const float* u, const float* v, const flo
   if (!u || !v || !w) return sg_context_fail(f->ctx, SG_ERR_INVALID, "masked faces: u, v and w buffers");
   cudaSetDevice(sg_context_device(f->ctx));
   cudaStream_t s = sg_context_stream(f->ctx);
-  const Geo& g = f->geo;
-  const size_t n = g.n;
+  const size_t n = f->fg.n;
   const int nb = blocks(n);
   auto fail_f = [&](const char* what, cudaError_t e) {
     return sg_context_fail(f->ctx, SG_ERR_DEVICE, (std::string("masked faces: ") + what + ": " + cudaGetErrorString(e)).c_str());
@@ -1131,23 +1134,19 @@ int sg_faces_set_velocity(sg_faces* f, const float* u, const float* v, const flo
   for (int k = 0; k < 3; k++)
     if ((e = cudaMemcpyAsync(dev[k], host[k], n * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail_f("copy in", e);
   MpState init{};
-  init.tolerance = f->tolerance; init.maxIt = f->maxIt; init.keepBB = 1;
+  init.tolerance = f->tolerance; init.maxIt = f->maxIt; init.keepRR = 1;
   if ((e = cudaMemcpyAsync(f->st, &init, sizeof(MpState), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-      (e = cudaMemsetAsync(f->q, 0, n * 8, s)) != cudaSuccess)
+      (e = cudaMemsetAsync(f->q, 0, n * 8, s)) != cudaSuccess || (e = cudaMemsetAsync(f->d[0], 0, n * 8, s)) != cudaSuccess)
     return fail_f("state", e);
-  // faces, shut next to the ground; b = -h div, bb (= the first rr); r = b; z = S0^-1 r, rz; d = z (:117-126).
+  // faces, shut next to the ground; r = b = -h div, bb (= the first rr); z = S0^-1 r, rz (:117-126).
   k_tm_faces<<<nb, TPB, 0, s>>>(f->u, f->v, f->w, f->mx, f->my, f->mz, f->fg);
-  k_tm_tdiv<0><<<nb, TPB, 0, s>>>(f->mx, f->my, f->mz, f->b, f->pRR, f->fg);
-  k_mp_reduce<R_BB><<<1, TPB, 0, s>>>(f->st, f->pRR, nb, 0);
-  if ((e = cudaMemcpyAsync(f->r, f->b, n * 8, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return fail_f("copy", e);
-  enqueue_face_precondition(f, s, ZERO);
-  k_mp_reduce<R_RZ0><<<1, TPB, 0, s>>>(f->st, f->pDot, g.ny * g.nc, ZERO);
-  k_mp_dir<<<nb, TPB, 0, s>>>(f->d, f->z, g, f->st, 1);
+  k_tm_tdiv<0><<<nb, TPB, 0, s>>>(f->mx, f->my, f->mz, f->r, f->part, f->arrived, f->fg, f->st);
+  enqueue_first_precondition(f->sp, f->z, f->r, nullptr, nullptr, f->part, f->arrived, f->st, s);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail_f("launch", e);
   if (!f->chunk) {
     cudaGraph_t graph = nullptr;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return fail_f("capture", e);
-    for (int it = 0; it < CHUNK; it++) enqueue_face_iteration(f, s);
+    for (int it = 0; it < REPLAY; it++) enqueue_face_iteration(f, it & 1, s);
     e = cudaStreamEndCapture(s, &graph);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&f->chunk, graph, 0);
     if (graph) cudaGraphDestroy(graph);
@@ -1157,13 +1156,13 @@ int sg_faces_set_velocity(sg_faces* f, const float* u, const float* v, const flo
   for (int c = 0;; c++) {
     if ((e = cudaMemcpyAsync(&done, &f->st->done, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return fail_f("solve", e);
-    if (done || c > f->maxIt / CHUNK + 1) break;
+    if (done || c > f->maxIt / REPLAY + 1) break;
     if ((e = cudaGraphLaunch(f->chunk, s)) != cudaSuccess) return fail_f("graph launch", e);
   }
   if (!done) return sg_context_fail(f->ctx, SG_ERR_DEVICE, "masked faces: the iterations did not stop");
   // The fluxes lose M rho0 grad(q); div the apertures' divergence over the node heights (:150-152).
   k_tm_correct<<<nb, TPB, 0, s>>>(f->q, f->mx, f->my, f->mz, f->fg, f->st);
-  k_tm_tdiv<1><<<nb, TPB, 0, s>>>(f->mx, f->my, f->mz, f->div, nullptr, f->fg);
+  k_tm_tdiv<1><<<nb, TPB, 0, s>>>(f->mx, f->my, f->mz, f->div, nullptr, nullptr, f->fg, f->st);
   MpState fin{};
   if ((e = cudaMemcpyAsync(&fin, f->st, sizeof(MpState), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return fail_f("state", e);
   double* outs[4] = {mx, my, mz, div};

@@ -973,7 +973,7 @@ int sg_run_create(sg_context* ctx, const sg_grid* g, const sg_base_state* b, con
   if (elec || two) { d.vfall = (float*)(mem + Lo.vfall); d.ez = (float*)(mem + Lo.ez); d.cpart = (double*)(mem + Lo.cpart); }
   if (elec) {
     r.lgt = std::make_unique<LgtHost>();
-    lightning_bind(mem + Lo.lgt, g->nx, g->ny, g->nz, r.lgt->dev);
+    lightning_bind(mem + Lo.lgt, g->nx, g->ny, g->nz, *r.lgt);
     r.lgt->seed = (uint32_t)sw->lightning_seed; r.lgt->corona = sw->corona != 0;
     r.zs.assign(g->zs, g->zs + g->nz); r.dzs.assign(g->dzs, g->dzs + g->nz - 1); r.hz.assign(g->hz, g->hz + g->nz);
     r.grid = *g; r.grid.zs = r.zs.data(); r.grid.dzs = r.dzs.data(); r.grid.hz = r.hz.data();
