@@ -539,72 +539,28 @@ __global__ void k_proj_div_xfft(const RunDesc* __restrict__ runs, const int4* it
   }
 }
 
-// One x-wavenumber m per item: the y-transform of every layer, one tridiagonal solve per y-wavenumber n along the
-// vertical in FP64, the inverse y-transform. The solve is Thomas' algorithm with the LU factors made on the host in
-// FP64 (the k = 0 uniform mode pinned at the ground, the null modes zero): per level the forward sweep
-// d_k = A_k r_k - B_k d_(k-1) and the back substitution x_k = d_k - C_k x_(k+1), one real recurrence per
-// (n, real/imaginary part), the two parts sharing the coefficients. FACE: rows -rho h lambda + vertical faces
-// (src/core/advection.ts:222-241); PRES: the density-weighted consistent Laplacian (src/core/pressure.ts:104-140).
-// The inverse transform is the forward one of the conjugate, conjugated: the back substitution stores conj(x).
-// Transform of `rows` rows at S (stride n) with a scratch of `cap` rows; the result ends in S.
-__device__ void fft_rows_grouped(float2* S, float2* T, int n, int rows, int cap, const FftPlan& P) {
-  for (int k0 = 0; k0 < rows; k0 += cap) {
-    const int g = min(cap, rows - k0);
-    float2* r = fft_rows_any(S + k0 * n, T, n, g, P);
-    if (r != S + k0 * n) {
-      for (int e = threadIdx.x; e < g * n; e += blockDim.x) S[k0 * n + e] = r[e];
-      __syncthreads();
-    }
-  }
-}
-
-// `group`: layers the scratch holds (all of them: the transforms ping-pong between the two buffers; fewer, for tall
-// or wide grids: the layers go through the scratch in groups).
-__global__ void k_proj_modes(const RunDesc* __restrict__ runs, const int4* items, int nitems, int mode, int group) {
+// The row path's y-transforms in place on the spectrum, `cols` columns (x-wavenumber, layer) an item: forward, or the
+// unnormalised inverse (the conjugate of the forward transform of the conjugate). With the mode sweeps between them
+// (k_proj_sweep) they are the row path's mode solves. One block per x-wavenumber used to do all three on its whole slab in
+// shared memory: 161 blocks of 200 KB on the 320-wide grid, two waves on 152 SMs, 283 us; the spectrum (26 MB there) stays
+// in L2 between the launches, so the split costs little traffic and spreads over all SMs.
+__global__ void __launch_bounds__(256) k_proj_ycols(const RunDesc* __restrict__ runs, const int4* items, int nitems, int mode, int inverse) {
   extern __shared__ float2 smc[];
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    const int m = items[it].y, ny = R.ny, nz = R.nz, nzc = mode == PROJ_FACE ? nz : nz - 1;
-    const bool whole = group >= nzc;
-    float2* S = smc;                   // [nzc][ny]
-    float2* T = smc + nzc * ny;        // [group][ny] scratch
-    float2* g = R.spec + (size_t)m * nzc * ny;
-    for (int e = threadIdx.x; e < nzc * ny; e += blockDim.x) S[e] = g[e];
+    const int ny = R.ny, nzc = mode == PROJ_FACE ? R.nz : R.nz - 1, columns = R.nm * nzc, cols = items[it].z;
+    const int c0 = items[it].y * cols, count = min(cols, columns - c0);
+    if (count <= 0) continue;  // (the items cover the face projection's columns, one layer more than the pressure's)
+    float2* S = smc;              // [count][ny]
+    float2* T = smc + cols * ny;  // scratch
+    float2* g = R.spec + (size_t)c0 * ny;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < count * ny; e += blockDim.x) { const float2 v = g[e]; S[e] = make_float2(v.x, inverse ? -v.y : v.y); }
     __syncthreads();
     FftPlan P{ny, R.fy_nf, R.fy_rad, R.twy};
-    float2* F = S;
-    if (whole) F = fft_rows_any(S, T, ny, nzc, P);
-    else fft_rows_grouped(S, T, ny, nzc, group, P);
-    float2* Fo = F == S ? T : S;       // the other buffer (whole slab case)
-    const TriAB* AB = (mode == PROJ_FACE ? R.tri_face : R.tri_pres) + (size_t)m * nzc * ny;
-    const double* Cc = reinterpret_cast<const double*>((mode == PROJ_FACE ? R.tri_face : R.tri_pres) + (size_t)R.nm * nzc * ny) + (size_t)m * nzc * ny;
-    // one FP64 recurrence per (n, real/imaginary part); values enter and leave FP64 through the integer-pipe
-    // conversions
-    float* Ff = reinterpret_cast<float*>(F);
-    for (int u = threadIdx.x; u < 2 * ny; u += blockDim.x) {
-      const int n = u >> 1, c = u & 1;
-      double d[MAXNZ];
-      double prev = 0;
-#pragma unroll 4
-      for (int k = 0; k < nzc; k++) {
-        const TriAB ab = AB[(size_t)k * ny + n];
-        prev = fma(-ab.b, prev, widen(__fmul_rn(ab.a, Ff[2 * (k * ny + n) + c])));
-        d[k] = prev;
-      }
-      double x = d[nzc - 1];
-      Ff[2 * ((nzc - 1) * ny + n) + c] = c ? -narrow(x) : narrow(x);
-#pragma unroll 4
-      for (int k = nzc - 2; k >= 0; k--) {
-        x = fma(-Cc[(size_t)k * ny + n], x, d[k]);
-        Ff[2 * (k * ny + n) + c] = c ? -narrow(x) : narrow(x);
-      }
-    }
-    __syncthreads();
-    const float2* G = F;
-    if (whole) G = fft_rows_any(F, Fo, ny, nzc, P);
-    else fft_rows_grouped(S, T, ny, nzc, group, P);
-    for (int e = threadIdx.x; e < nzc * ny; e += blockDim.x) { const float2 z = G[e]; g[e] = make_float2(z.x, -z.y); }
+    const float2* F = fft_rows_any(S, T, ny, count, P);
+    for (int e = threadIdx.x; e < count * ny; e += blockDim.x) { const float2 v = F[e]; g[e] = make_float2(v.x, inverse ? -v.y : v.y); }
     __syncthreads();
   }
 }
@@ -655,8 +611,8 @@ __global__ void k_proj_xifft(const RunDesc* __restrict__ runs, const int4* items
 
 
 // ---- the whole-layer path (grids whose layer spectrum fits in shared memory: the benchmark's 40x32 and 80x64):
-// the divergence kernel transforms each layer along x and y, the mode kernel is a pure FP64 sweep without
-// transforms or barriers, and the inverse kernel transforms back along y and x.
+// the divergence kernel transforms each layer along x and y, and the inverse kernel transforms back along y and x, with
+// the mode sweeps between them.
 
 // Builds the half spectrum X[m][y] (m <= nx/2) of the real rows held in pairs in Zf (spectral.ts:246-255).
 __device__ __forceinline__ void unpack_rows(const float2* Zf, float2* X, int nx, int ny, int rows, int nm) {
@@ -914,14 +870,20 @@ __global__ void __launch_bounds__(256, 5) k_proj_div_fft2(const RunDesc* __restr
   }
 }
 
-// One x-wavenumber m of one run per block, thread (n, real/imaginary): the FP64 sweeps of k_proj_modes on the 2-D
-// spectrum in place (the input and the output stay in global memory; no transform, no barrier).
-__global__ void k_proj_sweep(const RunDesc* __restrict__ runs, const int4* items, int nitems, int mode) {
+// One tridiagonal solve per mode along the vertical in FP64 on the 2-D spectrum in place (no transform, no barrier):
+// Thomas' algorithm with the LU factors made on the host in FP64 (the k = 0 uniform mode pinned at the ground, the null
+// modes zero): per level the forward sweep d_k = A_k r_k - B_k d_(k-1) and the back substitution x_k = d_k - C_k x_(k+1),
+// one real recurrence a thread (n, real/imaginary part), the two parts sharing the coefficients. FACE: rows -rho h lambda
+// + vertical faces (src/core/advection.ts:222-241); PRES: the density-weighted consistent Laplacian
+// (src/core/pressure.ts:104-140). Values enter and leave FP64 through the integer-pipe conversions. An x-wavenumber's
+// recurrences are split over blockIdx.y: nothing is shared between them, and blocks of two warps fill the SMs evenly.
+constexpr int SWEEP_THREADS = 64;
+__global__ void __launch_bounds__(SWEEP_THREADS) k_proj_sweep(const RunDesc* __restrict__ runs, const int4* items, int nitems, int mode) {
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
     const int m = items[it].y, ny = R.ny, nz = R.nz, nzc = mode == PROJ_FACE ? nz : nz - 1;
-    const int u = threadIdx.x;
+    const int u = blockIdx.y * SWEEP_THREADS + threadIdx.x;
     if (u >= 2 * ny) continue;
     const int n = u >> 1, c = u & 1;
     float* g = reinterpret_cast<float*>(R.spec + (size_t)m * nzc * ny) + c;
@@ -1806,13 +1768,8 @@ void launch_proj_div_xfft(const Launch& L, int mode, int set, int yc, int maxnx)
   size_t smem = (size_t)2 * ((yc + 1) / 2) * maxnx * sizeof(float2);
   k_proj_div_xfft<<<GRID(L.n, L.cap), 256, smem, L.stream>>>(L.runs, L.items, L.n, mode, set, yc);
 }
-void launch_proj_modes(const Launch& L, int mode, int maxnz, int maxny, int threads, int smem_budget) {
-  // the column slab [nz][ny] plus a scratch of `group` layers, all of them when they fit
-  const size_t slab = (size_t)maxnz * maxny * sizeof(float2);
-  int group = (int)std::min<size_t>(maxnz, (smem_budget - slab) / ((size_t)maxny * sizeof(float2)));
-  group = std::max(group, 1);
-  const size_t smem = slab + (size_t)group * maxny * sizeof(float2);
-  k_proj_modes<<<GRID(L.n, L.cap), threads, smem, L.stream>>>(L.runs, L.items, L.n, mode, group);
+void launch_proj_ycols(const Launch& L, int mode, int inverse, int points) {
+  k_proj_ycols<<<GRID(L.n, L.cap), 256, (size_t)2 * points * sizeof(float2), L.stream>>>(L.runs, L.items, L.n, mode, inverse);
 }
 size_t layer_fft_smem(int maxnx, int maxny) {
   return ((size_t)2 * ((maxny + 1) / 2) * maxnx + (size_t)2 * (maxnx / 2 + 1) * maxny + maxnx + maxny) * sizeof(float2);
@@ -1828,7 +1785,9 @@ void launch_proj_div_fft2(const Launch& L, int mode, int set, size_t smem) {
   k_proj_div_fft2<<<GRID(L.n, L.cap), 256, smem, L.stream>>>(L.runs, L.items, L.n, mode, set);
 }
 void launch_proj_sweep(const Launch& L, int mode, int maxny) {
-  k_proj_sweep<<<GRID(L.n, L.cap), (2 * maxny + 31) / 32 * 32, 0, L.stream>>>(L.runs, L.items, L.n, mode);
+  dim3 grid = GRID(L.n, L.cap);
+  grid.y = (2 * maxny + SWEEP_THREADS - 1) / SWEEP_THREADS;
+  k_proj_sweep<<<grid, SWEEP_THREADS, 0, L.stream>>>(L.runs, L.items, L.n, mode);
 }
 void launch_proj_ifft2(const Launch& L, int mode, size_t smem) {
   k_proj_ifft2<<<GRID(L.n, L.cap), 256, smem, L.stream>>>(L.runs, L.items, L.n, mode);
@@ -1885,7 +1844,7 @@ cudaError_t upload_tables() { return cudaMemcpyToSymbol(i2m::c_sweep, &i2m::h_sw
 
 cudaError_t set_smem_limits(int bytes) {
   cudaError_t e;
-  if ((e = smem_limit(k_proj_modes, bytes)) != cudaSuccess) return e;
+  if ((e = smem_limit(k_proj_ycols, bytes)) != cudaSuccess) return e;
   if ((e = smem_limit(k_proj_div_xfft, bytes)) != cudaSuccess) return e;
   if ((e = smem_limit(k_proj_xifft, bytes)) != cudaSuccess) return e;
   if ((e = smem_limit(k_sediment, bytes)) != cudaSuccess) return e;

@@ -25,7 +25,8 @@ void launch_theta_out(const Launch& L, float* dst);
 void launch_fall_courant(const Launch& L);
 void launch_sediment(const Launch& L, int maxnz);
 void launch_proj_div_xfft(const Launch& L, int mode, int set, int yc, int maxnx);
-void launch_proj_modes(const Launch& L, int mode, int maxnz, int maxny, int threads, int smem_budget);
+// The row path's y-transforms on items of `points` = columns x ny values at most.
+void launch_proj_ycols(const Launch& L, int mode, int inverse, int points);
 // The whole-layer path: 2-D transforms per layer, FP64 sweeps per (m, n) in global memory.
 size_t layer_fft_smem(int maxnx, int maxny);
 size_t layer_fft_smem_run(int nx, int ny);  // the layer transforms' shared memory for one run's grid

@@ -89,6 +89,7 @@ struct Plan {
   int refTX = 16, refTY = 8;                                          // refinement tile
   bool layerAny = false, rowAny = false;                              // some run takes the 2-D layer transforms / the row path
   int rowMaxnx = 0, rowMaxny = 0;                                     // the widest grid of the row path
+  int ycolPoints = 0;                                                 // its y-transform items' values at most
   size_t fftSmem = 0;                                                 // their shared memory: the largest over the runs
   bool refine = false;                                                // some run refines its final projection
   bool unrefined = false;                                             // some run does not (k_pres_correct<1> has work)
@@ -106,7 +107,7 @@ struct Plan {
   }
 };
 enum Family { FAM_NODE, FAM_COLS, FAM_ROWS_FACE, FAM_ROWS_PRES, FAM_MODES, FAM_RUNS, FAM_CELLS, FAM_T_WENO, FAM_T_DYN, FAM_MIX,
-              FAM_REFINE, FAM_T_CHG, FAM_T_CHG3, FAM_PHYS, FAM_PHYS_LAST = FAM_PHYS + 5, FAM_FILL, FAM_LROWS_FACE, FAM_LROWS_PRES, FAM_LMODES, FAM_COUNT };
+              FAM_REFINE, FAM_T_CHG, FAM_T_CHG3, FAM_PHYS, FAM_PHYS_LAST = FAM_PHYS + 5, FAM_FILL, FAM_YCOLS, FAM_LROWS_FACE, FAM_LROWS_PRES, FAM_LMODES, FAM_COUNT };
 
 }  // namespace
 
@@ -327,7 +328,7 @@ int validate(sg_context* ctx, const sg_grid* g, const sg_base_state* b, const sg
   if (!sw->pressure_in_stages) return fail(ctx, SG_ERR_UNSUPPORTED, "the device step needs the pressure in the RK3 stages");
   // the lightning's potential solve holds a row, a column and a half spectrum of a level in shared memory
   if (sw->lightning && sw->ice && (g->nx > 2048 || g->ny > 2048)) return fail(ctx, SG_ERR_UNSUPPORTED, "lightning: nx and ny at most 2048");
-  // The shared memory of the mode kernel: (nz + 8) * ny complex values.
+  // the row path's limit on a wavenumber's slab, (nz + 8) * ny complex values
   size_t smem = (size_t)(g->nz + 8) * g->ny * 8;
   if ((int)smem > ctx->maxSmem) return fail(ctx, SG_ERR_UNSUPPORTED, "(nz + 8) * ny too large for one block's shared memory");
   return SG_OK;
@@ -408,8 +409,8 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, Plan& P) {
   P.TY = 8;
   P.wenoG = 3;
   // Spectral solves, chosen run by run (so a run's bits do not depend on its batch): when a layer's spectrum fits in
-  // shared memory (the 40x32 and 80x64 grids), whole layers are transformed in 2-D and the mode kernel is a pure FP64
-  // sweep; otherwise rows of 16 or 32 are x-transformed and the mode kernel transforms along y around its sweep.
+  // shared memory (the 40x32 and 80x64 grids), whole layers are transformed in 2-D; otherwise rows of 16 or 32 are
+  // x-transformed and columns of the spectrum y-transformed before and after the sweeps.
   auto layerPath = [&](const Run& r) { return !ctx->rowsOnly && layer_fft_smem(r.nx, r.ny) <= (size_t)std::min(ctx->maxSmem, 100 * 1024); };
   for (int s : slots) {
     const Run& r = ctx->runs[s];
@@ -437,6 +438,10 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, Plan& P) {
       for (int k = 0; k < r.nz; k++) for (int y = 0; y < r.ny; y += P.yc) all[FAM_ROWS_FACE].push_back(make_int4(s, k, y, 0));
       for (int k = 0; k < r.nz - 1; k++) for (int y = 0; y < r.ny; y += P.yc) all[FAM_ROWS_PRES].push_back(make_int4(s, k, y, 0));
       for (int m = 0; m < r.nx / 2 + 1; m++) all[FAM_MODES].push_back(make_int4(s, m, 0, 0));
+      // the y-transforms' columns (x-wavenumber, layer): about 2048 points an item
+      const int columns = (r.nx / 2 + 1) * r.nz, per = std::max(1, 2048 / r.ny);
+      P.ycolPoints = std::max(P.ycolPoints, per * r.ny);
+      for (int c = 0; c * per < columns; c++) all[FAM_YCOLS].push_back(make_int4(s, c, per, 0));
     }
     all[FAM_RUNS].push_back(make_int4(s, 0, 0, 0));
     if (r.desc.flags & RF_REFINE) P.refine = true; else P.unrefined = true;
@@ -594,10 +599,12 @@ void enqueue_solve(sg_context* ctx, const Plan& P, int mode, int set, cudaStream
     rows.cap = rows.n;
     modes.cap = modes.n;
     rows.stream = modes.stream = stream;
-    const int mthreads = std::min(512, std::max(64, (2 * P.rowMaxny + 31) / 32 * 32));
-    const int mbudget = std::min(ctx->maxSmem, 200 * 1024);
+    Launch cols = lx(ctx, P, FAM_YCOLS);
+    cols.cap = cols.n; cols.stream = stream;
     launch_proj_div_xfft(rows, mode, set, P.yc, P.rowMaxnx); hook(h);
-    launch_proj_modes(modes, mode, P.maxnz, P.rowMaxny, mthreads, mbudget); hook(h + 1);
+    launch_proj_ycols(cols, mode, 0, P.ycolPoints);
+    launch_proj_sweep(modes, mode, P.rowMaxny);
+    launch_proj_ycols(cols, mode, 1, P.ycolPoints); hook(h + 1);
     launch_proj_xifft(rows, mode, P.yc, P.rowMaxnx); hook(h + 2);
   }
 }
