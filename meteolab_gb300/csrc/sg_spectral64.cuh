@@ -28,7 +28,8 @@ __device__ __forceinline__ double2 z_sub(double2 a, double2 b) { return make_dou
 // a times the conjugate of w (the tables hold exp(+2 pi i t / n), the forward transform turns by the conjugates)
 __device__ __forceinline__ double2 z_turn(double2 a, double2 w) { return make_double2(fma(a.x, w.x, a.y * w.y), fma(a.y, w.x, -(a.x * w.y))); }
 
-// One butterfly of a self-sorting (Stockham) stage: j in [0, n / r), Ns the product of the radices already applied.
+// One butterfly of a self-sorting (Stockham) stage of radix 4, 2, 3 or 5: j in [0, n / r), Ns the product of the radices
+// already applied.
 __device__ __forceinline__ void fft64_butterfly(const double2* x, double2* y, int n, int r, int Ns, int j, const double2* __restrict__ tw) {
   const int nb = n / r, k = j % Ns, t = k * (n / (Ns * r)), out = (j / Ns) * Ns * r + k;
   const bool turn = Ns > 1;  // (the first stage's turns are all 1)
@@ -68,18 +69,44 @@ __device__ __forceinline__ void fft64_butterfly(const double2* x, double2* y, in
     y[out + 4 * Ns] = make_double2(a.x - e.y, a.y + e.x);
     y[out + 2 * Ns] = make_double2(b.x + f.y, b.y - f.x);
     y[out + 3 * Ns] = make_double2(b.x - f.y, b.y + f.x);
-  } else {
-    const int base = n / r;  // exp(2 pi i / r) = tw[n / r]
-    for (int q1 = 0; q1 < r; q1++) {
-      double2 acc = x[j];
-      for (int q = 1; q < r; q++) {
-        int at = q * t + (int)((long long)q * q1 % r) * base;  // (both turns in one: below 2 n)
-        if (at >= n) at -= n;
-        acc = z_add(acc, z_turn(x[j + q * nb], tw[at]));
-      }
-      y[out + q1 * Ns] = acc;
-    }
   }
+}
+
+// A stage of any other (odd prime) radix r, over all rows: the turned inputs' sums and differences s_q = v_q + v_(r-q),
+// d_q = v_q - v_(r-q) take their places, then a thread forms the outputs k and r - k together from
+// v_0 + sum s_q cos(2 pi q k / r) and sum d_q sin(2 pi q k / r): r - 1 FMAs an output, a quarter of a direct sum's.
+__device__ __forceinline__ void fft64_prime_stage(double2* a, double2* b, int rows, int n, int r, int Ns, const double2* __restrict__ tw) {
+  const int nb = n / r, h = r / 2, step = n / (Ns * r);
+  for (int u = threadIdx.x; u < rows * h * nb; u += blockDim.x) {
+    const int row = u / (h * nb), e = u - row * h * nb, q = 1 + e / nb, j = e - (q - 1) * nb, t = (j % Ns) * step;
+    double2 *x = a + row * n + j + q * nb, *y = a + row * n + j + (r - q) * nb;
+    double2 v = *x, w = *y;
+    if (Ns > 1) { v = z_turn(v, tw[q * t]); w = z_turn(w, tw[(r - q) * t]); }
+    *x = z_add(v, w); *y = z_sub(v, w);
+  }
+  __syncthreads();
+  for (int u = threadIdx.x; u < rows * (h + 1) * nb; u += blockDim.x) {
+    const int row = u / ((h + 1) * nb), e = u - row * (h + 1) * nb, k = e / nb, j = e - k * nb, out = (j / Ns) * Ns * r + j % Ns;
+    const double2* x = a + row * n + j;
+    double2* y = b + row * n + out;
+    double2 A = x[0], B = make_double2(0, 0);
+    if (k == 0) {
+      for (int q = 1; q <= h; q++) A = z_add(A, x[q * nb]);
+      y[0] = A;
+      continue;
+    }
+    int at = 0;
+    for (int q = 1; q <= h; q++) {
+      at += k;
+      if (at >= r) at -= r;
+      const double2 w = tw[at * nb], sq = x[q * nb], dq = x[(r - q) * nb];  // exp(2 pi i q k / r)
+      A = make_double2(fma(sq.x, w.x, A.x), fma(sq.y, w.x, A.y));
+      B = make_double2(fma(dq.x, w.y, B.x), fma(dq.y, w.y, B.y));
+    }
+    y[k * Ns] = make_double2(A.x + B.y, A.y - B.x);
+    y[(r - k) * Ns] = make_double2(A.x - B.y, A.y + B.x);
+  }
+  __syncthreads();
 }
 
 // Forward transforms of `rows` rows of P.n values in shared memory, between a and b; returns the buffer with the result.
@@ -88,11 +115,14 @@ __device__ __forceinline__ double2* fft64_rows(double2* a, double2* b, int rows,
   int Ns = 1;
   for (int s = 0; s < P.nf; s++) {
     const int r = P.rad[s], nb = P.n / r, total = rows * nb;
-    for (int u = threadIdx.x; u < total; u += blockDim.x) {
-      const int row = u / nb, j = u - row * nb;
-      fft64_butterfly(a + row * P.n, b + row * P.n, P.n, r, Ns, j, tw);
+    if (r > 5) fft64_prime_stage(a, b, rows, P.n, r, Ns, tw);
+    else {
+      for (int u = threadIdx.x; u < total; u += blockDim.x) {
+        const int row = u / nb, j = u - row * nb;
+        fft64_butterfly(a + row * P.n, b + row * P.n, P.n, r, Ns, j, tw);
+      }
+      __syncthreads();
     }
-    __syncthreads();
     double2* t = a; a = b; b = t;
     Ns *= r;
   }
