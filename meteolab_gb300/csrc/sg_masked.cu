@@ -14,7 +14,8 @@
 // sweeps and y-inverse (sg_spectral64.cuh), and its x-inverse with r.z. Each dot product is finished, and acted on, by
 // the block that ends last, from the partials in a fixed order (the result does not depend on scheduling); alpha, beta
 // and the stopping test stay on the device. Eight iterations are one CUDA graph,
-// replayed until the device's stop flag is set: the host reads one int per eight iterations; every kernel of an
+// replayed until the device's stop flag is set: the host reads one int per eight iterations (a projection whose rounding
+// would decide its iterations starts again in the reference's order of operations: sg_masked_ordered.cu); every kernel of an
 // iteration after the stop returns at once, so the iterations done, the residual and the result are those
 // of the reference's loop (:313-329), which stops at the first top-of-loop test it passes. The FP64 pipe bounds the
 // kernels (two operations a clock and SM), so their FP64 instructions are counted: see k_mp_flux and sg_spectral64.cuh.
@@ -25,6 +26,7 @@
 #include <string>
 #include <vector>
 #include "sg_kernels.h"
+#include "sg_masked_ordered.cuh"
 #include "sg_spectral64.cuh"
 #include "stormgpu.h"
 
@@ -151,12 +153,12 @@ void slope_area(const HostGrid& g, const float* h, float* area) {
 // ---------------------------------------------------------------- device
 
 // The solve's scalars on the device. done: 0 iterating, 1 stopped (converged, no descent, or out of iterations),
-// 2 a zero right-hand side (nothing to project).
+// 2 a zero right-hand side (nothing to project), 4 the residuals have lost their orthogonality (see k_mp_xinv).
 struct MpState {
-  double bb, tol2bb, rz, rr, alpha, beta, tolerance;
+  double bb, tol2bb, rz, rr, rz0, alpha, beta, tolerance;
   int k, done, maxIt, keepRR;
 };
-enum { STOP = 1, ZERO = 2, ANY = 3 };
+enum { STOP = 1, ZERO = 2, DRIFT = 4, ANY = 7 };
 enum { R_BB, R_RR0, R_RZ0, R_DSD, R_RR, R_RZN };
 
 struct Geo {
@@ -195,24 +197,40 @@ __global__ void k_mp_mask(float* __restrict__ u, float* __restrict__ v, float* _
 
 // Adds a dot product's block sums and acts on it in the block that finishes last (a counter; no block waits): the
 // partials in a fixed order, so the result does not depend on which block that is (the scalars of :306-329).
-template <int OP>
-__device__ __forceinline__ void finish_dot(double dot, double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st) {
+// WATCH: with a second sum, r . z0.
+template <int OP, bool WATCH = false>
+__device__ __forceinline__ void finish_dot(double dot, double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st,
+                                           double dot0 = 0) {
   __shared__ double sh[32];
   __shared__ bool last;
   const int id = blockIdx.y * gridDim.x + blockIdx.x, nparts = gridDim.x * gridDim.y;
   const double mine = block_sum(dot, sh);
+  double mine0 = 0;
+  if (WATCH) {
+    __syncthreads();  // (sh is read by the first sum's warp)
+    mine0 = block_sum(dot0, sh);
+  }
   if (threadIdx.x == 0) {
     part[id] = mine;
+    if (WATCH) part[nparts + id] = mine0;
     __threadfence();
     last = atomicAdd(arrived, 1u) == (unsigned)nparts - 1u;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double v = 0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += __ldcg(part + i);
+  double v = 0, v0 = 0;
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
+    v += __ldcg(part + i);
+    if (WATCH) v0 += __ldcg(part + nparts + i);
+  }
   __syncthreads();  // (sh is read by the first sum's warp)
   const double s = block_sum(v, sh);
+  double s0 = 0;
+  if (WATCH) {
+    __syncthreads();
+    s0 = block_sum(v0, sh);
+  }
   if (threadIdx.x != 0) return;
   *arrived = 0;
   if (OP == R_BB) {
@@ -221,7 +239,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ part
   } else if (OP == R_RR0) {  // the first guess's residual: the first top-of-loop test
     if (st->maxIt > 0) { st->rr = s; if (s <= st->tol2bb) st->done = STOP; }
   } else if (OP == R_RZ0) {
-    st->rz = s;
+    st->rz = st->rz0 = s;
     if (st->maxIt <= 0 || (st->keepRR && !(st->rr > st->tol2bb))) st->done |= STOP;
   } else if (OP == R_DSD) {
     if (!(s > 0)) st->done = STOP;
@@ -240,6 +258,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ part
   } else {
     st->beta = s / st->rz; st->rz = s; st->k++;
     if (st->k >= st->maxIt) st->done = STOP;
+    if (WATCH && s0 * s0 > 1e-18 * st->rz0 * fmax(s, 1e-10 * st->rz0)) st->done = DRIFT;
   }
 }
 
@@ -336,6 +355,28 @@ __global__ void __launch_bounds__(TPB) k_mp_div(const double* __restrict__ fu, c
   if (DOT == 2) finish_dot<R_BB>(dot, part, arrived, st);
 }
 
+// What the iterations here take from the reference's tables, once a plan: the sweep's 1 / pivot (with the transforms'
+// factor) and lower / pivot, zero for the modes with an infinite pivot (which are left with a pivot of 1 and its
+// reciprocal of 0: OrderedSolve), the columns' shares of the fluxes, zero where a layer's upper half is shut, and the nodes' weights of w.
+__global__ void k_mp_tables(double* __restrict__ piv, double* __restrict__ rpiv, const double* __restrict__ lo, double* __restrict__ a,
+                            double* __restrict__ b, double factor, size_t spec, const double* __restrict__ low, const double* __restrict__ high,
+                            double* __restrict__ A, double* __restrict__ B, double* __restrict__ wMass, Geo g) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < spec) {
+    const double p = piv[i], ip = isinf(p) ? 0 : 1 / p;
+    if (ip == 0) piv[i] = 1;
+    rpiv[i] = ip; a[i] = factor * ip; b[i] = lo[i] * ip;
+  }
+  if (i < g.cells) {
+    const int k = (int)(i / g.layer);
+    const double lw = low[i], hi = high[i];
+    const bool solid = g.solid[i] != 0;
+    A[i] = hi > 0 && !solid ? g.rho4[k] * lw : 0;
+    B[i] = hi > 0 ? g.rho4[k + 1] * (hi + (solid ? lw : 0)) : 0;
+  }
+  if (i < g.n) wMass[i] = g.wall[i] || i < (size_t)g.layer || i >= g.n - g.layer ? 0 : g.rho4[i / g.layer] * g.invMass[i];
+}
+
 // The first guess q = V phi from the last pressure (:311).
 __global__ void k_mp_start(const double* __restrict__ p, double* __restrict__ q, double dt, Geo g, const MpState* __restrict__ st) {
   if (st->done & ZERO) return;
@@ -383,10 +424,19 @@ __global__ void k_mp_update_xfwd(double* __restrict__ q, double* __restrict__ r,
 
 // The preconditioner's x inverse: z = the plain solution (the face solve's), or with dzs V phi, zero in the dropped cells
 // (:355), and the sum r . z (OP: what it is for).
-template <int OP>
+//
+// WATCH: with r . z0, z0 the first z, which conjugate gradients keep at zero. Rounding makes it grow (over steep ground,
+// where a column's open shares are small, by a factor of ten in some iterations), and what it has grown to says how far
+// rounding has come to decide the iterations (Paige 1976): over 220 solves on drawn grounds and grids, disturbed in the
+// last bit, those with |r . z0| below 1e-9 of sqrt(r.z r0.z0) throughout agreed to 6e-13, of the others nine in ten to no
+// better than 1e-10 and half to no better than 1e-6. A solve that passes 1e-9 (or 1e-14 r0.z0, which r.z alone would be
+// compared with at tighter tolerances) stops, and starts again in the reference's order of operations (OrderedSolve).
+// An iteration there takes 0.39 ms on 80 x 64 x 50 nodes, 0.11 here; what is given up took a quarter of the iterations.
+template <int OP, bool WATCH = false>
 __global__ void k_mp_xinv(const double2* __restrict__ S, double* __restrict__ out, const double* __restrict__ r, int nx, int ny, int pairs, Fft64 P,
                           const double2* __restrict__ tw, const double* __restrict__ dzs, const uint8_t* __restrict__ dropped,
-                          double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st, int skip) {
+                          double* __restrict__ part, unsigned* __restrict__ arrived, MpState* __restrict__ st, int skip,
+                          const double* __restrict__ z0 = nullptr) {
   extern __shared__ double2 z64[];
   if (st->done & skip) return;
   const int k = blockIdx.y, y0 = blockIdx.x * 2 * pairs, rows = min(2 * pairs, ny - y0);
@@ -395,16 +445,18 @@ __global__ void k_mp_xinv(const double2* __restrict__ S, double* __restrict__ ou
   const double2* Z = fft64_rows(z64, z64 + pairs * nx, (rows + 1) / 2, P, tw);
   const size_t base = (size_t)k * nx * ny + (size_t)y0 * nx;
   const double h = dzs ? dzs[k] : 1;
-  double dot = 0;
+  double dot = 0, dot0 = 0;
   for (int e = threadIdx.x; e < rows * nx; e += blockDim.x) {
     const int row = e / nx, x = e - row * nx;
     const double2 v = Z[(row >> 1) * nx + x];
     double val = row & 1 ? -v.y : v.x;
     if (dzs) val = dropped[base + e] ? 0 : val * h;
-    dot = fma(r[base + e], val, dot);
+    const double re = r[base + e];
+    dot = fma(re, val, dot);
+    if (WATCH) dot0 = fma(re, z0[base + e], dot0);
     out[base + e] = val;
   }
-  finish_dot<OP>(dot, part, arrived, st);
+  finish_dot<OP, WATCH>(dot, part, arrived, st, dot0);
 }
 
 // The potential phi = q / V and the pressure kept, phi / dt (:332).
@@ -581,7 +633,7 @@ int blocks(size_t count) { return (int)((count + TPB - 1) / TPB); }
 // Shared memory beyond 48 KB for rows of more than 1536 points.
 cudaError_t solve_limits() {
   cudaError_t e = spectral64_limits();
-  for (const void* k : {(const void*)k_mp_update_xfwd, (const void*)k_mp_xinv<R_RZ0>, (const void*)k_mp_xinv<R_RZN>})
+  for (const void* k : {(const void*)k_mp_update_xfwd, (const void*)k_mp_xinv<R_RZ0>, (const void*)k_mp_xinv<R_RZN>, (const void*)k_mp_xinv<R_RZN, true>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SPECTRAL64_SMEM);
   return e;
 }
@@ -601,12 +653,13 @@ struct sg_masked {
   char* mem = nullptr;
   float *u = nullptr, *v = nullptr, *w = nullptr;
   double *p = nullptr, *b = nullptr, *q = nullptr, *r = nullptr, *z = nullptr, *d[2] = {}, *sd = nullptr, *fu = nullptr, *fv = nullptr,
-         *fw = nullptr, *part = nullptr;
+         *fw = nullptr, *z0 = nullptr, *part = nullptr;
   unsigned* arrived = nullptr;
   Spectral64 sp;
+  OrderedSolve ordered{};
   MpState* st = nullptr;
   std::vector<uint8_t> dropped;
-  cudaGraphExec_t chunk = nullptr;
+  cudaGraphExec_t chunk = nullptr, orderedChunk = nullptr;
   int iterations = 0;
   double residual = 0;
 };
@@ -633,20 +686,20 @@ namespace {
 constexpr int REPLAY = 8;
 
 // The preconditioner's x-inverse into z with r . z, on the shape of a solve.
-template <int OP>
+template <int OP, bool WATCH = false>
 void enqueue_xinv(const Spectral64& S, double* z, const double* r, const double* dzs, const uint8_t* dropped, double* part, unsigned* arrived,
-                  MpState* st, int skip, cudaStream_t s) {
-  k_mp_xinv<OP><<<dim3(S.x.groups, S.levels), S.x.threads, S.x.smem, s>>>(S.S, z, r, S.nx, S.ny, S.x.pairs, S.px, S.twx, dzs, dropped, part, arrived, st, skip);
+                  MpState* st, int skip, cudaStream_t s, const double* z0 = nullptr) {
+  k_mp_xinv<OP, WATCH><<<dim3(S.x.groups, S.levels), S.x.threads, S.x.smem, s>>>(S.S, z, r, S.nx, S.ny, S.x.pairs, S.px, S.twx, dzs, dropped, part, arrived, st, skip, z0);
 }
 // The preconditioner after the x-transform of r: the flat solve of -r (:351-356; the face solve's flatSolve,
 // advection.ts:179-184, whose right-hand side over and back times each level's height is -r too).
-template <int OP>
+template <int OP, bool WATCH = false>
 void enqueue_precondition(const Spectral64& S, double* z, const double* r, const double* dzs, const uint8_t* dropped, double* part, unsigned* arrived,
-                          MpState* st, int skip, cudaStream_t s) {
+                          MpState* st, int skip, cudaStream_t s, const double* z0 = nullptr) {
   S.forward_y(s, &st->done, skip);
   S.sweep(s, 1, &st->done, skip);
   S.inverse_y(s, &st->done, skip);
-  enqueue_xinv<OP>(S, z, r, dzs, dropped, part, arrived, st, skip, s);
+  enqueue_xinv<OP, WATCH>(S, z, r, dzs, dropped, part, arrived, st, skip, s, z0);
 }
 // The start's: the x-transform of r as it stands, then the same.
 void enqueue_first_precondition(const Spectral64& S, double* z, const double* r, const double* dzs, const uint8_t* dropped, double* part,
@@ -654,18 +707,19 @@ void enqueue_first_precondition(const Spectral64& S, double* z, const double* r,
   S.forward_x(r, s, &st->done, ANY);
   enqueue_precondition<R_RZ0>(S, z, r, dzs, dropped, part, arrived, st, ANY, s);
 }
-// The end of an iteration from S d on: the update with its x-transform, the preconditioner.
+// The end of an iteration from S d on: the update with its x-transform, the preconditioner (WATCH: with its watch on z0).
+template <bool WATCH>
 void enqueue_descent(const Spectral64& S, double* q, double* r, double* z, const double* d, const double* sd, const double* dzs, const uint8_t* dropped,
-                     double* part, unsigned* arrived, MpState* st, cudaStream_t s) {
+                     double* part, unsigned* arrived, MpState* st, cudaStream_t s, const double* z0 = nullptr) {
   k_mp_update_xfwd<<<dim3(S.x.groups, S.levels), S.x.threads, S.x.smem, s>>>(q, r, d, sd, S.S, S.nx, S.ny, S.x.pairs, S.px, S.twx, part, arrived, st);
-  enqueue_precondition<R_RZN>(S, z, r, dzs, dropped, part, arrived, st, ANY, s);
+  enqueue_precondition<R_RZN, WATCH>(S, z, r, dzs, dropped, part, arrived, st, ANY, s, z0);
 }
 
 // One iteration of setVelocityMasked's loop (:127-145); `odd`: which of the two direction buffers is the last one's.
 void enqueue_face_iteration(sg_faces* f, int odd, cudaStream_t s) {
   double *last = f->d[odd], *next = f->d[odd ^ 1];
   k_tm_apply<<<blocks(f->fg.n), TPB, 0, s>>>(last, f->z, next, f->sd, f->part, f->arrived, f->fg, f->st);
-  enqueue_descent(f->sp, f->q, f->r, f->z, next, f->sd, nullptr, nullptr, f->part, f->arrived, f->st, s);
+  enqueue_descent<false>(f->sp, f->q, f->r, f->z, next, f->sd, nullptr, nullptr, f->part, f->arrived, f->st, s);
 }
 
 // The fluxes of a cell vector's gradient (of z + beta d where dn is given).
@@ -683,7 +737,7 @@ void enqueue_iteration(sg_masked* m, int odd, cudaStream_t s) {
   double *last = m->d[odd], *next = m->d[odd ^ 1];
   enqueue_flux(m, last, m->z, next, ANY, s);
   k_mp_div<1><<<blocks(g.cells), TPB, 0, s>>>(m->fu, m->fv, m->fw, m->sd, next, 1 / (g.dx * g.dx), 1 / (g.dy * g.dy), m->part, m->arrived, g, m->st, ANY);
-  enqueue_descent(m->sp, m->q, m->r, m->z, next, m->sd, g.dzs, g.dropped, m->part, m->arrived, m->st, s);
+  enqueue_descent<true>(m->sp, m->q, m->r, m->z, next, m->sd, g.dzs, g.dropped, m->part, m->arrived, m->st, s, m->z0);
 }
 
 int fail(sg_masked* m, const char* what, cudaError_t e) {
@@ -744,12 +798,11 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
   Spectral64 sp;
   sp.shape(nx, ny, nc);
 
-  // The constructor (:190-218): solid and wall nodes, 1 / (rho0 hn), dropped cells, and as k_mp_flux takes them the
-  // columns' shares of each cell layer's fluxes (of the layer's half below its middle and above it that are above the
-  // ground) and the nodes' weights.
-  std::vector<uint8_t> solid(n), wall(n, 0), blocked(cells), dropped(cells);
+  // The constructor (:190-218): solid and wall nodes, 1 / (rho0 hn), the columns' shares of each
+  // cell layer (of its half below the middle and above it that are above the ground), dropped cells.
+  std::vector<uint8_t> solid(n), wall(n, 0), dropped(cells);
   std::vector<int32_t> levels(layer);
-  std::vector<double> heights(n), inv(n, 0.0), wm(n, 0.0), sa(cells), sb(cells), rho4(nz), idz(nz, 0.0);
+  std::vector<double> heights(n), inv(n, 0.0), low(cells), high(cells), rho4(nz), idz(nz, 0.0);
   solid_levels(g, ground, solid.data(), levels.data());
   node_heights(g, solid.data(), levels.data(), ground, heights.data());
   bool any = false;
@@ -758,38 +811,39 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
   for (int k = 0; k < nz; k++) rho4[k] = rho[k] / 4;
   for (int k = 0; k < nc; k++) idz[k] = 1 / g.dzs[k];
   for (int k = 0; k < nz; k++) {
-    const double r = rho[k], r4 = k > 0 && k < nz - 1 ? rho4[k] : 0;
+    const double r = rho[k];
     for (int c = 0; c < layer; c++) {
       const size_t i = c + (size_t)k * layer;
       if (solid[i]) continue;
       inv[i] = 1 / (r * heights[i]);
-      if (g.zs[k] <= (double)ground[c]) wall[i] = 1; else wm[i] = r4 * inv[i];
+      if (g.zs[k] <= (double)ground[c]) wall[i] = 1;
     }
   }
   for (int k = 0; k < nc; k++) {
-    const double half = g.dzs[k] / 2, middle = g.zs[k] + half, per = 1 / half;
+    const double half = g.dzs[k] / 2, middle = g.zs[k] + half;
     for (int c = 0; c < layer; c++) {
       const size_t at = c + (size_t)k * layer;
       const double h = (double)ground[c];
-      const double low = std::min(1.0, std::max(0.0, (middle - std::max(h, g.zs[k])) * per));
-      const double high = std::min(1.0, std::max(0.0, (g.zs[k + 1] - std::max(h, middle)) * per));
-      blocked[at] = high == 0;
-      sa[at] = high > 0 && !solid[at] ? rho4[k] * low : 0;
-      sb[at] = high > 0 ? rho4[k + 1] * (high + (solid[at] ? low : 0)) : 0;
+      low[at] = std::min(1.0, std::max(0.0, (middle - std::max(h, g.zs[k])) / half));
+      high[at] = std::min(1.0, std::max(0.0, (g.zs[k + 1] - std::max(h, middle)) / half));
     }
   }
   for (int k = 0; k < nc; k++)
     for (int j = 0; j < ny; j++) {
-      const uint8_t *b0 = blocked.data() + (size_t)k * layer + (size_t)j * nx, *b1 = blocked.data() + (size_t)k * layer + (size_t)((j + 1) % ny) * nx;
+      const double *b0 = high.data() + (size_t)k * layer + (size_t)j * nx, *b1 = high.data() + (size_t)k * layer + (size_t)((j + 1) % ny) * nx;
       uint8_t* out = dropped.data() + (size_t)k * layer + (size_t)j * nx;
-      for (int i = 0; i < nx; i++) { const int i1 = i + 1 == nx ? 0 : i + 1; out[i] = b0[i] & b0[i1] & b1[i] & b1[i1]; }
+      for (int i = 0; i < nx; i++) {
+        const int i1 = i + 1 == nx ? 0 : i + 1;
+        out[i] = b0[i] == 0 && b0[i1] == 0 && b1[i] == 0 && b1[i1] == 0;
+      }
     }
 
-  // The flat solve's rows per mode (pressure.ts:36-44, :118-140) as the sweep takes them: a = 1 / pivot (with the
-  // transforms' factor), b = lower / pivot and c = upper / pivot of each cell layer in the reference's elimination order.
-  // Modes it zeroes and the uniform mode's pinned lowest cell have a and b zero (their values come out zero).
-  const double factor = sp.factor();
-  std::vector<double> ta(spec, 0.0), tb(spec, 0.0), tcp(spec, 0.0);
+  // The flat solve's rows per mode (pressure.ts:36-44, :118-140): lower coefficient, pivot and cp = up / pivot of each
+  // cell layer in the reference's elimination order. Modes it zeroes and the uniform mode's pinned lowest cell get an
+  // infinite pivot (their values come out zero).
+  std::vector<double> tlo(spec, 0.0), tcp(spec, 0.0), tpiv(spec, 0.0);
+  std::vector<double> own(nc);
+  for (int k = 0; k < nc; k++) own[k] = rho[k] * g.dzs[k] / (2 * g.hz[k]) + rho[k + 1] * g.dzs[k] / (2 * g.hz[k + 1]);
   auto exact = [](double x) { return x < 1e-12 ? 0 : x > 1 - 1e-12 ? 1 : x; };
   for (int m = 0; m <= mh; m++)
     for (int q = 0; q < ny; q++) {
@@ -797,20 +851,23 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
       const double sy = exact(std::pow(std::sin(PI_ * q / ny), 2)), cy = exact(std::pow(std::cos(PI_ * q / ny), 2));
       const double a = 4 * (sx * cy / (g.dx * g.dx) + cx * sy / (g.dy * g.dy)), b = cx * cy;
       const size_t mode = (size_t)m * ny + q;
-      if ((a == 0 && b == 0) || (nc == 1 && a == 0)) continue;
+      if ((a == 0 && b == 0) || (nc == 1 && a == 0)) {
+        for (int k = 0; k < nc; k++) tpiv[(size_t)k * modes + mode] = INFINITY;
+        continue;
+      }
       const bool pinned = a == 0;
       double cprev = 0;
       for (int k = 0; k < nc; k++) {
-        double di = -a / 2 * (rho[k] * g.dzs[k] / (2 * g.hz[k]) + rho[k + 1] * g.dzs[k] / (2 * g.hz[k + 1])), lo = 0, up = 0;
+        double di = -a / 2 * own[k], lo = 0, up = 0;
         if (k > 0) { lo = -a / 2 * rho[k] * g.dzs[k - 1] / (2 * g.hz[k]); const double v = b * rho[k] / (g.hz[k] * g.dzs[k]); lo += v; di -= v; }
         if (k < nc - 1) { up = -a / 2 * rho[k + 1] * g.dzs[k + 1] / (2 * g.hz[k + 1]); const double v = b * rho[k + 1] / (g.hz[k + 1] * g.dzs[k]); up += v; di -= v; }
         bool zero = false;
         if (pinned && k == 0) { lo = 0; di = 1; up = 0; zero = true; }
         if (pinned && k == 1) lo = 0;
-        const double ip = 1 / (k == 0 ? di : di - lo * cprev);
-        cprev = up * ip;
+        const double piv = k == 0 ? di : di - lo * cprev;
+        cprev = up / piv;
         const size_t at = (size_t)k * modes + mode;
-        ta[at] = zero ? 0 : factor * ip; tb[at] = zero ? 0 : lo * ip; tcp[at] = cprev;
+        tlo[at] = lo; tcp[at] = cprev; tpiv[at] = zero ? INFINITY : piv;
       }
     }
   std::vector<double2> tx(nx), ty(ny);
@@ -819,12 +876,13 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
 
   // One allocation, 256-byte aligned parts.
   auto al = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-  const size_t nparts = std::max((size_t)blocks(cells), (size_t)sp.x.groups * nc);
+  const size_t nparts = std::max({(size_t)blocks(cells), 2 * (size_t)sp.x.groups * nc, (size_t)ny * nc});  // (two sums a group: the watch)
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += al(bytes); return o; };
   const size_t oU = take(n * 4), oV = take(n * 4), oW = take(n * 4), oP = take(cells * 8), oB = take(cells * 8), oQ = take(cells * 8), oR = take(cells * 8),
-               oZ = take(cells * 8), oD = take(cells * 8), oD2 = take(cells * 8), oSd = take(cells * 8), oFu = take(cells * 8), oFv = take(cells * 8),
-               oFw = take(cells * 8), oPart = take(nparts * 8), oA = take(spec * 8), oBb = take(spec * 8), oC = take(spec * 8), oS = take(spec * 16),
+               oZ = take(cells * 8), oD = take(cells * 8), oD2 = take(cells * 8), oSd = take(cells * 8), oFu = take(n * 8), oFv = take(n * 8),
+               oFw = take(n * 8), oPart = take(nparts * 8), oLo = take(spec * 8), oPv = take(spec * 8),
+               oRpv = take(spec * 8), oS1 = take(spec * 16), oLow = oQ, oHigh = oR, oOst = take(sizeof(OrderedState)), oA = take(spec * 8), oBb = take(spec * 8), oC = take(spec * 8), oS = take(spec * 16),
                oTx = take((size_t)nx * 16), oTy = take((size_t)ny * 16), oSt = take(sizeof(MpState)), oArr = take(sizeof(unsigned)), oSol = take(n),
                oWal = take(n), oDr = take(cells), oInv = take(n * 8), oWm = take(n * 8), oSa = take(cells * 8), oSb = take(cells * 8),
                oRho = take((size_t)nz * 8), oR4 = take((size_t)nz * 8), oDz = take((size_t)nz * 8), oIdz = take((size_t)nz * 8), oHz = take((size_t)nz * 8),
@@ -840,7 +898,8 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
   s->u = (float*)(M + oU); s->v = (float*)(M + oV); s->w = (float*)(M + oW);
   s->p = (double*)(M + oP); s->b = (double*)(M + oB); s->q = (double*)(M + oQ); s->r = (double*)(M + oR); s->z = (double*)(M + oZ);
   s->d[0] = (double*)(M + oD); s->d[1] = (double*)(M + oD2); s->sd = (double*)(M + oSd); s->fu = (double*)(M + oFu); s->fv = (double*)(M + oFv);
-  s->fw = (double*)(M + oFw); s->part = (double*)(M + oPart); s->arrived = (unsigned*)(M + oArr); s->st = (MpState*)(M + oSt);
+  s->fw = (double*)(M + oFw); s->z0 = (double*)(M + oS1);  // (each of the two routes' own)
+  s->part = (double*)(M + oPart); s->arrived = (unsigned*)(M + oArr); s->st = (MpState*)(M + oSt);
   sp.a = (double*)(M + oA); sp.b = (double*)(M + oBb); sp.c = (double*)(M + oC); sp.S = (double2*)(M + oS);
   sp.twx = (double2*)(M + oTx); sp.twy = (double2*)(M + oTy);
   s->sp = sp;
@@ -850,18 +909,31 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
   G.rho = (const double*)(M + oRho); G.rho4 = (const double*)(M + oR4); G.dzs = (const double*)(M + oDz); G.idz = (const double*)(M + oIdz);
   G.hz = (const double*)(M + oHz);
   G.nx = nx; G.ny = ny; G.nz = nz; G.layer = layer; G.nc = nc; G.n = n; G.cells = cells; G.dx = g.dx; G.dy = g.dy;
+  OrderedSolve& O = s->ordered;
+  O.solid = G.solid; O.wall = G.wall; O.dropped = G.dropped; O.A = G.A; O.B = G.B; O.invMass = G.invMass; O.rho4 = G.rho4;
+  O.dzs = G.dzs; O.idz = G.idz; O.lo = (const double*)(M + oLo); O.cp = sp.c; O.piv = (const double*)(M + oPv); O.rpiv = (const double*)(M + oRpv);
+  O.twx = sp.twx; O.twy = sp.twy;
+  O.nx = nx; O.ny = ny; O.nz = nz; O.layer = layer; O.nc = nc; O.mh = mh; O.modes = modes; O.n = n; O.cells = cells;
+  O.dx = g.dx; O.dy = g.dy; O.rdx = 1 / g.dx; O.rdy = 1 / g.dy;
+  O.b = s->b; O.q = s->q; O.r = s->r; O.z = s->z; O.d = s->d[0]; O.e = s->d[1]; O.sd = s->sd; O.fu = s->fu; O.fv = s->fv; O.fw = s->fw;
+  O.part = s->part; O.S1 = (double2*)(M + oS1); O.S2 = sp.S; O.arrived = s->arrived; O.st = (OrderedState*)(M + oOst);
   cudaStream_t st = sg_context_stream(ctx);
   std::vector<double> dz(nz, 0.0);
   std::copy(g.dzs, g.dzs + nz - 1, dz.begin());
   struct Up { size_t off; const void* src; size_t bytes; };
-  const Up ups[] = {{oA, ta.data(), spec * 8}, {oBb, tb.data(), spec * 8}, {oC, tcp.data(), spec * 8}, {oTx, tx.data(), (size_t)nx * 16},
+  const Up ups[] = {{oLo, tlo.data(), spec * 8}, {oPv, tpiv.data(), spec * 8}, {oC, tcp.data(), spec * 8}, {oTx, tx.data(), (size_t)nx * 16},
                     {oTy, ty.data(), (size_t)ny * 16}, {oSol, solid.data(), n}, {oWal, wall.data(), n}, {oDr, dropped.data(), cells},
-                    {oInv, inv.data(), n * 8}, {oWm, wm.data(), n * 8}, {oSa, sa.data(), cells * 8}, {oSb, sb.data(), cells * 8},
+                    {oInv, inv.data(), n * 8}, {oLow, low.data(), cells * 8}, {oHigh, high.data(), cells * 8},
                     {oRho, rho, (size_t)nz * 8}, {oR4, rho4.data(), (size_t)nz * 8}, {oDz, dz.data(), (size_t)nz * 8},
                     {oIdz, idz.data(), (size_t)nz * 8}, {oHz, g.hz, (size_t)nz * 8}};
   for (const Up& up : ups)
     if ((e = cudaMemcpyAsync(M + up.off, up.src, up.bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
   if (e == cudaSuccess) e = cudaMemsetAsync(s->arrived, 0, sizeof(unsigned), st);
+  if (e == cudaSuccess) {
+    k_mp_tables<<<blocks(std::max(spec, n)), TPB, 0, st>>>((double*)(M + oPv), (double*)(M + oRpv), O.lo, (double*)(M + oA), (double*)(M + oBb),
+                                                               sp.factor(), spec, (const double*)(M + oLow), (const double*)(M + oHigh), (double*)(M + oSa), (double*)(M + oSb), (double*)(M + oWm), G);
+    e = cudaGetLastError();
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     cudaFree(s->mem); delete s;
@@ -943,6 +1015,7 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
     k_mp_div<0><<<cb, TPB, 0, s>>>(m->fu, m->fv, m->fw, m->sd, nullptr, 1 / (g.dx * g.dx), 1 / (g.dy * g.dy), nullptr, nullptr, g, m->st, ZERO);
     k_mp_resid<<<cb, TPB, 0, s>>>(m->b, m->sd, m->r, m->part, m->arrived, g, m->st);
     enqueue_first_precondition(m->sp, m->z, m->r, g.dzs, g.dropped, m->part, m->arrived, m->st, s);
+    if ((e = cudaMemcpyAsync(m->z0, m->z, cells * 8, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return fail(m, "first direction", e);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(m, "launch", e);
     if (!m->chunk) {
       // Eight iterations as one graph (the buffers are the object's own, so one capture serves every call).
@@ -963,13 +1036,20 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
       if ((e = cudaGraphLaunch(m->chunk, s)) != cudaSuccess) return fail(m, "graph launch", e);
     }
     if (!done) return sg_context_fail(m->ctx, SG_ERR_DEVICE, "masked projection: the iterations did not stop");
-    // u = M (u* - G phi); the pressure kept is phi / dt (:332-336).
-    k_mp_finish<<<cb, TPB, 0, s>>>(m->q, m->p, dt, g, m->st);
-    k_mp_correct<<<nb, TPB, 0, s>>>(m->u, m->v, m->w, m->q, g, m->st);
-    MpState fin{};
-    if ((e = cudaMemcpyAsync(&fin, m->st, sizeof(MpState), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return fail(m, "state", e);
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(m, "solve", e);
-    if (fin.done != ZERO) { m->iterations = fin.k; m->residual = std::sqrt(fin.rr / fin.bb); }
+    if (done == DRIFT) {
+      // The winds and the first guess are still as they were.
+      OrderedState fin{};
+      if ((e = m->ordered.solve(m->u, m->v, m->w, m->p, dt, m->maxIt, m->tolerance, &m->orderedChunk, &fin, s)) != cudaSuccess) return fail(m, "solve", e);
+      if (fin.done != ZERO) { m->iterations = fin.k; m->residual = std::sqrt(fin.rr / fin.bb); }
+    } else {
+      // u = M (u* - G phi); the pressure kept is phi / dt (:332-336).
+      k_mp_finish<<<cb, TPB, 0, s>>>(m->q, m->p, dt, g, m->st);
+      k_mp_correct<<<nb, TPB, 0, s>>>(m->u, m->v, m->w, m->q, g, m->st);
+      MpState fin{};
+      if ((e = cudaMemcpyAsync(&fin, m->st, sizeof(MpState), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return fail(m, "state", e);
+      if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(m, "solve", e);
+      if (fin.done != ZERO) { m->iterations = fin.k; m->residual = std::sqrt(fin.rr / fin.bb); }
+    }
   }
   for (int f = 0; f < 3; f++)
     if ((e = cudaMemcpyAsync(host[f], dev[f], n * 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return fail(m, "copy out", e);
@@ -1197,6 +1277,7 @@ int sg_masked_destroy(sg_masked* m) {
   cudaSetDevice(sg_context_device(m->ctx));
   cudaStreamSynchronize(sg_context_stream(m->ctx));
   if (m->chunk) cudaGraphExecDestroy(m->chunk);
+  if (m->orderedChunk) cudaGraphExecDestroy(m->orderedChunk);
   cudaFree(m->mem);
   delete m;
   return SG_OK;
