@@ -148,11 +148,13 @@ constexpr int CHUNK = 4096;   // nodes per packed-transfer item, and at most per
 // us, the sums 70, 72 and 88 (a block's sums cost it as much as four nodes a thread).
 SG_HD int chunk_nodes(size_t n) { return n <= (1u << 20) ? 1024 : CHUNK; }
 // Nodes per item of the pointwise kernels without sums (node items: slot, first node, end), free to follow the batch:
-// the largest power of two that still gives `blocks` items, within 512..4096. A single standard run's step (658 us) is
-// 125 us faster with 512-node items than with 4096; the 64-run batch's corrections are 15% faster with 2048 than 1024.
-inline int node_chunk(size_t nodes, size_t blocks) {
+// the largest power of two in 512..4096 that gives eight items an SM, but 2048 where that gives three. A single standard
+// run's step (658 us) is 125 us faster with 512-node items than with 4096, a block of 256 threads then taking two nodes a
+// thread; larger batches lose by that, since the kernels load four nodes a thread a pass: 16 runs' corrections take 15 us
+// with 2048-node items and 19 with 512, and the pipelined round trips of four such groups 3.9 ms a step against 4.05.
+inline int node_chunk(size_t nodes, size_t sms) {
   int c = CHUNK;
-  while (c > 512 && nodes / c < blocks) c /= 2;
+  while (c > 512 && nodes / c < sms * (c > 2048 ? 8 : 3)) c /= 2;
   return c;
 }
 

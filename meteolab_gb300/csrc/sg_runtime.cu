@@ -77,6 +77,7 @@ struct Run {
 
 struct Plan {
   std::vector<int> slots;
+  int share = 1;          // plans of this size that run at the same time (the groups of the host round trips)
   int4* items = nullptr;  // device
   int off[24] = {0}, cnt[24] = {0};
   int maxnx = 0, maxny = 0, maxnz = 0, TX = 40, TY = 8, wenoG = 3;  // transport tile and WENO fields per item
@@ -340,26 +341,41 @@ Run* find(sg_context* ctx, sg_run run) {
 }
 
 // ------------------------------------------------------------------ plans
-// Transport work items (run, field group, tile) of a plan for a tile shape and WENO group size: groups 0-2 are the
-// WENO fields in threes, 4-12 one by one, 3 the dynamics {u, v, w, theta'}.
-void transport_items(sg_context* ctx, const std::vector<int>& slots, int TX, int TY, int wenoG, std::vector<int4>* fam) {
+// Slabs of levels a transport item's columns are cut into: while a plan's items leave SMs idle, as many as give each SM
+// one, of at least eight levels (a slab loads six planes and forms one face beyond its own). The column's march is serial:
+// the dynamics of one standard run are eight blocks and took 90 us a stage, 39 in slabs. A batch that fills the chip is
+// left alone, and so is one of several that together do (share): there the slabs' extra loads cost more than they give (the
+// round trips of 64 standard runs in four groups 3.9 ms a step without slabs in the dynamics, 4.2 with two).
+int transport_slabs(const sg_context* ctx, size_t items, int nz) {
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->sms / std::max<size_t>(1, items), (size_t)nz / 8));
+}
+int slab_levels(int nz, int slabs, int s) {  // slab s's levels, first | end << 16
+  return (nz * s / slabs) | (nz * (s + 1) / slabs) << 16;
+}
+// Transport work items (run, field group, tile, levels) of a plan for a tile shape and WENO group size: groups 0-2 are
+// the WENO fields in threes, 4-12 one by one, 3 the dynamics {u, v, w, theta'}. The bulk-copy kernels take whole columns.
+void transport_items(sg_context* ctx, const Plan& P, int TX, int TY, int wenoG, bool bulk, std::vector<int4>* fam) {
+  const std::vector<int>& slots = P.slots;
+  const int grp0 = wenoG == 3 ? 0 : 4, ngrp = wenoG == 3 ? 3 : 9;
+  size_t tilesAll = 0;
+  for (int s : slots) { const Run& r = ctx->runs[s]; tilesAll += (size_t)((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY); }
   for (int s : slots) {
     const Run& r = ctx->runs[s];
     const int tiles = ((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY);
-    const int grp0 = wenoG == 3 ? 0 : 4, ngrp = wenoG == 3 ? 3 : 9;
-    for (int g = grp0; g < grp0 + ngrp; g++) for (int t = 0; t < tiles; t++) fam[0].push_back(make_int4(s, g, t, 0));
-    for (int t = 0; t < tiles; t++) fam[1].push_back(make_int4(s, 3, t, 0));
+    const int sw = bulk ? 1 : transport_slabs(ctx, tilesAll * ngrp * P.share, r.nz), sd = bulk ? 1 : transport_slabs(ctx, tilesAll * P.share, r.nz);
+    for (int g = grp0; g < grp0 + ngrp; g++)
+      for (int t = 0; t < tiles; t++) for (int k = 0; k < sw; k++) fam[0].push_back(make_int4(s, g, t, slab_levels(r.nz, sw, k)));
+    for (int t = 0; t < tiles; t++) for (int k = 0; k < sd; k++) fam[1].push_back(make_int4(s, 3, t, slab_levels(r.nz, sd, k)));
   }
 }
 
-// The extra fields of the plan's runs, one WENO field an item on the plan's tile: the charge carriers of the
-// electrified runs (groups 13-16), the raindrop number of the two-moment ones (group 17).
-// The extra fields' transport items: three fields an item where a run carries a whole triple (groups 22: the first
-// three charge carriers, 23: the drop number with graupel's number and volume, 24: hail's number and volume with the
-// ions' charge), the rest one an item (groups 13-21).
-void charge_items(sg_context* ctx, const std::vector<int>& slots, int TX, int TY, std::vector<int4>& out, std::vector<int4>& out3) {
+// The extra fields' transport items on the plan's tile: three fields an item where a run carries a whole triple (groups
+// 22: the first three charge carriers, 23: the drop number with graupel's number and volume, 24: hail's number and volume
+// with the ions' charge), the rest one an item (groups 13-16: charge carriers, 17: the raindrop number, 18-21: the ice
+// classes' numbers and volumes); slabs of levels as above.
+void charge_items(sg_context* ctx, const Plan& P, int TX, int TY, std::vector<int4>& out, std::vector<int4>& out3) {
   out.clear(); out3.clear();
-  for (int s : slots) {
+  for (int s : P.slots) {
     const Run& r = ctx->runs[s];
     const int tiles = ((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY);
     const bool elec = r.desc.flags & RF_ELEC, rain2 = r.desc.flags & RF_RAIN2M, ice2 = r.desc.flags & RF_ICE2M;
@@ -373,6 +389,14 @@ void charge_items(sg_context* ctx, const std::vector<int>& slots, int TX, int TY
     }
     for (int g : threes) for (int t = 0; t < tiles; t++) out3.push_back(make_int4(s, g, t, 0));
     for (int g : ones) for (int t = 0; t < tiles; t++) out.push_back(make_int4(s, g, t, 0));
+  }
+  for (std::vector<int4>* list : {&out, &out3}) {
+    std::vector<int4> cut;
+    for (const int4& i : *list) {
+      const int nz = ctx->runs[i.x].nz, slabs = transport_slabs(ctx, list->size() * P.share, nz);
+      for (int k = 0; k < slabs; k++) cut.push_back(make_int4(i.x, i.y, i.z, slab_levels(nz, slabs, k)));
+    }
+    list->swap(cut);
   }
 }
 
@@ -392,8 +416,9 @@ int upload_items(sg_context* ctx, Plan& P, std::vector<int4>* all) {
 
 int autotune_transport(sg_context* ctx, Plan& P);
 
-int build_plan(sg_context* ctx, const std::vector<int>& slots, Plan& P) {
+int build_plan(sg_context* ctx, const std::vector<int>& slots, int share, Plan& P) {
   P.slots = slots;
+  P.share = share;
   std::vector<int4> all[FAM_COUNT];
   bool all40 = true;
   for (int s : slots) {
@@ -420,7 +445,7 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, Plan& P) {
   P.yc = P.rowAny ? std::min(P.rowMaxnx > 128 ? 16 : 32, (P.rowMaxny + 1) / 2 * 2) : 32;
   size_t nodes = 0;
   for (int s : slots) nodes += (size_t)ctx->runs[s].desc.n;
-  const int step = node_chunk(nodes, (size_t)ctx->sms * 8);
+  const int step = node_chunk(nodes * P.share, (size_t)ctx->sms);
   for (int s : slots) {
     const Run& r = ctx->runs[s];
     int n = r.nx * r.ny * r.nz, chunk = r.desc.chunk, nch = (n + chunk - 1) / chunk, layer = r.nx * r.ny, cells = layer * (r.nz - 1);
@@ -450,31 +475,35 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, Plan& P) {
     if (r.desc.flags & RF_EXTRA) P.extra = true;
     if (r.desc.flags & RF_RAIN2M) P.rain2m = true;
   }
-  // mixing items: (run, tile, z0, z1), the column in four level ranges
+  // mixing items and, for refined runs, refinement items: (run, tile, z0, z1). A column is cut into four level ranges, and
+  // where the batch's tiles are few into as many as give each SM an item, of at least six levels (each range reloads the
+  // planes at its ends): one standard run's mixing 28 -> 21 us, its refinement 25 -> 18.
+  auto ranges = [&](int TX, int TY, int fam, bool refinedOnly) {
+    size_t tilesAll = 0;
+    for (int s : slots) { const Run& r = ctx->runs[s]; tilesAll += (size_t)((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY); }
+    for (int s : slots) {
+      const Run& r = ctx->runs[s];
+      if (refinedOnly && !(r.desc.flags & RF_REFINE)) continue;
+      const int tiles = ((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY);
+      const int cuts = std::max(4, std::min((int)((size_t)ctx->sms / (tilesAll * P.share)), r.nz / 6)), zc = (r.nz + cuts - 1) / cuts;
+      for (int t = 0; t < tiles; t++)
+        for (int z0 = 0; z0 < r.nz; z0 += zc) all[fam].push_back(make_int4(s, t, z0, std::min(r.nz, z0 + zc)));
+    }
+  };
   P.mixTX = all40 ? 40 : 32; P.mixTY = 8;
-  for (int s : slots) {
-    const Run& r = ctx->runs[s];
-    const int tiles = ((r.nx + P.mixTX - 1) / P.mixTX) * ((r.ny + P.mixTY - 1) / P.mixTY), zc = (r.nz + 3) / 4;
-    for (int t = 0; t < tiles; t++)
-      for (int z0 = 0; z0 < r.nz; z0 += zc) all[FAM_MIX].push_back(make_int4(s, t, z0, std::min(r.nz, z0 + zc)));
-  }
-  // refinement items (refined runs only): (run, tile, z0, z1) on tiles whose nodes, halo included, fit one block
-  P.refTX = all40 ? 20 : 16; P.refTY = 8;
-  for (int s : slots) {
-    const Run& r = ctx->runs[s];
-    if (!(r.desc.flags & RF_REFINE)) continue;
-    const int tiles = ((r.nx + P.refTX - 1) / P.refTX) * ((r.ny + P.refTY - 1) / P.refTY), zc = (r.nz + 3) / 4;
-    for (int t = 0; t < tiles; t++)
-      for (int z0 = 0; z0 < r.nz; z0 += zc) all[FAM_REFINE].push_back(make_int4(s, t, z0, std::min(r.nz, z0 + zc)));
-  }
+  ranges(P.mixTX, P.mixTY, FAM_MIX, false);
+  P.refTX = all40 ? 20 : 16; P.refTY = 8;  // tiles whose nodes, halo included, fit one block
+  ranges(P.refTX, P.refTY, FAM_REFINE, true);
   if (ctx->pinned[0]) { P.TX = ctx->pinned[0]; P.TY = ctx->pinned[1]; P.wenoG = ctx->pinned[2]; P.minb = ctx->pinned[3]; }
   P.bulk = P.minb == 2 && ctx->bulk && transport_bulk_ok(P.TX, P.TY, P.minnx, P.nx4) &&
            std::max(transport_smem_bulk(TK_WENO, P.wenoG, P.TX, P.TY), transport_smem_bulk(TK_DYN, 4, P.TX, P.TY)) <= (size_t)ctx->maxSmem;
-  transport_items(ctx, slots, P.TX, P.TY, P.wenoG, all + FAM_T_WENO);
-  charge_items(ctx, slots, P.TX, P.TY, all[FAM_T_CHG], all[FAM_T_CHG3]);
-  int st = upload_items(ctx, P, all);
-  if (st != SG_OK) return st;
-  return ctx->autotune && !ctx->pinned[0] ? autotune_transport(ctx, P) : SG_OK;
+  if (ctx->autotune && !ctx->pinned[0]) {
+    const int st = autotune_transport(ctx, P);
+    if (st != SG_OK) return st;
+  }
+  transport_items(ctx, P, P.TX, P.TY, P.wenoG, P.bulk, all + FAM_T_WENO);
+  charge_items(ctx, P, P.TX, P.TY, all[FAM_T_CHG], all[FAM_T_CHG3]);
+  return upload_items(ctx, P, all);
 }
 
 Launch lx(sg_context* ctx, const Plan& P, int fam, int capPerSm = 8) {
@@ -506,7 +535,7 @@ void launch_transport_kinds(sg_context* ctx, const Plan& P, int in, int out, flo
   }
 }
 
-// Picks the transport tile (TX x TY columns) and WENO fields per item by timing every candidate on the plan's own
+// Picks the plan's transport tile (TX x TY columns) and WENO fields per item, before its items are made, by timing every candidate on the plan's own
 // runs: the two transport kinds of one RK3 stage (set A in, set C out; C is scratch between steps), best of three
 // after a warm-up. Results are cached per batch signature (the sorted grid shapes, and the run count to a power of
 // two), so a serving loop whose batch changes run by run tunes each kind of batch once.
@@ -522,6 +551,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     for (auto& d : dims) sig.insert(sig.end(), d.begin(), d.end());
     int c = 1; while (c < (int)P.slots.size()) c *= 2;
     sig.push_back(c);
+    sig.push_back(P.share);
   }
   std::array<int, 5> best{P.TX, P.TY, P.wenoG, P.minb, P.bulk ? 1 : 0};
   auto it = ctx->tuning.find(sig);
@@ -533,7 +563,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1));
     float bestMs = 1e30f;
     Plan T;  // candidate items only
-    T.slots = P.slots; T.maxnx = P.maxnx; T.maxny = P.maxny; T.maxnz = P.maxnz; T.minnx = P.minnx; T.nx4 = P.nx4;
+    T.slots = P.slots; T.share = P.share; T.maxnx = P.maxnx; T.maxny = P.maxny; T.maxnz = P.maxnz; T.minnx = P.minnx; T.nx4 = P.nx4;
     for (auto& sh : shapes) {
       const int TX = sh[0], TY = sh[1];
       if (TX > 2 * P.maxnx || TY > 2 * P.maxny) continue;
@@ -546,7 +576,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
                                  : transport_smem(TK_WENO, G, TX, TY);
         if (need > (size_t)ctx->maxSmem) continue;
         std::vector<int4> all[FAM_COUNT];
-        transport_items(ctx, P.slots, TX, TY, G, all + FAM_T_WENO);
+        transport_items(ctx, T, TX, TY, G, bulk, all + FAM_T_WENO);
         int st = upload_items(ctx, T, all);
         if (st != SG_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return st; }
         T.TX = TX; T.TY = TY; T.wenoG = G; T.minb = MB; T.bulk = bulk;
@@ -569,15 +599,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     ctx->tuning[sig] = best;
   }
   P.TX = best[0]; P.TY = best[1]; P.wenoG = best[2]; P.minb = best[3]; P.bulk = best[4] != 0; P.tuned = true;
-  std::vector<int4> all[FAM_COUNT];
-  for (int f = 0; f < FAM_COUNT; f++) {  // keep the other families, rebuild the transport ones
-    if (f == FAM_T_WENO || f == FAM_T_DYN || f == FAM_T_CHG || f == FAM_T_CHG3) continue;
-    all[f].resize(P.cnt[f]);
-    if (P.cnt[f]) CK(cudaMemcpy(all[f].data(), P.items + P.off[f], P.cnt[f] * sizeof(int4), cudaMemcpyDeviceToHost));
-  }
-  transport_items(ctx, P.slots, P.TX, P.TY, P.wenoG, all + FAM_T_WENO);
-  charge_items(ctx, P.slots, P.TX, P.TY, all[FAM_T_CHG], all[FAM_T_CHG3]);
-  return upload_items(ctx, P, all);
+  return SG_OK;
 }
 
 // The three stages of a spectral solve (divergence and forward transform, mode solves, inverse transform) on the
@@ -731,15 +753,19 @@ const char* KERNEL_NAMES[NKERNELS] = {"fall_courant", "sediment", "face_div_xfft
                                       "refine_residual", "refine_unused", "refine_div_xfft", "refine_modes", "refine_xifft", "refine_correct",
                                       "rotation_columns", "rotation_summary", "sediment_2m", "transport_extra"};
 
-Plan* get_plan(sg_context* ctx, const std::vector<int>& slots, int* status) {
-  auto it = ctx->plans.find(slots);
+// The plan of a batch; `share` > 1: of one group of that many that are stepped at the same time (its own plan: the key
+// ends in -share).
+Plan* get_plan(sg_context* ctx, const std::vector<int>& slots, int* status, int share = 1) {
+  std::vector<int> key = slots;
+  if (share > 1) key.push_back(-share);
+  auto it = ctx->plans.find(key);
   if (it != ctx->plans.end()) { *status = SG_OK; return it->second.get(); }
   if (ctx->plans.size() > 256) ctx->plans.clear();
   auto P = std::make_unique<Plan>();
-  *status = build_plan(ctx, slots, *P);
+  *status = build_plan(ctx, slots, share, *P);
   if (*status != SG_OK) return nullptr;
   Plan* raw = P.get();
-  ctx->plans[slots] = std::move(P);
+  ctx->plans[key] = std::move(P);
   return raw;
 }
 
@@ -1196,7 +1222,7 @@ static int batch_step_io(sg_context* ctx, const sg_run* runs, int n, uint32_t ma
     x.first = (int)((int64_t)n * g / groups);
     x.count = (int)((int64_t)n * (g + 1) / groups) - x.first;
     const std::vector<int> slots(all.begin() + x.first, all.begin() + x.first + x.count);
-    if (!(x.P = get_plan(ctx, slots, &st))) return st;
+    if (!(x.P = get_plan(ctx, slots, &st, groups))) return st;
     if (x.P->elec) return fail(ctx, SG_ERR_UNSUPPORTED, "host round trips of electrified runs: step them with sg_batch_step (the lightning is host-stepped)");
     if ((st = ensure_graph(ctx, *x.P)) != SG_OK) return st;
     if ((st = pack_items(ctx, runs + x.first, x.count, mask, x.items, x.total)) != SG_OK) return st;

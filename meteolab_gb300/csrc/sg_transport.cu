@@ -21,6 +21,8 @@ namespace sg {
 // arithmetic, every thread reconstructs the east and north faces of its own cell (as one packed pair) and the top face,
 // threads 0..TY-1 and TY..TY+TX-1 reconstruct the tile's west and south edge faces, the x and y faces are exchanged
 // through shared memory (double-buffered), and one barrier separates the levels. The group shares the face-flux loads.
+// An item is a slab of levels of the tile: the column's march is a serial chain of some 1.7 us a level, and a small
+// batch has fewer tiles than the chip has SMs, so the plan cuts its columns (transport_slabs, sg_runtime.cu).
 constexpr int TMAXC = 4;  // plane cells per thread: (TX + 6)(TY + 6) <= TMAXC * TX * TY
 // Per-level constants staged in shared memory, rows of MAXNZ: 1/hz, 1/rho (both kinds), theta's four base-profile
 // face values, thb, qb, thv_env (dynamics).
@@ -82,11 +84,12 @@ __device__ __forceinline__ void face_stencil(const float* P, int s, bool pos, fl
 // of the block waits for at every level's barrier.
 constexpr int TEDGE = 64;  // edge threads of an EW block
 template <int KIND, int G, int CTX, int CTY, bool EW>
-__device__ __forceinline__ void transport_item(const RunDesc& Rg, int group, int tile, int in_set, int out_set, float frac, int stage,
+__device__ __forceinline__ void transport_item(const RunDesc& Rg, int group, int tile, int levels, int in_set, int out_set, float frac, int stage,
                                                int TXr, int TYr, float* sm) {
   const int TX = CTX ? CTX : TXr, TY = CTY ? CTY : TYr;
   const int nx = Rg.nx, ny = Rg.ny, nz = Rg.nz, layer = Rg.layer;
   const size_t n = Rg.n;
+  const int z0 = levels & 0xffff, z1 = levels >> 16;  // the slab's levels
   const float inv_dx = Rg.inv_dx, inv_dy = Rg.inv_dy, fdt = frac * Rg.dt;
   const int flags = Rg.flags;
   const float4* __restrict__ F4 = reinterpret_cast<const float4*>(Rg.faces);
@@ -152,25 +155,27 @@ __device__ __forceinline__ void transport_item(const RunDesc& Rg, int group, int
   }
   const bool loadBuoy = KIND == TK_DYN && (flags & RF_STAGES);
   const bool loading = flags & RF_LOADING;
-  // prologue: ring slots of the virtual levels -3..3 (clamped), level 0's inputs
-  for (int v = -3; v <= 3; v++) {
+  // prologue: ring slots of the virtual levels z0 - 3..z0 + 3 (clamped), level z0's inputs
+  for (int v = z0 - 3; v <= z0 + 3; v++) {
     const int lev = clampi(v, 0, nz - 1), slot = (v + 7) % 7;
 #pragma unroll
     for (int g = 0; g < G; g++)
 #pragma unroll
       for (int j = 0; j < CJ; j++) if (off[j] >= 0) ring[(g * 7 + slot) * NCELL + t + j * NT] = QP(g)[off[j] + lev * layer];
   }
-  if (on) cp_async16(fcs + t, F4 + col);
-  float me = edgeW ? F4[eoff].x : edgeS ? F4[eoff].y : 0.f;
+  const int l0 = z0 * layer;
+  if (on) cp_async16(fcs + (z0 & 1) * NT + t, F4 + col + l0);
+  float me = edgeW ? F4[eoff + l0].x : edgeS ? F4[eoff + l0].y : 0.f;
   float s0[G];
 #pragma unroll
-  for (int g = 0; g < G; g++) s0[g] = on && stage > 0 ? SP(g)[col] : 0.f;
+  for (int g = 0; g < G; g++) s0[g] = on && stage > 0 ? SP(g)[col + l0] : 0.f;
   // buoyancy inputs of the level (dynamics): the vapour and the condensate load (theta' is the ring's centre value)
   float bQ = 0.f, bL = 0.f;
   if (loadBuoy && on) {
-    bQ = inb[Q * n + col];
-    bL = inb[CLOUD * n + col] + inb[ICE * n + col] +
-         (loading ? (inb[RAIN * n + col] + inb[SNOW * n + col]) + (inb[GRAUPEL * n + col] + inb[HAIL * n + col]) : 0.f);
+    const int c0 = col + l0;
+    bQ = inb[Q * n + c0];
+    bL = inb[CLOUD * n + c0] + inb[ICE * n + c0] +
+         (loading ? (inb[RAIN * n + c0] + inb[SNOW * n + c0]) + (inb[GRAUPEL * n + c0] + inb[HAIL * n + c0]) : 0.f);
   }
   cp_async_wait_all();
   __syncthreads();
@@ -179,9 +184,28 @@ __device__ __forceinline__ void transport_item(const RunDesc& Rg, int group, int
   for (int g = 0; g < G; g++) fzD[g] = 0.f;
   float mzD = 0.f;
   const int cidx = (ly + 3) * PW + (lx + 3);
-  for (int z = 0; z < nz; z++) {
+  // a slab above the ground: the face below it, formed as the level below forms its top face (the same bits)
+  if (z0 > 0 && on) {
+    mzD = F4[col + l0 - layer].z;
+    const bool pz = mzD >= 0.f;
+    const int s_m3 = (z0 + 4) % 7, s_m2 = (z0 + 5) % 7, s_m1 = (z0 + 6) % 7, s_0 = z0 % 7, s_p1 = (z0 + 1) % 7, s_p2 = (z0 + 2) % 7;
+#pragma unroll
+    for (int g = 0; g < G; g += 2) {
+      const int g2 = g + 1 < G ? g + 1 : g;
+      const float* R = ring + g * 7 * NCELL + cidx;
+      const float* S = ring + g2 * 7 * NCELL + cidx;
+      const float2 a2 = make_float2(R[s_m3 * NCELL], S[s_m3 * NCELL]), a1 = make_float2(R[s_m2 * NCELL], S[s_m2 * NCELL]);
+      const float2 c0 = make_float2(R[s_m1 * NCELL], S[s_m1 * NCELL]), b1 = make_float2(R[s_0 * NCELL], S[s_0 * NCELL]);
+      const float2 b2 = make_float2(R[s_p1 * NCELL], S[s_p1 * NCELL]), b3 = make_float2(R[s_p2 * NCELL], S[s_p2 * NCELL]);
+      const float2 A = pz ? a2 : b3, B = pz ? a1 : b2, C = pz ? c0 : b1, D = pz ? b1 : c0, E = pz ? b2 : a1;
+      const float2 r = recon2<KIND>(A, B, C, D, E);
+      fzD[g] = mzD * r.x;
+      if (g + 1 < G) fzD[g + 1] = mzD * r.y;
+    }
+  }
+  for (int z = z0; z < z1; z++) {
     const int buf = z & 1, l = z * layer;
-    const bool more = z + 1 < nz;
+    const bool more = z + 1 < z1;
     const int ln = l + layer;
     // loads for later levels, issued before this level's arithmetic: the plane z + 4 into the ring slot of z - 3
     // (read last by the previous level, before its barrier) by asynchronous copies; level z + 1's faces, start values
@@ -316,7 +340,7 @@ __global__ void __launch_bounds__(EW ? 320 + TEDGE : 320, MINB) k_transport(cons
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
     if (R.cnt[C_FAILED]) continue;
-    transport_item<KIND, G, CTX, CTY, EW>(R, items[it].y, items[it].z, in_set, out_set, frac, stage, TX, TY, sm);
+    transport_item<KIND, G, CTX, CTY, EW>(R, items[it].y, items[it].z, items[it].w, in_set, out_set, frac, stage, TX, TY, sm);
   }
 }
 
