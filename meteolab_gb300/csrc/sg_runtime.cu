@@ -343,7 +343,7 @@ Run* find(sg_context* ctx, sg_run run) {
 // ------------------------------------------------------------------ plans
 // Slabs of levels a transport item's columns are cut into: while a plan's items leave SMs idle, as many as give each SM
 // one, of at least eight levels (a slab loads six planes and forms one face beyond its own). The column's march is serial:
-// the dynamics of one standard run are eight blocks and took 90 us a stage, 39 in slabs. A batch that fills the chip is
+// the dynamics of one standard run are eight blocks and took 90 us a stage, 27 in slabs. A batch that fills the chip is
 // left alone, and so is one of several that together do (share): there the slabs' extra loads cost more than they give (the
 // round trips of 64 standard runs in four groups 3.9 ms a step without slabs in the dynamics, 4.2 with two).
 int transport_slabs(const sg_context* ctx, size_t items, int nz) {
