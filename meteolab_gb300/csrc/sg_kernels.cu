@@ -1564,8 +1564,9 @@ __global__ void k_viscosity(const RunDesc* __restrict__ runs, const int4* items,
 // Explicit flux-form diffusion of each mixed field's departure (Turbulence.mix, src/core/turbulence.ts:143-185),
 // then the ground drag balanced against the environment's own and rigid w at the ground and top (mixStep, :1179-1194).
 // In: set `in`; out: set A. A block takes one tile of columns of one run and a range of levels [z0, z1), marching up:
-// per level the planes of the mixed fields and of K_h (1-node periodic halo) arrive in shared memory by asynchronous
-// copies issued a level ahead, the vertical neighbours and K_m stay in registers, one barrier per level.
+// per level the planes of the mixed fields and of K_h (1-node periodic halo) arrive in one of three shared-memory buffers
+// by asynchronous copies issued two levels ahead, so the level above is there too; the level below's values and K_m stay in
+// registers, one barrier per level.
 constexpr int MIX_MAXC = 2;  // plane cells per thread: (TX + 2)(TY + 2) <= MIX_MAXC * TX * TY
 template <int NM>
 __device__ __forceinline__ void mix_item(const RunDesc& R, int tile, int z0, int z1, int in, int TX, int TY, float* sm) {
@@ -1596,39 +1597,28 @@ __device__ __forceinline__ void mix_item(const RunDesc& R, int tile, int z0, int
     gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
     off[j] = e < NCELL ? gx + gy * nx : 0;
   }
-  // plane z0 into buffer 0; the centre values of z0 - 1, z0, z0 + 1 into registers
+  auto load_plane = [&](int z, float* to) {
 #pragma unroll
-  for (int p = 0; p < NP; p++)
+    for (int p = 0; p < NP; p++)
 #pragma unroll
-    for (int j = 0; j < MIX_MAXC; j++) if (cell[j] >= 0) sm[p * NCELL + cell[j]] = SRC(p)[off[j] + z0 * layer];
-  float below[NM], cur[NM], above[NM];
+      for (int j = 0; j < MIX_MAXC; j++) if (cell[j] >= 0) cp_async4(to + p * NCELL + cell[j], SRC(p) + off[j] + z * layer);
+  };
+  // planes z0 and z0 + 1 into buffers 0 and 1; the centre values of z0 - 1 into registers
+  load_plane(z0, sm);
+  if (z0 + 1 < nz) load_plane(z0 + 1, sm + NP * NCELL);
+  float below[NM];
 #pragma unroll
-  for (int k = 0; k < NM; k++) {
-    cur[k] = SRC(k)[col + z0 * layer];
-    below[k] = z0 > 0 ? SRC(k)[col + (z0 - 1) * layer] : 0.f;
-    above[k] = z0 + 1 < nz ? SRC(k)[col + (z0 + 1) * layer] : 0.f;
-  }
+  for (int k = 0; k < NM; k++) below[k] = z0 > 0 ? SRC(k)[col + (z0 - 1) * layer] : 0.f;
   float kmD = z0 > 0 ? km[col + (z0 - 1) * layer] : 0.f, kmC = km[col + z0 * layer], kmU = z0 + 1 < nz ? km[col + (z0 + 1) * layer] : 0.f;
+  cp_async_wait_all();
   __syncthreads();
   const float ix2 = R.inv_dx * R.inv_dx, iy2 = R.inv_dy * R.inv_dy, dt = R.dt;
   const int cc = (ly + 1) * PW + lx + 1;
+  float *P = sm, *A1 = sm + NP * NCELL, *A2 = sm + 2 * NP * NCELL;  // this level's planes, the level above's, the next
   for (int z = z0; z < z1; z++) {
-    const int buf = (z - z0) & 1;
-    const float* P = sm + buf * NP * NCELL;
-    // a level ahead: plane z + 1 (asynchronous copies into the other buffer), the centre values of z + 2
-    if (z + 1 < z1) {
-      float* Q = sm + (buf ^ 1) * NP * NCELL;
-#pragma unroll
-      for (int p = 0; p < NP; p++)
-#pragma unroll
-        for (int j = 0; j < MIX_MAXC; j++) if (cell[j] >= 0) cp_async4(Q + p * NCELL + cell[j], SRC(p) + off[j] + (z + 1) * layer);
-    }
-    float nextv[NM];
-    float kmN = 0.f;
-    const bool more = z + 2 < nz;
-#pragma unroll
-    for (int k = 0; k < NM; k++) nextv[k] = more ? SRC(k)[col + (z + 2) * layer] : 0.f;
-    if (more) kmN = km[col + (z + 2) * layer];
+    // two levels ahead, into the buffer of the level below (read before the last barrier)
+    if (z + 1 < z1 && z + 2 < nz) load_plane(z + 2, A2);
+    const float kmN = z + 2 < nz ? km[col + (z + 2) * layer] : 0.f;
     if (on) {
       const float* KH = P + NM * NCELL + cc;
       const float khi = KH[0];
@@ -1642,7 +1632,7 @@ __device__ __forceinline__ void mix_item(const RunDesc& R, int tile, int z0, int
         const int f = mix_field(k);
         const float factor = k < 3 ? 1.f : 3.f;
         const float* A = P + k * NCELL + cc;
-        const float ai = cur[k];
+        const float ai = A[0], above = A1[k * NCELL + cc];
         // vertical departures: the base differences to the level above / below (u, v, q carry a base profile;
         // theta' is already a departure; w, cloud, ice, number have none)
         float bu = 0.f, bd = 0.f;
@@ -1651,7 +1641,8 @@ __device__ __forceinline__ void mix_item(const RunDesc& R, int tile, int z0, int
         else if (f == Q) { bu = z < nz - 1 ? lvl(R, L_DQB, z) : 0.f; bd = z > 0 ? lvl(R, L_DQB, z - 1) : 0.f; }
         const float tx = (hE * (A[1] - ai) - hW * (ai - A[-1])) * ix2;
         const float ty = (hN * (A[PW] - ai) - hS * (ai - A[-PW])) * iy2;
-        const float tz = (z < nz - 1 ? vU * ((above[k] - ai) - bu) : 0.f) - (z > 0 ? vD * ((ai - below[k]) - bd) : 0.f);
+        const float tz = (z < nz - 1 ? vU * ((above - ai) - bu) : 0.f) - (z > 0 ? vD * ((ai - below[k]) - bd) : 0.f);
+        below[k] = ai;
         float out = ai + dt * factor * (tx + ty + tz);
         if (f == U) uu = out;
         else if (f == V) vv = out;
@@ -1667,9 +1658,9 @@ __device__ __forceinline__ void mix_item(const RunDesc& R, int tile, int z0, int
       }
       field(R, 0, U)[i] = uu; field(R, 0, V)[i] = vv;
     }
-#pragma unroll
-    for (int k = 0; k < NM; k++) { below[k] = cur[k]; cur[k] = above[k]; above[k] = nextv[k]; }
     kmD = kmC; kmC = kmU; kmU = kmN;
+    float* const done = P;
+    P = A1; A1 = A2; A2 = done;
     cp_async_wait_all();
     __syncthreads();
   }
@@ -1845,7 +1836,7 @@ void launch_physics(const Launch& L, int in, int mid, int variant) {
   }
 }
 void launch_viscosity(const Launch& L, int set) { k_viscosity<<<GRID(L.n, L.cap), 256, 0, L.stream>>>(L.runs, L.items, L.n, set); }
-size_t mix_smem(int TX, int TY) { return (size_t)2 * (NMIX + 1) * (TX + 2) * (TY + 2) * sizeof(float); }
+size_t mix_smem(int TX, int TY) { return (size_t)3 * (NMIX + 1) * (TX + 2) * (TY + 2) * sizeof(float); }
 void launch_mix(const Launch& L, int in, int TX, int TY) {
   k_mix_tile<<<GRID(L.n, L.cap), TX * TY, mix_smem(TX, TY), L.stream>>>(L.runs, L.items, L.n, in, TX, TY);
 }
