@@ -341,6 +341,7 @@ SG_HD void microphysics(phys::Node& s, float& rn, Fields& f, const phys::Level& 
   const float exner = L.exner, rho = L.rho;
   float evap = (flags & RF_RAINFORM) ? r2m::processes(s, rn, L, dt, breakup, (flags & RF_EVAP) != 0) : 0.f;
   if (evap > 0.f) { const float cool = LV / CP / exner * evap; s.thp -= cool; s.cold += cool; }
+  SG_PHASE();
   float rainMark = s.rain;
   const float frozenDrops = rn, graupelMark = s.graupel;
   freezeRain(s, exner);
@@ -348,12 +349,15 @@ SG_HD void microphysics(phys::Node& s, float& rn, Fields& f, const phys::Level& 
   r2m::numberChange(s, rn, rainMark, rho, 0.f); rainMark = s.rain;
   settleCrystals(s);
   s.cold += iceProcesses(s, L, dt);
+    SG_PHASE();
   const float iceBefore = s.ice, cloudBefore = s.cloud;
   const float snowMass = r2m::exponentialMeanMass(s.snow, N0S, RHO_S, rho);
   s.cold += snowProcesses(s, L, dt);
+    SG_PHASE();
   r2m::numberChange(s, rn, rainMark, rho, snowMass);
   const float rainBefore = s.rain;
   s.cold += processes(s, rn, f, L, dt, wetG, wetH);
+    SG_PHASE();
   const float rainFrozen = tcOf(s, exner) < 0.f ? fmaxf(0.f, rainBefore - s.rain) : 0.f;
   if (iceBefore > 0.f) s.inum *= s.ice / iceBefore;
   const float splinters = splintering(tcOf(s, exner)) * SPLINTERS * fmaxf(0.f, cloudBefore - s.cloud)

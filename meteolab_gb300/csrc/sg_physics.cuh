@@ -5,6 +5,10 @@
 // - 273.15 of the level from FP64: FP32 resolves it to ~1e-6 K (an FP32 kelvin value near 290 K only to 3e-5 K,
 // which moves the saturation mixing ratio by ~2e-6 of itself and small condensation amounts by up to a percent).
 #pragma once
+// Between the processes of a node: the physics kernel's block goes from one to the next together (sg_kernels.cu).
+#ifndef SG_PHASE
+#define SG_PHASE()
+#endif
 #include <math.h>
 #include <algorithm>
 #include <cmath>
@@ -342,17 +346,22 @@ SG_HD void microphysics(Node& s, const Level& L, float dt, int flags, float& eva
   const float exner = L.exner, rho = L.rho;
   float evap = (flags & RF_RAINFORM) ? rainProcesses(s, L, dt, (flags & RF_EVAP) != 0) : 0.f;
   if (evap > 0.f) { float cool = LV / CP / exner * evap; s.thp -= cool; s.cold += cool; }
+  SG_PHASE();
   float cond;
   if (flags & RF_ICE) {
     freezeRain(s, exner);
     settleCrystals(s);
     s.cold += iceProcesses(s, L, dt);
+    SG_PHASE();
     float iceBefore = s.ice, cloudBefore = s.cloud;
     s.cold += snowProcesses(s, L, dt);
+    SG_PHASE();
     float rainBefore = s.rain;
     s.cold += graupelProcesses(s, L, dt);
+    SG_PHASE();
     float rainFrozen = tcOf(s, exner) < 0.f ? fmaxf(0.f, rainBefore - s.rain) : 0.f;
     s.cold += hailProcesses(s, L, dt);
+    SG_PHASE();
     if (iceBefore > 0.f) s.inum *= s.ice / iceBefore;
     float splinters = splintering(tcOf(s, exner)) * SPLINTERS * fmaxf(0.f, cloudBefore - s.cloud)
       + (rainFrozen > 0.f ? fragmentsPerKg(root4(PI * RHO_W * N0R / (rho * rainBefore))) * rainFrozen : 0.f);

@@ -117,6 +117,7 @@ SG_HD void microphysics(phys::Node& s, float& number, const phys::Level& L, floa
   const float exner = L.exner, rho = L.rho;
   float evap = (flags & RF_RAINFORM) ? processes(s, number, L, dt, breakup, (flags & RF_EVAP) != 0) : 0.f;
   if (evap > 0.f) { float cool = LV / CP / exner * evap; s.thp -= cool; s.cold += cool; }
+  SG_PHASE();
   float cond;
   if (flags & RF_ICE) {
     float rainMark = s.rain;
@@ -124,17 +125,21 @@ SG_HD void microphysics(phys::Node& s, float& number, const phys::Level& L, floa
     numberChange(s, number, rainMark, rho, 0.f); rainMark = s.rain;
     settleCrystals(s);
     s.cold += iceProcesses(s, L, dt);
+    SG_PHASE();
     float iceBefore = s.ice, cloudBefore = s.cloud;
     const float snowMass = exponentialMeanMass(s.snow, N0S, RHO_S, rho);
     s.cold += snowProcesses(s, L, dt);
+    SG_PHASE();
     numberChange(s, number, rainMark, rho, snowMass); rainMark = s.rain;
     float rainBefore = s.rain;
     const float graupelMass = exponentialMeanMass(s.graupel, N0G, RHO_G, rho);
     s.cold += graupelProcesses(s, L, dt);
+    SG_PHASE();
     numberChange(s, number, rainMark, rho, graupelMass); rainMark = s.rain;
     float rainFrozen = tcOf(s, exner) < 0.f ? fmaxf(0.f, rainBefore - s.rain) : 0.f;
     const float hailMass = exponentialMeanMass(s.hail, N0H, RHO_H, rho);
     s.cold += hailProcesses(s, L, dt);
+    SG_PHASE();
     numberChange(s, number, rainMark, rho, hailMass);
     if (iceBefore > 0.f) s.inum *= s.ice / iceBefore;
     float splinters = splintering(tcOf(s, exner)) * SPLINTERS * fmaxf(0.f, cloudBefore - s.cloud)
