@@ -80,11 +80,13 @@ struct Plan {
   int share = 1;          // plans of this size that run at the same time (the groups of the host round trips)
   int4* items = nullptr;  // device
   int off[24] = {0}, cnt[24] = {0};
-  int maxnx = 0, maxny = 0, maxnz = 0, TX = 40, TY = 8, wenoG = 3;  // transport tile and WENO fields per item
+  int maxnx = 0, maxny = 0, maxnz = 0, TX = 40, TY = 8, wenoG = 3;  // WENO transport tile and fields per item
   int minb = 2;                                                       // WENO transport blocks per SM (register budget)
   int minnx = 1 << 30;                                                // the narrowest grid of the plan
   bool nx4 = true;                                                    // every grid width a multiple of 4
-  bool bulk = false;                                                  // transport inputs by TMA bulk copies (producer warp)
+  bool bulk = false;                                                  // WENO transport inputs by TMA bulk copies (producer warp)
+  int dTX = 40, dTY = 8;                                              // dynamics transport tile
+  bool dBulk = false;                                                 // its inputs by bulk copies
   int yc = 32;                                                        // layer rows per x-transform item
   int mixTX = 32, mixTY = 8;                                          // mixing tile
   int refTX = 16, refTY = 8;                                          // refinement tile
@@ -134,7 +136,7 @@ struct sg_context {
   bool edgeWarps = true;                // per-thread transport with two edge warps (SG_TRANSPORT_EDGE_WARPS=0: the column threads take the edges)
   bool rowsOnly = false;                // row-transform spectral path for every grid (SG_SPECTRAL_ROWS=1)
   int pinned[4] = {0, 0, 0, 2};         // transport tile, WENO group, blocks per SM fixed by the caller (TX = 0: tune)
-  std::map<std::vector<int>, std::array<int, 5>> tuning;  // batch signature -> (TX, TY, wenoG, minb, bulk)
+  std::map<std::vector<int>, std::array<int, 8>> tuning;  // batch signature -> (TX, TY, wenoG, minb, bulk, dTX, dTY, dBulk)
   // packed transfers: a device staging buffer (grown on demand) and the item lists per (runs, mask)
   float* staging = nullptr;
   size_t stagingBytes = 0;
@@ -342,30 +344,30 @@ Run* find(sg_context* ctx, sg_run run) {
 
 // ------------------------------------------------------------------ plans
 // Slabs of levels a transport item's columns are cut into: while a plan's items leave SMs idle, as many as give each SM
-// one, of at least eight levels (a slab loads six planes and forms one face beyond its own). The column's march is serial:
-// the dynamics of one standard run are eight blocks and took 90 us a stage, 27 in slabs. A batch that fills the chip is
-// left alone, and so is one of several that together do (share): there the slabs' extra loads cost more than they give (the
-// round trips of 64 standard runs in four groups 3.9 ms a step without slabs in the dynamics, 4.2 with two).
+// one, of at least five levels (a slab loads six planes and forms one face beyond its own). The column's march is serial:
+// the dynamics of one standard run are eight blocks and took 90 us a stage, 27 in slabs of eight levels, 18 of five or
+// four. A batch that fills the chip is left alone, and so is one of several that together do (share): there the slabs'
+// extra loads cost more than they give (the round trips of 64 standard runs in four groups 3.9 ms a step without slabs in
+// the dynamics, 4.2 with two).
 int transport_slabs(const sg_context* ctx, size_t items, int nz) {
-  return (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->sms / std::max<size_t>(1, items), (size_t)nz / 8));
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->sms / std::max<size_t>(1, items), (size_t)nz / 5));
 }
 int slab_levels(int nz, int slabs, int s) {  // slab s's levels, first | end << 16
   return (nz * s / slabs) | (nz * (s + 1) / slabs) << 16;
 }
-// Transport work items (run, field group, tile, levels) of a plan for a tile shape and WENO group size: groups 0-2 are
-// the WENO fields in threes, 4-12 one by one, 3 the dynamics {u, v, w, theta'}. The bulk-copy kernels take whole columns.
-void transport_items(sg_context* ctx, const Plan& P, int TX, int TY, int wenoG, bool bulk, std::vector<int4>* fam) {
-  const std::vector<int>& slots = P.slots;
-  const int grp0 = wenoG == 3 ? 0 : 4, ngrp = wenoG == 3 ? 3 : 9;
+// Transport work items (run, field group, tile, levels) of a plan for a tile shape: of the WENO fields in groups of
+// wenoG (groups 0-2 in threes, 4-12 one by one), or of the dynamics {u, v, w, theta'} (group 3). The bulk-copy kernels
+// take whole columns.
+void transport_items(sg_context* ctx, const Plan& P, int kind, int TX, int TY, int wenoG, bool bulk, std::vector<int4>& out) {
+  const int grp0 = kind == TK_DYN ? 3 : wenoG == 3 ? 0 : 4, ngrp = kind == TK_DYN ? 1 : wenoG == 3 ? 3 : 9;
   size_t tilesAll = 0;
-  for (int s : slots) { const Run& r = ctx->runs[s]; tilesAll += (size_t)((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY); }
-  for (int s : slots) {
+  for (int s : P.slots) { const Run& r = ctx->runs[s]; tilesAll += (size_t)((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY); }
+  for (int s : P.slots) {
     const Run& r = ctx->runs[s];
     const int tiles = ((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY);
-    const int sw = bulk ? 1 : transport_slabs(ctx, tilesAll * ngrp * P.share, r.nz), sd = bulk ? 1 : transport_slabs(ctx, tilesAll * P.share, r.nz);
+    const int slabs = bulk ? 1 : transport_slabs(ctx, tilesAll * ngrp * P.share, r.nz);
     for (int g = grp0; g < grp0 + ngrp; g++)
-      for (int t = 0; t < tiles; t++) for (int k = 0; k < sw; k++) fam[0].push_back(make_int4(s, g, t, slab_levels(r.nz, sw, k)));
-    for (int t = 0; t < tiles; t++) for (int k = 0; k < sd; k++) fam[1].push_back(make_int4(s, 3, t, slab_levels(r.nz, sd, k)));
+      for (int t = 0; t < tiles; t++) for (int k = 0; k < slabs; k++) out.push_back(make_int4(s, g, t, slab_levels(r.nz, slabs, k)));
   }
 }
 
@@ -497,11 +499,13 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, int share, Plan& 
   if (ctx->pinned[0]) { P.TX = ctx->pinned[0]; P.TY = ctx->pinned[1]; P.wenoG = ctx->pinned[2]; P.minb = ctx->pinned[3]; }
   P.bulk = P.minb == 2 && ctx->bulk && transport_bulk_ok(P.TX, P.TY, P.minnx, P.nx4) &&
            std::max(transport_smem_bulk(TK_WENO, P.wenoG, P.TX, P.TY), transport_smem_bulk(TK_DYN, 4, P.TX, P.TY)) <= (size_t)ctx->maxSmem;
+  P.dTX = P.TX; P.dTY = P.TY; P.dBulk = P.bulk;
   if (ctx->autotune && !ctx->pinned[0]) {
     const int st = autotune_transport(ctx, P);
     if (st != SG_OK) return st;
   }
-  transport_items(ctx, P, P.TX, P.TY, P.wenoG, P.bulk, all + FAM_T_WENO);
+  transport_items(ctx, P, TK_WENO, P.TX, P.TY, P.wenoG, P.bulk, all[FAM_T_WENO]);
+  transport_items(ctx, P, TK_DYN, P.dTX, P.dTY, 0, P.dBulk, all[FAM_T_DYN]);
   charge_items(ctx, P, P.TX, P.TY, all[FAM_T_CHG], all[FAM_T_CHG3]);
   return upload_items(ctx, P, all);
 }
@@ -521,24 +525,29 @@ void launch_charges(sg_context* ctx, const Plan& P, int in, int out, float frac,
   if (C.n) launch_transport(C, TK_WENO, 1, P.minb, in, out, frac, stage, P.TX, P.TY, false, ctx->edgeWarps);
 }
 
-// Transport launches: one block per item, so the hardware block scheduler balances items of uneven cost (tiles of
-// empty air skip their WENO weights) across the SMs.
+// One stage's transport of a plan's WENO fields or dynamics, on the launch's stream: one block per item, so the hardware
+// block scheduler balances items of uneven cost (tiles of empty air skip their WENO weights) across the SMs.
+void launch_transport_kind(sg_context* ctx, const Plan& P, int kind, int in, int out, float frac, int stage, cudaStream_t stream) {
+  Launch L = lx(ctx, P, kind == TK_WENO ? FAM_T_WENO : FAM_T_DYN);
+  L.cap = L.n; L.stream = stream;
+  if (!L.n) return;
+  if (kind == TK_WENO) launch_transport(L, kind, P.wenoG, P.minb, in, out, frac, stage, P.TX, P.TY, P.bulk, ctx->edgeWarps);
+  else launch_transport(L, kind, 4, 2, in, out, frac, stage, P.dTX, P.dTY, P.dBulk, ctx->edgeWarps);
+}
 void launch_transport_kinds(sg_context* ctx, const Plan& P, int in, int out, float frac, int stage, int hookBase,
                             const std::function<void(int)>& hook) {
-  const int fams[2] = {FAM_T_WENO, FAM_T_DYN};
-  for (int k = 0; k < 2; k++) {
-    Launch L = lx(ctx, P, fams[k]);
-    L.cap = L.n;
-    if (L.n) launch_transport(L, k, P.wenoG, P.minb, in, out, frac, stage, P.TX, P.TY, P.bulk, ctx->edgeWarps);
-    hook(hookBase + k);
-    if (k == 0 && P.extra) { launch_charges(ctx, P, in, out, frac, stage, ctx->stream); hook(29); }
+  for (int kind : {TK_WENO, TK_DYN}) {
+    launch_transport_kind(ctx, P, kind, in, out, frac, stage, ctx->stream);
+    hook(hookBase + (kind == TK_DYN));
+    if (kind == TK_WENO && P.extra) { launch_charges(ctx, P, in, out, frac, stage, ctx->stream); hook(29); }
   }
 }
 
-// Picks the plan's transport tile (TX x TY columns) and WENO fields per item, before its items are made, by timing every candidate on the plan's own
-// runs: the two transport kinds of one RK3 stage (set A in, set C out; C is scratch between steps), best of three
-// after a warm-up. Results are cached per batch signature (the sorted grid shapes, and the run count to a power of
-// two), so a serving loop whose batch changes run by run tunes each kind of batch once.
+// Picks the plan's transport tiles (TX x TY columns) and WENO fields per item, before its items are made, by timing every
+// candidate on the plan's own runs: each of the two transport kinds of one RK3 stage by itself (set A in, set C out; C is
+// scratch between steps), best of three after a warm-up. Tuned together, the kinds shared a tile that suited their sum:
+// 16 standard runs 1.08 ms a step, tuned apart 1.00. Results are cached per batch signature (the sorted grid shapes, the run count to a power of two, and the
+// concurrent groups), so a serving loop whose batch changes run by run tunes each kind of batch once.
 int autotune_transport(sg_context* ctx, Plan& P) {
   std::vector<int> sig;
   for (int s : P.slots) { const Run& r = ctx->runs[s]; sig.push_back(r.nx); sig.push_back(r.ny); sig.push_back(r.nz); }
@@ -553,7 +562,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     sig.push_back(c);
     sig.push_back(P.share);
   }
-  std::array<int, 5> best{P.TX, P.TY, P.wenoG, P.minb, P.bulk ? 1 : 0};
+  std::array<int, 8> best{P.TX, P.TY, P.wenoG, P.minb, P.bulk, P.dTX, P.dTY, P.dBulk};
   auto it = ctx->tuning.find(sig);
   if (it != ctx->tuning.end()) {
     best = it->second;
@@ -561,44 +570,47 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     static const int shapes[][2] = {{40, 8}, {32, 8}, {20, 8}, {16, 16}, {16, 8}, {40, 4}, {32, 4}, {8, 8}};
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1));
-    float bestMs = 1e30f;
     Plan T;  // candidate items only
     T.slots = P.slots; T.share = P.share; T.maxnx = P.maxnx; T.maxny = P.maxny; T.maxnz = P.maxnz; T.minnx = P.minnx; T.nx4 = P.nx4;
-    for (auto& sh : shapes) {
+    float bestMs[2] = {1e30f, 1e30f};
+    for (auto& sh : shapes) for (int kind : {TK_WENO, TK_DYN}) {
       const int TX = sh[0], TY = sh[1];
       if (TX > 2 * P.maxnx || TY > 2 * P.maxny) continue;
-      // variants: per-thread copies at 2 or 3 blocks an SM, and (where the shape allows them) the bulk copies at 2
+      // variants: per-thread copies at 2 or (WENO) 3 blocks an SM, and (where the shape allows them) the bulk copies at 2
       for (int G : {3, 1}) for (int V : {0, 1, 2}) {
-        const int MB = V == 1 ? 3 : 2;
+        if (kind == TK_DYN && (G == 1 || V == 1)) continue;
+        const int MB = V == 1 ? 3 : 2, fields = kind == TK_DYN ? 4 : G;
         const bool bulk = V == 2;
         if (bulk && !(ctx->bulk && transport_bulk_ok(TX, TY, P.minnx, P.nx4))) continue;
-        const size_t need = bulk ? std::max(transport_smem_bulk(TK_WENO, G, TX, TY), transport_smem_bulk(TK_DYN, 4, TX, TY))
-                                 : transport_smem(TK_WENO, G, TX, TY);
-        if (need > (size_t)ctx->maxSmem) continue;
+        if ((bulk ? transport_smem_bulk(kind, fields, TX, TY) : transport_smem(kind, fields, TX, TY)) > (size_t)ctx->maxSmem) continue;
         std::vector<int4> all[FAM_COUNT];
-        transport_items(ctx, T, TX, TY, G, bulk, all + FAM_T_WENO);
+        transport_items(ctx, T, kind, TX, TY, G, bulk, all[kind == TK_WENO ? FAM_T_WENO : FAM_T_DYN]);
         int st = upload_items(ctx, T, all);
         if (st != SG_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return st; }
-        T.TX = TX; T.TY = TY; T.wenoG = G; T.minb = MB; T.bulk = bulk;
+        T.TX = T.dTX = TX; T.TY = T.dTY = TY; T.wenoG = G; T.minb = MB; T.bulk = T.dBulk = bulk;
         float ms = 1e30f;
         for (int rep = 0; rep < 4; rep++) {
           cudaEventRecord(e0, ctx->stream);
-          launch_transport_kinds(ctx, T, 0, 2, 1.f / 3.f, 0, 0, [](int) {});
+          launch_transport_kind(ctx, T, kind, 0, 2, 1.f / 3.f, 0, ctx->stream);
           cudaEventRecord(e1, ctx->stream);
           CK(cudaEventSynchronize(e1));
           float t = 0; cudaEventElapsedTime(&t, e0, e1);
           if (rep) ms = std::min(ms, t);
         }
         CK(cudaGetLastError());
-        if (ctx->tuneLog) fprintf(stderr, "stormgpu tuner: tile %dx%d, %d WENO fields an item, %d blocks an SM, %s: %.4f ms\n", TX, TY, G, MB,
-                                  bulk ? "bulk copies" : "per-thread copies", ms);
-        if (ms < bestMs) { bestMs = ms; best = {TX, TY, G, MB, bulk ? 1 : 0}; }
+        if (ctx->tuneLog) fprintf(stderr, "stormgpu tuner: %s, tile %dx%d, %d fields an item, %d blocks an SM, %s: %.4f ms\n", kind == TK_WENO ? "WENO" : "dynamics",
+                                  TX, TY, fields, MB, bulk ? "bulk copies" : "per-thread copies", ms);
+        if (ms >= bestMs[kind == TK_DYN]) continue;
+        bestMs[kind == TK_DYN] = ms;
+        if (kind == TK_WENO) { best[0] = TX; best[1] = TY; best[2] = G; best[3] = MB; best[4] = bulk; }
+        else { best[5] = TX; best[6] = TY; best[7] = bulk; }
       }
     }
     cudaEventDestroy(e0); cudaEventDestroy(e1);
     ctx->tuning[sig] = best;
   }
-  P.TX = best[0]; P.TY = best[1]; P.wenoG = best[2]; P.minb = best[3]; P.bulk = best[4] != 0; P.tuned = true;
+  P.TX = best[0]; P.TY = best[1]; P.wenoG = best[2]; P.minb = best[3]; P.bulk = best[4] != 0;
+  P.dTX = best[5]; P.dTY = best[6]; P.dBulk = best[7] != 0; P.tuned = true;
   return SG_OK;
 }
 
@@ -718,18 +730,16 @@ void enqueue_dynamics_graph(sg_context* ctx, const Plan& P) {
   launch_face_correct(node, A);
   cudaEventRecord(ev[1], main);
   cudaStreamWaitEvent(side, ev[1], 0);  // the face fluxes
-  Launch W = lx(ctx, P, FAM_T_WENO), D = lx(ctx, P, FAM_T_DYN);
-  W.cap = W.n; D.cap = D.n; W.stream = side;
   const int in[3] = {A, B, C}, out[3] = {B, C, B};
   // ev[2 + s]: WENO stage s done; ev[5]: dynamics stage 1 done; ev[6]: the sedimentation done
   for (int s = 0; s < 3; s++) {
     if (s == 2) cudaStreamWaitEvent(side, ev[5], 0);     // dynamics stage 1 has read set B's scalars
-    if (W.n) launch_transport(W, TK_WENO, P.wenoG, P.minb, in[s], out[s], (float)RK3[s], s, P.TX, P.TY, P.bulk, ctx->edgeWarps);
+    launch_transport_kind(ctx, P, TK_WENO, in[s], out[s], (float)RK3[s], s, side);
     launch_charges(ctx, P, in[s], out[s], (float)RK3[s], s, side);
     cudaEventRecord(ev[2 + s], side);
     // the stage's input scalars: for stage 0 the step-start fields after the sedimentation, later the WENO stage's
     cudaStreamWaitEvent(main, s == 0 ? ev[6] : ev[1 + s], 0);
-    if (D.n) launch_transport(D, TK_DYN, P.wenoG, P.minb, in[s], out[s], (float)RK3[s], s, P.TX, P.TY, P.bulk, ctx->edgeWarps);
+    launch_transport_kind(ctx, P, TK_DYN, in[s], out[s], (float)RK3[s], s, main);
     if (s == 1) cudaEventRecord(ev[5], main);
     if (s < 2) enqueue_project(ctx, P, out[s], 0, main, none);
   }
