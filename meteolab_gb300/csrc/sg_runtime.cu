@@ -412,7 +412,10 @@ int upload_items(sg_context* ctx, Plan& P, std::vector<int4>* all) {
   for (int f = 0; f < FAM_COUNT; f++) { P.off[f] = (int)flat.size(); P.cnt[f] = (int)all[f].size(); flat.insert(flat.end(), all[f].begin(), all[f].end()); }
   if (P.items) { cudaFree(P.items); P.items = nullptr; }
   CK(cudaMalloc(&P.items, flat.size() * sizeof(int4)));
-  CK(cudaMemcpy(P.items, flat.data(), flat.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  // on the context's stream and waited for: a plain cudaMemcpy from pageable memory may return before its last bytes are on
+  // the device, and the context's streams, which do not wait for the legacy stream, would then read items not yet written
+  CK(cudaMemcpyAsync(P.items, flat.data(), flat.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
   return SG_OK;
 }
 
@@ -1160,7 +1163,9 @@ static int pack_items(sg_context* ctx, const sg_run* runs, int n, uint32_t mask,
     }
     int4* d = nullptr;
     CK(cudaMalloc(&d, items.size() * sizeof(int4)));
-    CK(cudaMemcpy(d, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    cudaError_t e = cudaMemcpyAsync(d, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // (before any stream reads them, as in upload_items)
+    if (e != cudaSuccess) { cudaFree(d); return cudaFail(ctx, e, "placing items"); }
     if (ctx->packs.size() > 64) { for (auto& p : ctx->packs) cudaFree(p.second.first); ctx->packs.clear(); }
     it = ctx->packs.emplace(key, std::make_pair(d, (int)items.size())).first;
   }
