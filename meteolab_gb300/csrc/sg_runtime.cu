@@ -568,10 +568,12 @@ void launch_transport_kinds(sg_context* ctx, const Plan& P, int in, int out, flo
 }
 
 // Picks the plan's transport tiles (TX x TY columns) and WENO fields per item, before its items are made, by timing every
-// candidate on the plan's own runs: each of the two transport kinds of one RK3 stage by itself (set A in, set C out; C is
-// scratch between steps), best of three after a warm-up. Tuned together, the kinds shared a tile that suited their sum:
-// 16 standard runs 1.08 ms a step, tuned apart 1.00. Results are cached per batch signature (the sorted grid shapes, the run count to a power of two, and the
-// concurrent groups), so a serving loop whose batch changes run by run tunes each kind of batch once.
+// candidate on the plan's own runs: each of the two transport kinds of one RK3 stage by itself, the WENO fields with the
+// extra ones, which share their tile (set A in, set C out; C is scratch between steps), best of three after a warm-up.
+// Tuned together, the kinds shared a tile that suited their sum: 16 standard runs 1.08 ms a step, tuned apart 1.00; tuned
+// without the extra fields, 32 two-moment runs took 2.74 or 2.91 ms by chance. Results are cached per batch signature (the
+// sorted grid shapes, the run count to a power of two, the concurrent groups and the extra fields), so a serving loop
+// whose batch changes run by run tunes each kind of batch once.
 int autotune_transport(sg_context* ctx, Plan& P) {
   std::vector<int> sig;
   for (int s : P.slots) { const Run& r = ctx->runs[s]; sig.push_back(r.nx); sig.push_back(r.ny); sig.push_back(r.nz); }
@@ -585,6 +587,9 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     int c = 1; while (c < (int)P.slots.size()) c *= 2;
     sig.push_back(c);
     sig.push_back(P.share);
+    int extra = 0;
+    for (int s : P.slots) extra |= ctx->runs[s].desc.flags & RF_EXTRA;
+    sig.push_back(extra);
   }
   std::array<int, 8> best{P.TX, P.TY, P.wenoG, P.minb, P.bulk, P.dTX, P.dTY, P.dBulk};
   auto it = ctx->tuning.find(sig);
@@ -595,7 +600,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1));
     Plan T;  // candidate items only
-    T.slots = P.slots; T.share = P.share; T.maxnx = P.maxnx; T.maxny = P.maxny; T.maxnz = P.maxnz; T.minnx = P.minnx; T.nx4 = P.nx4;
+    T.slots = P.slots; T.share = P.share; T.extra = P.extra; T.maxnx = P.maxnx; T.maxny = P.maxny; T.maxnz = P.maxnz; T.minnx = P.minnx; T.nx4 = P.nx4;
     float bestMs[2] = {1e30f, 1e30f};
     for (auto& sh : shapes) for (int kind : {TK_WENO, TK_DYN}) {
       const int TX = sh[0], TY = sh[1];
@@ -609,6 +614,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
         if ((bulk ? transport_smem_bulk(kind, fields, TX, TY) : transport_smem(kind, fields, TX, TY)) > (size_t)ctx->maxSmem) continue;
         std::vector<int4> all[FAM_COUNT];
         transport_items(ctx, T, kind, TX, TY, G, bulk, all[kind == TK_WENO ? FAM_T_WENO : FAM_T_DYN]);
+        if (kind == TK_WENO && T.extra) charge_items(ctx, T, TX, TY, all[FAM_T_CHG], all[FAM_T_CHG3]);
         int st = upload_items(ctx, T, all);
         if (st != SG_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return st; }
         T.TX = T.dTX = TX; T.TY = T.dTY = TY; T.wenoG = G; T.minb = MB; T.bulk = T.dBulk = bulk;
@@ -616,6 +622,7 @@ int autotune_transport(sg_context* ctx, Plan& P) {
         for (int rep = 0; rep < 4; rep++) {
           cudaEventRecord(e0, ctx->stream);
           launch_transport_kind(ctx, T, kind, 0, 2, 1.f / 3.f, 0, ctx->stream);
+          if (kind == TK_WENO && T.extra) launch_charges(ctx, T, 0, 2, 1.f / 3.f, 0, ctx->stream);
           cudaEventRecord(e1, ctx->stream);
           CK(cudaEventSynchronize(e1));
           float t = 0; cudaEventElapsedTime(&t, e0, e1);
