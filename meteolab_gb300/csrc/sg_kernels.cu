@@ -893,11 +893,15 @@ __global__ void __launch_bounds__(256, 5) k_proj_div_fft2(const RunDesc* __restr
 // modes zero): per level the forward sweep d_k = A_k r_k - B_k d_(k-1) and the back substitution x_k = d_k - C_k x_(k+1),
 // one real recurrence a thread (n, real/imaginary part), the two parts sharing the coefficients. FACE: rows -rho h lambda
 // + vertical faces (src/core/advection.ts:222-241); PRES: the density-weighted consistent Laplacian
-// (src/core/pressure.ts:104-140). Values enter and leave FP64 through the integer-pipe conversions. An x-wavenumber's
+// (src/core/pressure.ts:104-140). Values enter and leave FP64 through the integer-pipe conversions or, where the launch gives
+// an SM at most one block (HW), by the hardware's: the FP64 pipe then idles and their latency is shorter (one run's step 278
+// -> 268 us); with two blocks an SM and more the pipe is the scarcer one (16 runs' solves 22 -> 23 us, 64 runs' 36 -> 42).
+// An x-wavenumber's
 // recurrences are split over blockIdx.y: nothing is shared between them, and blocks of two warps fill the SMs evenly.
 // Bound by the latency of its loads along the column: with the next eight levels' coefficients and values loaded while
 // eight levels step, 64 runs take 35 us a solve instead of 49, one run 19 instead of 22.
 constexpr int SWEEP_THREADS = 64;
+template <bool HW>
 __global__ void __launch_bounds__(SWEEP_THREADS) k_proj_sweep(const RunDesc* __restrict__ runs, const int4* items, int nitems, int mode) {
   FOR_ITEMS {
     const RunDesc& R = runs[items[it].x];
@@ -909,6 +913,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_proj_sweep(const RunDesc* __r
     float* g = reinterpret_cast<float*>(R.spec + (size_t)m * nzc * ny) + c;
     const TriAB* AB = (mode == PROJ_FACE ? R.tri_face : R.tri_pres) + (size_t)m * nzc * ny;
     const double* Cc = reinterpret_cast<const double*>((mode == PROJ_FACE ? R.tri_face : R.tri_pres) + (size_t)R.nm * nzc * ny) + (size_t)m * nzc * ny;
+    auto in = [](float v) { return HW ? (double)v : widen(v); };
+    auto out = [](double v) { return HW ? (float)v : narrow(v); };
     double d[MAXNZ];
     double prev = 0;
     // levels in blocks of 8, the next block's coefficients and values on their way while this block's recurrence steps
@@ -929,7 +935,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_proj_sweep(const RunDesc* __r
       if (k0 + 8 < nzc) load(k0 + 8);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        if (k0 + j < nzc) { prev = fma(-ab[j].b, prev, widen(__fmul_rn(ab[j].a, r[j]))); d[k0 + j] = prev; }
+        if (k0 + j < nzc) { prev = fma(-ab[j].b, prev, in(__fmul_rn(ab[j].a, r[j]))); d[k0 + j] = prev; }
       }
     }
     double cc[8], dd[8], ccn[8], ddn[8];
@@ -939,7 +945,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_proj_sweep(const RunDesc* __r
     };
     load_back(nzc - 2);
     double x = d[nzc - 1];
-    g[2 * ((size_t)(nzc - 1) * ny + n)] = narrow(x);
+    g[2 * ((size_t)(nzc - 1) * ny + n)] = out(x);
     for (int k1 = nzc - 2; k1 >= 0; k1 -= 8) {
 #pragma unroll
       for (int j = 0; j < 8; j++) { cc[j] = ccn[j]; dd[j] = ddn[j]; }
@@ -947,7 +953,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_proj_sweep(const RunDesc* __r
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         const int k = k1 - j;
-        if (k >= 0) { x = fma(-cc[j], x, dd[j]); g[2 * ((size_t)k * ny + n)] = narrow(x); }
+        if (k >= 0) { x = fma(-cc[j], x, dd[j]); g[2 * ((size_t)k * ny + n)] = out(x); }
       }
     }
   }
@@ -1816,10 +1822,12 @@ size_t layer_fft_smem_run(int nx, int ny) {
 void launch_proj_div_fft2(const Launch& L, int mode, int set, size_t smem) {
   k_proj_div_fft2<<<GRID(L.n, L.cap), 256, smem, L.stream>>>(L.runs, L.items, L.n, mode, set);
 }
-void launch_proj_sweep(const Launch& L, int mode, int maxny) {
+void launch_proj_sweep(const Launch& L, int mode, int maxny, int sms) {
+  const bool hw = (size_t)L.n * ((2 * maxny + SWEEP_THREADS - 1) / SWEEP_THREADS) <= (size_t)sms;
   dim3 grid = GRID(L.n, L.cap);
   grid.y = (2 * maxny + SWEEP_THREADS - 1) / SWEEP_THREADS;
-  k_proj_sweep<<<grid, SWEEP_THREADS, 0, L.stream>>>(L.runs, L.items, L.n, mode);
+  if (hw) k_proj_sweep<true><<<grid, SWEEP_THREADS, 0, L.stream>>>(L.runs, L.items, L.n, mode);
+  else k_proj_sweep<false><<<grid, SWEEP_THREADS, 0, L.stream>>>(L.runs, L.items, L.n, mode);
 }
 void launch_proj_ifft2(const Launch& L, int mode, size_t smem) {
   k_proj_ifft2<<<GRID(L.n, L.cap), 256, smem, L.stream>>>(L.runs, L.items, L.n, mode);

@@ -656,7 +656,7 @@ void enqueue_solve(sg_context* ctx, const Plan& P, int mode, int set, cudaStream
     modes.cap = modes.n;  // one block per wavenumber: its column solves are serial in z, so spread them over the SMs
     rows.stream = modes.stream = stream;
     launch_proj_div_fft2(rows, mode, set, P.fftSmem); hook(h);
-    launch_proj_sweep(modes, mode, P.maxny); hook(h + 1);
+    launch_proj_sweep(modes, mode, P.maxny, ctx->sms); hook(h + 1);
     launch_proj_ifft2(rows, mode, P.fftSmem); hook(h + 2);
   }
   if (P.rowAny) {  // the runs of the row path
@@ -668,7 +668,7 @@ void enqueue_solve(sg_context* ctx, const Plan& P, int mode, int set, cudaStream
     cols.cap = cols.n; cols.stream = stream;
     launch_proj_div_xfft(rows, mode, set, P.yc, P.rowMaxnx); hook(h);
     launch_proj_ycols(cols, mode, 0, P.ycolPoints);
-    launch_proj_sweep(modes, mode, P.rowMaxny);
+    launch_proj_sweep(modes, mode, P.rowMaxny, ctx->sms);
     launch_proj_ycols(cols, mode, 1, P.ycolPoints); hook(h + 1);
     launch_proj_xifft(rows, mode, P.yc, P.rowMaxnx); hook(h + 2);
   }
