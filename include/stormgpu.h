@@ -355,8 +355,8 @@ int sg_run_divergence(sg_context* ctx, sg_run run, double* max_abs_div);
  * The tuner also picks the WENO kernel's register budget. sg_set_transport_shape pins one shape for every later plan
  * (tile_x = 0 returns to tuning and forgets earlier results, so the next plan of a batch is tuned on its runs as they are
  * then, e.g. developed storms after a spin-up; register budget for 2 blocks per SM); results are the same bits
- * for every shape. sg_batch_transport_shape reports the shape a batch runs with. No counterpart in the reference (its
- * CPU transport has no tiles). */
+ * for every shape. The tuner gives the dynamics a tile of its own; a pinned shape holds for both. sg_batch_transport_shape
+ * reports the shape a batch's WENO fields run with. No counterpart in the reference (its CPU transport has no tiles). */
 int sg_set_transport_shape(sg_context* ctx, int tile_x, int tile_y, int weno_group);
 /* shape4 = (tile_x, tile_y, weno_group, blocks per SM the WENO kernel's register budget is cut for: 2 or 3). */
 int sg_batch_transport_shape(sg_context* ctx, const sg_run* runs, int n, int* shape4);

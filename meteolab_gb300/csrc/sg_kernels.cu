@@ -896,9 +896,8 @@ __global__ void __launch_bounds__(256, 5) k_proj_div_fft2(const RunDesc* __restr
 // (src/core/pressure.ts:104-140). Values enter and leave FP64 through the integer-pipe conversions or, where the launch gives
 // an SM at most one block (HW), by the hardware's: the FP64 pipe then idles and their latency is shorter (one run's step 278
 // -> 268 us); with two blocks an SM and more the pipe is the scarcer one (16 runs' solves 22 -> 23 us, 64 runs' 36 -> 42).
-// An x-wavenumber's
-// recurrences are split over blockIdx.y: nothing is shared between them, and blocks of two warps fill the SMs evenly.
-// Bound by the latency of its loads along the column: with the next eight levels' coefficients and values loaded while
+// An x-wavenumber's recurrences are split over blockIdx.y: nothing is shared between them, and blocks of two warps fill the
+// SMs evenly. Bound by the latency of its loads along the column: with the next eight levels' coefficients and values loaded while
 // eight levels step, 64 runs take 35 us a solve instead of 49, one run 19 instead of 22.
 constexpr int SWEEP_THREADS = 64;
 template <bool HW>

@@ -502,8 +502,9 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, int share, Plan& 
     if (r.desc.flags & RF_RAIN2M) P.rain2m = true;
   }
   // mixing items and, for refined runs, refinement items: (run, tile, z0, z1). A column is cut into four level ranges, and
-  // where the batch's tiles are few into as many as give each SM an item, of at least six levels (each range reloads the
-  // planes at its ends): one standard run's mixing 28 -> 21 us, its refinement 25 -> 18.
+  // where the batch's tiles are few into as many as give each SM an item, of at least three levels (each range reloads the
+  // planes at its ends): one standard run's mixing took 28 us in four ranges, 18 in eight, 15 in sixteen, its refinement 25, 18
+  // and 14.
   auto ranges = [&](int TX, int TY, int fam, bool refinedOnly) {
     size_t tilesAll = 0;
     for (int s : slots) { const Run& r = ctx->runs[s]; tilesAll += (size_t)((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY); }
@@ -511,7 +512,7 @@ int build_plan(sg_context* ctx, const std::vector<int>& slots, int share, Plan& 
       const Run& r = ctx->runs[s];
       if (refinedOnly && !(r.desc.flags & RF_REFINE)) continue;
       const int tiles = ((r.nx + TX - 1) / TX) * ((r.ny + TY - 1) / TY);
-      const int cuts = std::max(4, std::min((int)((size_t)ctx->sms / (tilesAll * P.share)), r.nz / 6)), zc = (r.nz + cuts - 1) / cuts;
+      const int cuts = std::max(4, std::min((int)((size_t)ctx->sms / (tilesAll * P.share)), r.nz / 3)), zc = (r.nz + cuts - 1) / cuts;
       for (int t = 0; t < tiles; t++)
         for (int z0 = 0; z0 < r.nz; z0 += zc) all[fam].push_back(make_int4(s, t, z0, std::min(r.nz, z0 + zc)));
     }
