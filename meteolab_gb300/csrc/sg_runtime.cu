@@ -257,9 +257,7 @@ void build_tables(const sg_grid* g, const sg_base_state* b, const sg_switches* s
   // Face projection factorisation [m][k][n] (src/core/advection.ts:222-241): rows -rho h lambda - lo - up.
   T.triF.assign((size_t)nm * nz * ny, TriAB{0, 0.f, 0.f}); T.triFc.assign((size_t)nm * nz * ny, 0.0);
   auto faceRho = [&](int k) { return k < 0 || k >= nz - 1 ? 0.0 : (rho[k] + rho[k + 1]) / 2; };
-  split(nm, (size_t)nm * nz * ny, [&](int m0, int m1) {
-  double cp[128];
-  for (int m = m0; m < m1; m++) for (int n = 0; n < ny; n++) {
+  split(nm, (size_t)nm * nz * ny, [&](int m0, int m1) { double cp[128]; for (int m = m0; m < m1; m++) for (int n = 0; n < ny; n++) {
     double lam = (m == 0 && n == 0) ? 0 : 4 * std::pow(std::sin(M_PI * m / nx), 2) / (dx * dx) + 4 * std::pow(std::sin(M_PI * n / ny), 2) / (dy * dy);
     bool pinned = lam == 0;
     for (int k = 0; k < nz; k++) {
@@ -273,16 +271,13 @@ void build_tables(const sg_grid* g, const sg_base_state* b, const sg_switches* s
       T.triF[((size_t)m * nz + k) * ny + n] = TriAB{ip * lower, (float)(ip * hz[k]), 0.f};
       T.triFc[((size_t)m * nz + k) * ny + n] = cp[k];
     }
-  }
-  });
+  } });
   // Pressure factorisation [m][k][n] (src/core/pressure.ts:37-44, :104-140), the symbols snapped as there.
   const int nc = nz - 1;
   T.triP.assign((size_t)nm * nc * ny, TriAB{0, 0.f, 0.f}); T.triPc.assign((size_t)nm * nc * ny, 0.0);
   T.ab.assign((size_t)nm * ny, make_double2(0, 0));
   auto exact = [](double x) { return x < 1e-12 ? 0 : x > 1 - 1e-12 ? 1 : x; };
-  split(nm, (size_t)nm * nc * ny, [&](int m0, int m1) {
-  double cp[128];
-  for (int m = m0; m < m1; m++) for (int n = 0; n < ny; n++) {
+  split(nm, (size_t)nm * nc * ny, [&](int m0, int m1) { double cp[128]; for (int m = m0; m < m1; m++) for (int n = 0; n < ny; n++) {
     double sx = exact(std::pow(std::sin(M_PI * m / nx), 2)), cx = exact(std::pow(std::cos(M_PI * m / nx), 2));
     double sy = exact(std::pow(std::sin(M_PI * n / ny), 2)), cy = exact(std::pow(std::cos(M_PI * n / ny), 2));
     double a = 4 * (sx * cy / (dx * dx) + cx * sy / (dy * dy)), bb = cx * cy;
@@ -301,8 +296,7 @@ void build_tables(const sg_grid* g, const sg_base_state* b, const sg_switches* s
       T.triP[((size_t)m * nc + k) * ny + n] = TriAB{ip * lo, (float)ip, 0.f};
       T.triPc[((size_t)m * nc + k) * ny + n] = cp[k];
     }
-  }
-  });
+  } });
   twiddles(nx, T.twx); twiddles(ny, T.twy);
   d.nx = nx; d.ny = ny; d.nz = nz; d.layer = nx * ny; d.n = nx * ny * nz; d.nm = nm; d.mh = nx / 2; d.ncells = nx * ny * (nz - 1);
   d.fx_nf = fft_plan_factors(nx, d.fx_rad); d.fy_nf = fft_plan_factors(ny, d.fy_rad);
