@@ -205,6 +205,9 @@ __device__ __forceinline__ void transport_item(const RunDesc& Rg, int group, int
       if (g + 1 < G) fzD[g + 1] = mzD * r.y;
     }
   }
+  // the slab's first level copies plane z0 + 4 into the slot of z0 - 3, which that face has just read (a whole column's
+  // first level fills a slot no face reads)
+  if (z0 > 0) __syncthreads();
   for (int z = z0; z < z1; z++) {
     const int buf = z & 1, l = z * layer;
     const bool more = z + 1 < z1;
