@@ -191,14 +191,14 @@ SG_D double weightOf(double pj, double inv, int node, unsigned tag, int layer, i
 }
 
 // add() of Lightning.flash (:294-304) and extend() (:389-404) by one warp, all 32 lanes, on the block's copy of the state
-// record and the front. Lane l takes the l-th candidate of the reference's loop (level k from z - 1 up, then dj, then
-// di); the candidates are distinct nodes, so each lane keeps its node's shorter link on its own, and the new links go on
-// the front in the reference's order (a ballot over the lanes). Everything the candidates need is loaded before the
-// potential's sum and divide, which take their latency's time.
-SG_D void addNodeWarp(const RunDesc& R, const LgtDev& L, const Front& F, volatile LgtState& V, int j, int from, bool clear, double pj, int id,
+// record and the front: node j, the channel's nn-th. Lane l takes the l-th candidate of the reference's loop (level k from
+// z - 1 up, then dj, then di); the candidates are distinct nodes, so each lane keeps its node's shorter link on its own,
+// and the new links go on the front in the reference's order (a ballot over the lanes). Everything the candidates need is
+// loaded before the potential's sum and its quotient, which take their latency's time.
+SG_D void addNodeWarp(const RunDesc& R, const LgtDev& L, const Front& F, volatile LgtState& V, int j, int nn, int from, bool clear, double pj, int id,
                       double count, double icount) {
   const int lane = threadIdx.x & 31, nx = R.nx, ny = R.ny, nz = R.nz, layer = R.layer;
-  const int z = j / layer, y = (j - z * layer) / nx, x = j - z * layer - y * nx, nn = V.nnodes;
+  const int z = j / layer, y = (j - z * layer) / nx, x = j - z * layer - y * nx;
   int q = -1, reach = 0, mark = 0, seen = 0, pos = -1;
   bool upward = false;
   double rho = 0, phi = 0;
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(GROW_THREADS) k_lgt_grow(const RunDesc R, cons
       V.start = start; V.id = id;
     }
     __syncthreads();
-    if (warp == 0) addNodeWarp(R, L, F, V, start, -1, clearOf(L.rho[start], L.cloudy[start]), L.phi[start], id, 1.0, 1.0);
+    if (warp == 0) addNodeWarp(R, L, F, V, start, 0, -1, clearOf(L.rho[start], L.cloudy[start]), L.phi[start], id, 1.0, 1.0);
   } else {
     for (int f = t; f < V.size; f += GROW_THREADS) {
       // the last stage's deposit changed the charge: the potentials and the clear air are the present ones
@@ -318,8 +318,9 @@ __global__ void __launch_bounds__(GROW_THREADS) k_lgt_grow(const RunDesc R, cons
   if (warp == 0) ahead(0, rng, V.nnodes + 1);
   __syncthreads();
   for (int iter = 0; iter < MAX_CHANNEL; iter++) {
-    if (V.nnodes >= MAX_CHANNEL || V.size == 0) break;
-    const int size = V.size, ground = V.ground;
+    // what the holder changes below is read here, before the barrier: past it the holder may be ahead of any other thread
+    const int size = V.size, ground = V.ground, nodes = V.nnodes, left = V.left;
+    if (nodes >= MAX_CHANNEL || size == 0) break;
     const double before = V.before, potential = V.potential;
     const int C = ((size + GROW_THREADS - 1) / GROW_THREADS) | 1, f0 = min(size, t * C), f1 = min(size, f0 + C);
     double acc = 0;
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(GROW_THREADS) k_lgt_grow(const RunDesc R, cons
     int holder = W - 1;
 #pragma unroll
     for (int w = W - 2; w >= 0; w--) if (bitsOf(pick) <= bitsOf(upTo[w])) holder = w;
-    if (warp == (holder + 1) % W) ahead((iter + 1) & 1, rng, V.nnodes + 2);
+    if (warp == (holder + 1) % W) ahead((iter + 1) & 1, rng, nodes + 2);
     if (warp == holder) {
       // the part, then the link (by scans over its weights)
       const unsigned parts = __ballot_sync(ALL, bitsOf(acc) != 0 && bitsOf(pick) <= bitsOf(dadd(mine, inc)));
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(GROW_THREADS) k_lgt_grow(const RunDesc R, cons
       const double pj = linkPj(F, L, n);
       const bool clear = tag & TAG_CLEAR;
       __syncwarp();
-      if (!V.left && ground < 0 && clear) {  // the first step out of the cloud
+      if (!left && ground < 0 && clear) {  // the first step out of the cloud
         if (lane == 0) { V.left = 1; V.event = 1; stop = 1; }
       } else {
         int m = size - 1;
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(GROW_THREADS) k_lgt_grow(const RunDesc R, cons
         }
         if (lane == 0) V.size = m;
         __syncwarp();
-        addNodeWarp(R, L, F, V, j, from, clear, pj, id, next[iter & 1].n, next[iter & 1].inv);
+        addNodeWarp(R, L, F, V, j, nodes, from, clear, pj, id, next[iter & 1].n, next[iter & 1].inv);
         if (lane == 0 && V.touched) { V.touched = 0; V.event = 1; stop = 1; }
       }
     }

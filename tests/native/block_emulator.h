@@ -12,6 +12,7 @@
 #include <cstring>
 #include <functional>
 #include <vector>
+#include <cstdio>
 
 namespace emu {
 
@@ -91,7 +92,7 @@ inline bool run(int threads, int order, const std::function<void()>& body) {
     if (next) { b.self = next; swapcontext(&b.home, &next->ctx); continue; }
     bool ended = true, all = true;
     for (const Thread& f : b.threads) { ended = ended && f.state == Thread::ENDED; all = all && (f.state == Thread::BARRIER || f.state == Thread::ENDED); }
-    if (ended || !all) { b.deadlock = !ended; break; }
+    if (ended || !all) { b.deadlock = !ended; if(!ended) for (const Thread& f : b.threads) fprintf(stderr,"%d:%d(%u) ", f.id, (int)f.state, f.generation); break; }
     for (Thread& f : b.threads) if (f.state == Thread::BARRIER) f.state = Thread::READY;
   }
   block() = nullptr;
@@ -117,8 +118,8 @@ inline Dim block_dim() { return Dim{(unsigned)block()->threads.size()}; }
 #define __launch_bounds__(...)
 #define __forceinline__ inline
 
-using std::max;
-using std::min;
+inline int min(int a, int b) { return a < b ? a : b; }
+inline int max(int a, int b) { return a > b ? a : b; }
 inline void __syncthreads() { emu::barrier(); }
 inline void __syncwarp() { emu::collect(0); }
 template <class T> T __shfl_sync(unsigned, T v, int lane) { return emu::from<T>(emu::collect(emu::bits(v))[lane & 31]); }

@@ -63,3 +63,66 @@ def test_slabs_of_levels_give_the_whole_columns_bits_whichever_warp_is_ahead(tra
     for order in range(2 + threads // 32):
         assert np.array_equal(stage(1, order), want), order
         assert np.array_equal(stage(slabs, order), want), order
+
+
+MAX_CHANNEL = 3000
+GROW_WARPS = 4
+
+
+def _growth(tmp, front):
+    """The channel's growth with `front` links of its front in shared memory."""
+    helpers = _excerpt("sg_lightning.cu", "constexpr double EPS0", "// Block sum in a fixed order")
+    grow = _excerpt("sg_lightning.cu", "// The state record in shared memory", "// deposit() (:352-381)")
+    for old, new in (("constexpr int FRONT = 5120", f"constexpr int FRONT = {front}"), ("extern __shared__ double fsm[];", "double* fsm = dynamic_shared.data();")):
+        assert grow.count(old) == 1
+        grow = grow.replace(old, new)
+    return _compile(tmp, "lightning_block", {"lightning_helpers.inc": helpers, "lightning_grow.inc": grow})
+
+
+@pytest.fixture(scope="module")
+def growth(tmp_path_factory):
+    return _growth(tmp_path_factory.mktemp("growth"), 5120)
+
+
+def _flash(lib, seed, order, stages=3):
+    """A flash in a storm of two charge layers, clear air around its cloud; later stages on a weakened, disturbed field."""
+    nx, ny, nz = 14, 12, 16
+    rng = np.random.default_rng(seed)
+    zs = np.cumsum(rng.uniform(300, 500, nz)) - 300
+    air = 1.2 * np.exp(-zs / 9000)
+    z, y, x = np.meshgrid(zs / zs[-1], np.arange(ny) / ny, np.arange(nx) / nx, indexing="ij")
+    inside = np.exp(-((x - .5) ** 2 + (y - .5) ** 2) / .08)
+    base = 4e8 * inside * np.sin(2 * np.pi * z) * (1 + .2 * rng.standard_normal((nz, ny, nx)))
+    base[0] = base[-1] = 0
+    phi = np.ascontiguousarray([base * f + 1e6 * rng.standard_normal(base.shape) * (z > 0) for f in np.linspace(1, .7, stages)])
+    rho = np.where(inside > .15, 1e-9 * np.sin(2 * np.pi * z), 0.)
+    cloudy = np.where(inside > .3, 1e-3, 0.).astype(np.float32)
+    start = int(np.ravel_multi_index((nz // 4, ny // 2, nx // 2), (nz, ny, nx)))
+    out, state = np.zeros(2 * MAX_CHANNEL, np.int32), np.zeros(7)
+    dp = C.POINTER(C.c_double)
+    lib.lb_flash.argtypes = [C.c_int] * 3 + [C.c_double] * 2 + [dp] * 4 + [C.POINTER(C.c_float), C.c_int, C.c_int, C.c_uint, C.c_int, C.POINTER(C.c_int), dp]
+    d = lambda a: np.ascontiguousarray(a, float).ctypes.data_as(dp)  # noqa: E731
+    largest = lib.lb_flash(nx, ny, nz, 1000., 900., d(zs), d(air), d(rho), d(phi), _fp(cloudy), stages, start, 1000 + seed, order,
+                           out.ctypes.data_as(C.POINTER(C.c_int)), d(state))
+    return largest, out, state
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_a_channel_grows_the_same_whichever_warp_is_ahead(growth, seed):
+    largest, nodes, state = _flash(growth, seed, 0)
+    assert largest > 128 and state[0] > 40, (largest, state)  # a front of several links a thread, a channel of many picks
+    for order in range(1, 2 + GROW_WARPS):
+        got = _flash(growth, seed, order)
+        assert got[0] == largest and np.array_equal(got[1], nodes) and np.array_equal(got[2], state), order
+
+
+@pytest.mark.parametrize("front", [64, 200])
+def test_a_front_longer_than_shared_memory_grows_the_same_channel(growth, tmp_path, front):
+    """Links past the front's part in shared memory live in the run's buffers: the same picks and the same channel."""
+    lib = _growth(tmp_path, front)
+    for seed in (1, 2, 3):
+        largest, nodes, state = _flash(growth, seed, 0)
+        assert largest > front
+        for order in (0, 1, 3):
+            got = _flash(lib, seed, order)
+            assert got[0] == largest and np.array_equal(got[1], nodes) and np.array_equal(got[2], state), (seed, order)
