@@ -2,7 +2,7 @@
 // waits (a block barrier or a warp's collective), and of the threads that can run the scheduler always takes the first
 // in a given order of the warps and lanes. So a warp can be let run ahead of the others as far as its barriers allow, a
 // schedule the device may pick too; code whose results depend on the order lacks a barrier. Asynchronous copies land
-// when they are issued (the earliest they may).
+// when they are issued or, with `late`, when their thread waits for them: the earliest and the latest they may.
 #pragma once
 #include <cuda_runtime.h>
 #include <ucontext.h>
@@ -11,17 +11,21 @@
 #include <cstdint>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <vector>
 #include <cstdio>
 
 namespace emu {
 
+constexpr size_t STACK = 256 * 1024;
 struct Thread {
   ucontext_t ctx;
-  std::vector<char> stack;
+  std::unique_ptr<char[]> stack;
   int id = 0;
   enum { READY, BARRIER, WARP, ENDED } state = READY;
   unsigned generation = 0;  // warp collectives this thread has entered
+  struct Copy { void* to; const void* from; size_t bytes; };
+  std::vector<Copy> copies;  // not yet landed
 };
 struct Warp {
   uint64_t values[2][32];
@@ -34,7 +38,7 @@ struct Block {
   ucontext_t home;
   Thread* self = nullptr;
   std::function<void()> body;
-  bool deadlock = false;
+  bool late = false, deadlock = false;
 };
 inline Block*& block() { static Block* b = nullptr; return b; }
 
@@ -65,19 +69,28 @@ inline const uint64_t* collect(uint64_t v) {
   }
   return w.values[side];
 }
+inline void copy(void* to, const void* from, size_t bytes) {
+  if (block()->late) block()->self->copies.push_back({to, from, bytes});
+  else std::memcpy(to, from, bytes);
+}
+inline void land() {
+  for (const Thread::Copy& c : block()->self->copies) std::memcpy(c.to, c.from, c.bytes);
+  block()->self->copies.clear();
+}
 inline void barrier() { block()->self->state = Thread::BARRIER; yield(); }
 
 // Runs `body` as `threads` device threads (whole warps). order 0: warps and lanes ascending; 1: both descending; k >= 2:
 // warp k - 2 first, then ascending. False where the threads wait for one another forever.
-inline bool run(int threads, int order, const std::function<void()>& body) {
+inline bool run(int threads, int order, const std::function<void()>& body, bool late = false) {
   Block b;
+  b.late = late;
   b.threads.resize(threads); b.warps.resize(threads / 32); b.body = body;
   block() = &b;
   for (int t = 0; t < threads; t++) {
     Thread& f = b.threads[t];
-    f.id = t; f.stack.resize(256 * 1024);
+    f.id = t; f.stack.reset(new char[STACK]);
     getcontext(&f.ctx);
-    f.ctx.uc_stack.ss_sp = f.stack.data(); f.ctx.uc_stack.ss_size = f.stack.size(); f.ctx.uc_link = &b.home;
+    f.ctx.uc_stack.ss_sp = f.stack.get(); f.ctx.uc_stack.ss_size = STACK; f.ctx.uc_link = &b.home;
     makecontext(&f.ctx, entry, 0);
     b.order.push_back(t);
   }
@@ -146,6 +159,6 @@ inline float __fdividef(float a, float b) { return a / b; }
 inline float2 __fmul2_rn(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 inline float2 __fadd2_rn(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 inline float2 __ffma2_rn(float2 a, float2 b, float2 c) { return make_float2(std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)); }
-inline void cp_async4(float* to, const float* from) { *to = *from; }
-inline void cp_async16(void* to, const void* from) { std::memcpy(to, from, 16); }
-inline void cp_async_wait_all() {}
+inline void cp_async4(float* to, const float* from) { emu::copy(to, from, 4); }
+inline void cp_async16(void* to, const void* from) { emu::copy(to, from, 16); }
+inline void cp_async_wait_all() { emu::land(); }

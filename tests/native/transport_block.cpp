@@ -12,9 +12,9 @@ enum TKind { TK_WENO = 0, TK_DYN = 1 };
 using namespace sg;
 
 // One stage (start set 0, input set `in`, output set 2) of a run's fields `fld` (three sets of the base fields), every
-// column cut into `slabs` slabs of levels, the threads of each block in the scheduler's order `order`. 0, or -1 where a
-// block's threads wait forever.
-extern "C" int tb_transport(int kind, int G, int ew, int TX, int TY, int nx, int ny, int nz, int slabs, int order, int flags, int in, int stage,
+// column cut into `slabs` slabs of levels, the threads of each block in the scheduler's order `order`, the copies landing
+// `late` or early. 0, or -1 where a block's threads wait forever.
+extern "C" int tb_transport(int kind, int G, int ew, int TX, int TY, int nx, int ny, int nz, int slabs, int order, int late, int flags, int in, int stage,
                             float* fld, float* faces, const float* lv) {
   RunDesc R{};
   R.nx = nx; R.ny = ny; R.nz = nz; R.layer = nx * ny; R.n = nx * ny * nz; R.flags = flags;
@@ -33,7 +33,7 @@ extern "C" int tb_transport(int kind, int G, int ew, int TX, int TY, int nx, int
         else if (G == 3 && ew) transport_item<TK_WENO, 3, 0, 0, true>(R, 0, tile, levels, in, 2, .5f, stage, TX, TY, sm);
         else if (G == 3) transport_item<TK_WENO, 3, 0, 0, false>(R, 0, tile, levels, in, 2, .5f, stage, TX, TY, sm);
         else transport_item<TK_WENO, 1, 0, 0, false>(R, 4, tile, levels, in, 2, .5f, stage, TX, TY, sm);
-      });
+      }, late != 0);
       if (!ended) return -1;
     }
   return 0;

@@ -53,9 +53,9 @@ def test_slabs_of_levels_give_the_whole_columns_bits_whichever_warp_is_ahead(tra
     lv = rng.uniform(.5, 1.5, 64 * nz).astype(np.float32)
     threads = 64 + (64 if ew else 0)
 
-    def stage(slabs, order):
+    def stage(slabs, order, late=0):
         fld = start.copy()
-        assert transport.tb_transport(kind, G, ew, 8, 8, nx, ny, nz, slabs, order, 64 | 1, 1, 1, _fp(fld), _fp(faces), _fp(lv)) == 0
+        assert transport.tb_transport(kind, G, ew, 8, 8, nx, ny, nz, slabs, order, late, 64 | 1, 1, 1, _fp(fld), _fp(faces), _fp(lv)) == 0
         return fld
 
     want = stage(1, 0)
@@ -63,6 +63,7 @@ def test_slabs_of_levels_give_the_whole_columns_bits_whichever_warp_is_ahead(tra
     for order in range(2 + threads // 32):
         assert np.array_equal(stage(1, order), want), order
         assert np.array_equal(stage(slabs, order), want), order
+        assert np.array_equal(stage(slabs, order, late=1), want), order
 
 
 MAX_CHANNEL = 3000
