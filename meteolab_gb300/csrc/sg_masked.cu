@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(TPB) k_mp_flux(const double* __restrict__ d, c
   }
 }
 
-// The column fluxes of the node winds (divergencePart, :240-264).
+// The column fluxes of the node winds (divergencePart, :240-264). Where a column has no open share of the layer the winds
+// are not read: what the arrays hold under the ground stays out, numbers or not.
 __global__ void __launch_bounds__(TPB) k_mp_wind_flux(const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
                                                       double* __restrict__ fu, double* __restrict__ fv, double* __restrict__ fw, Geo g) {
   const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -324,8 +325,9 @@ __global__ void __launch_bounds__(TPB) k_mp_wind_flux(const float* __restrict__ 
   const int k = (int)(c / g.layer);
   const size_t up = c + g.layer;
   const double a = g.A[c], b = g.B[c];
-  fu[c] = a * (double)u[c] + b * (double)u[up];
-  fv[c] = a * (double)v[c] + b * (double)v[up];
+  const bool open = b > 0;
+  fu[c] = open ? a * (double)u[c] + b * (double)u[up] : 0;
+  fv[c] = open ? a * (double)v[c] + b * (double)v[up] : 0;
   fw[c] = g.rho4[k + 1] * (double)w[up] - g.rho4[k] * (double)w[c];
 }
 

@@ -167,15 +167,16 @@ __global__ void __launch_bounds__(64) k_or_march(Geo g, int seg, int skip) {
   }
 }
 
-// The column fluxes of the node winds.
+// The column fluxes of the node winds; no wind is read where a column has no open share of the layer.
 __global__ void __launch_bounds__(TPB) k_or_wind(const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w, Geo g) {
   const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.cells) return;
   const int k = (int)(c / g.layer);
   const size_t up = c + g.layer;
   const double a = g.A[c], b = g.B[c];
-  g.fu[c] = __fma_rn(a, (double)u[c], __dmul_rn(b, (double)u[up]));
-  g.fv[c] = __fma_rn(a, (double)v[c], __dmul_rn(b, (double)v[up]));
+  const bool open = b > 0;
+  g.fu[c] = open ? __fma_rn(a, (double)u[c], __dmul_rn(b, (double)u[up])) : 0;
+  g.fv[c] = open ? __fma_rn(a, (double)v[c], __dmul_rn(b, (double)v[up])) : 0;
   g.fw[c] = __fma_rn(g.rho4[k + 1], (double)w[up], -__dmul_rn(g.rho4[k], (double)w[c]));
 }
 
