@@ -15,7 +15,7 @@
 // the block that ends last, from the partials in a fixed order (the result does not depend on scheduling); alpha, beta
 // and the stopping test stay on the device. Eight iterations are one CUDA graph,
 // replayed until the device's stop flag is set: the host reads one int per eight iterations (a projection whose rounding
-// would decide its iterations starts again in the reference's order of operations: sg_masked_ordered.cu); every kernel of an
+// would decide its iterations starts again in a fixed order of operations: sg_masked_ordered.cu); every kernel of an
 // iteration after the stop returns at once, so the iterations done, the residual and the result are those
 // of the reference's loop (:313-329), which stops at the first top-of-loop test it passes. The FP64 pipe bounds the
 // kernels (two operations a clock and SM), so their FP64 instructions are counted: see k_mp_flux and sg_spectral64.cuh.
@@ -432,7 +432,7 @@ __global__ void k_mp_update_xfwd(double* __restrict__ q, double* __restrict__ r,
 // rounding has come to decide the iterations (Paige 1976): over 220 solves on drawn grounds and grids, disturbed in the
 // last bit, those with |r . z0| below 1e-9 of sqrt(r.z r0.z0) throughout agreed to 6e-13, of the others nine in ten to no
 // better than 1e-10 and half to no better than 1e-6. A solve that passes 1e-9 (or 1e-14 r0.z0, which r.z alone would be
-// compared with at tighter tolerances) stops, and starts again in the reference's order of operations (OrderedSolve).
+// compared with at tighter tolerances) stops, and starts again in one fixed order of operations (OrderedSolve).
 // An iteration there takes 0.39 ms on 80 x 64 x 50 nodes, 0.11 here; what is given up took a quarter of the iterations.
 template <int OP, bool WATCH = false>
 __global__ void k_mp_xinv(const double2* __restrict__ S, double* __restrict__ out, const double* __restrict__ r, int nx, int ny, int pairs, Fft64 P,

@@ -20,11 +20,10 @@ using Geo = OrderedSolve;
 
 // x / d to the last bit, from r = 1 / d correctly rounded: x r is within 1.5 units, the first remainder brings it within
 // one, the second gives the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990). Five FP64 operations against a
-// divide's ten; finite operands away from underflow.
+// divide's ten; finite operands away from underflow, or a zero, whose sign the remainders would lose.
 __device__ __forceinline__ double quotient(double x, double d, double r) {
-  double q = __dmul_rn(x, r);
-  q = __fma_rn(__fma_rn(-q, d, x), r, q);
-  return __fma_rn(__fma_rn(-q, d, x), r, q);
+  const double q0 = __dmul_rn(x, r), q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0), q2 = __fma_rn(__fma_rn(-q1, d, x), r, q1);
+  return (__double_as_longlong(x) << 1) == 0 ? q0 : q2;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -1,7 +1,8 @@
-// The masked projection's conjugate gradients with every sum in the reference's order (src/core/terrain.ts:306-336):
-// direct Fourier sums, node by node gradients, quotients where the reference divides. sg_masked.cu runs it where the
-// solve's residuals lose their orthogonality, so that rounding decides the iterations and another order of operations
-// would give another answer: see k_mp_xinv's watch.
+// The masked projection's conjugate gradients (src/core/terrain.ts:306-336) in one order of operations that stays as it is:
+// the reference's where a value is formed (node by node gradients, quotients where it divides, direct Fourier sums from
+// the first term on), with the products fused into their sums, and trees over blocks of 256 for the dot products, which
+// the reference adds one by one. sg_masked.cu runs it where the solve's residuals lose their orthogonality, so that
+// rounding decides the iterations and every other order gives another answer: see k_mp_xinv's watch.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>

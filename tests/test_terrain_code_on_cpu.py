@@ -47,3 +47,23 @@ def test_winds_under_the_ground_stay_out_of_the_divergence(code):
     for junk in (np.nan, np.inf, 7e8):
         got = divergence(np.where(buried, junk, u).astype(np.float32), np.where(buried, junk, v).astype(np.float32))
         assert np.array_equal(got, want), junk
+
+
+def test_quotients_from_reciprocals_are_the_division_to_the_last_bit(code):
+    """x / d from 1 / d (Markstein 1990): the last bit of a division, over spacings, pivots and mode values of any size
+    the solve meets, over quotients next to a half of the last place, and over divisors whose reciprocal rounds the worst
+    (all bits set, and powers of two)."""
+    rng = np.random.default_rng(11)
+    n = 2_000_000
+    x = rng.standard_normal(n) * 10.0 ** rng.uniform(-60, 60, n)
+    d = rng.standard_normal(n) * 10.0 ** rng.uniform(-60, 60, n)
+    third = n // 3
+    # x the rounded product of d and a short number and its neighbours: quotients a hair off a double, or off a midpoint of two
+    y = np.round(rng.uniform(1, 2, third) * 2.0 ** 26) / 2.0 ** 26 + rng.integers(-2, 3, third) * 2.0 ** -53
+    x[:third] = np.nextafter(d[:third] * y, np.where(rng.random(third) < .5, np.inf, -np.inf))
+    ones = np.ldexp(2 - 2.0 ** -52, rng.integers(-100, 100, third))
+    d[third:2 * third] = np.where(rng.random(third) < .5, ones, np.ldexp(1.0, rng.integers(-100, 100, third)))
+    edge = [(0., 3.), (-0., 3.), (1., 3.), (np.pi, -7.), (1., 2 - 2.0 ** -52), (2 - 2.0 ** -52, 1 + 2.0 ** -52)]
+    x[-len(edge):], d[-len(edge):] = zip(*edge)
+    dp = lambda a: a.ctypes.data_as(DP)  # noqa: E731
+    assert code.tc_quotients(dp(x), dp(d), n) == 0
