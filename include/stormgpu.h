@@ -389,6 +389,9 @@ int sg_divergence_max_static(int device, const float* u, const float* v, const f
 int sg_debug_step_part(sg_context* ctx, sg_run run, int part);
 int sg_debug_read_set(sg_context* ctx, sg_run run, int set, int field, float* host);
 int sg_debug_read_faces(sg_context* ctx, sg_run run, float* faces4);
+/* The solve the last sg_masked_project took (route: 0 none, 1 the fast one, 2 the one in a fixed order of operations), and
+ * the one its next calls take (force: 0 as the residuals say, 1 or 2 that solve, -1 as before). */
+int sg_debug_masked_route(sg_masked* m, int force, int32_t* route);
 
 /* ---- serving: a request loop with HBM-budget admission, device-resident runs and mid-batch retirement ---- */
 typedef struct sg_server sg_server;

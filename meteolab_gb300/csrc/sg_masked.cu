@@ -156,8 +156,10 @@ void slope_area(const HostGrid& g, const float* h, float* area) {
 // 2 a zero right-hand side (nothing to project), 4 the residuals have lost their orthogonality (see k_mp_xinv).
 struct MpState {
   double bb, tol2bb, rz, rr, rz0, alpha, beta, tolerance;
+  double watch;  // the square of what r . z0 may grow to, of r.z r0.z0
   int k, done, maxIt, keepRR;
 };
+constexpr double WATCH_LIMIT = 1e-18;
 enum { STOP = 1, ZERO = 2, DRIFT = 4, ANY = 7 };
 enum { R_BB, R_RR0, R_RZ0, R_DSD, R_RR, R_RZN };
 
@@ -258,7 +260,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ part
   } else {
     st->beta = s / st->rz; st->rz = s; st->k++;
     if (st->k >= st->maxIt) st->done = STOP;
-    if (WATCH && s0 * s0 > 1e-18 * st->rz0 * fmax(s, 1e-10 * st->rz0)) st->done = DRIFT;
+    if (WATCH && s0 * s0 > st->watch * st->rz0 * fmax(s, 1e-10 * st->rz0)) st->done = DRIFT;
   }
 }
 
@@ -427,13 +429,14 @@ __global__ void k_mp_update_xfwd(double* __restrict__ q, double* __restrict__ r,
 // The preconditioner's x inverse: z = the plain solution (the face solve's), or with dzs V phi, zero in the dropped cells
 // (:355), and the sum r . z (OP: what it is for).
 //
-// WATCH: with r . z0, z0 the first z, which conjugate gradients keep at zero. Rounding makes it grow (over steep ground,
-// where a column's open shares are small, by a factor of ten in some iterations), and what it has grown to says how far
-// rounding has come to decide the iterations (Paige 1976): over 220 solves on drawn grounds and grids, disturbed in the
-// last bit, those with |r . z0| below 1e-9 of sqrt(r.z r0.z0) throughout agreed to 6e-13, of the others nine in ten to no
-// better than 1e-10 and half to no better than 1e-6. A solve that passes 1e-9 (or 1e-14 r0.z0, which r.z alone would be
-// compared with at tighter tolerances) stops, and starts again in one fixed order of operations (OrderedSolve).
-// An iteration there takes 0.39 ms on 80 x 64 x 50 nodes, 0.11 here; what is given up took a quarter of the iterations.
+// WATCH: with r . z0, z0 the first z, which conjugate gradients keep at zero. Rounding makes it grow (over ground that
+// leaves a column a small open share of a layer, by a factor of ten in some iterations), and what it has grown to says how
+// far rounding has come to decide the iterations (Paige 1976). Over 220 solves on drawn grounds and grids, again with a
+// first guess of 1e-16 of the pressure: the 120 with |r . z0| below 1e-9 of sqrt(r.z r0.z0) throughout agreed to 3e-10, half
+// of them to 1e-14, and as well with the ordered solve; of the 100 others nine in ten agreed to no better than 9e-10, half to
+// no better than 1e-7, the worst to 5e-3 (profiles/masked_projection_routes.md). A solve that passes 1e-9 (or 1e-14 r0.z0, which
+// r.z alone would be compared with at tighter tolerances) stops, and starts again in one fixed order of operations
+// (OrderedSolve). An iteration there takes 0.39 ms on 80 x 64 x 50 nodes, 0.13 here.
 template <int OP, bool WATCH = false>
 __global__ void k_mp_xinv(const double2* __restrict__ S, double* __restrict__ out, const double* __restrict__ r, int nx, int ny, int pairs, Fft64 P,
                           const double2* __restrict__ tw, const double* __restrict__ dzs, const uint8_t* __restrict__ dropped,
@@ -662,6 +665,7 @@ struct sg_masked {
   MpState* st = nullptr;
   std::vector<uint8_t> dropped;
   cudaGraphExec_t chunk = nullptr, orderedChunk = nullptr;
+  int force = 0, route = 0;  // sg_debug_masked_route
   int iterations = 0;
   double residual = 0;
 };
@@ -998,7 +1002,7 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
     if ((e = cudaMemcpyAsync(dev[f], host[f], n * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail(m, "copy in", e);
   if ((e = cudaMemcpyAsync(m->p, pressure, cells * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail(m, "copy in", e);
   k_mp_mask<<<nb, TPB, 0, s>>>(m->u, m->v, m->w, g);
-  m->iterations = 0; m->residual = 0;
+  m->iterations = 0; m->residual = 0; m->route = 0;
   if (!m->any) {
     // No terrain at all: the flat projection exactly (:336-339); the pressure is the flat solve's, not a first guess.
     k_mp_flat_div<<<cb, TPB, 0, s>>>(m->u, m->v, m->w, m->b, dt, g);
@@ -1006,7 +1010,7 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
     k_mp_flat_correct<<<nb, TPB, 0, s>>>(m->p, m->u, m->v, m->w, dt, g);
   } else {
     MpState init{};
-    init.tolerance = m->tolerance; init.maxIt = m->maxIt;
+    init.tolerance = m->tolerance; init.maxIt = m->maxIt; init.watch = m->force == 1 ? INFINITY : WATCH_LIMIT;
     if ((e = cudaMemcpyAsync(m->st, &init, sizeof(MpState), cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail(m, "state", e);
     if ((e = cudaMemsetAsync(m->d[0], 0, cells * 8, s)) != cudaSuccess) return fail(m, "direction", e);  // (the first direction: z + 0 d)
     // b = D R M u*, bb; q from the first guess, r = -b - S q and its first test, z = P S0^-1 P r, rz (:306-312).
@@ -1030,14 +1034,15 @@ int sg_masked_project(sg_masked* m, float* u, float* v, float* w, double dt, dou
       if (e != cudaSuccess) { m->chunk = nullptr; return fail(m, "graph", e); }
     }
     // Every iteration either counts or stops, so maxIt / REPLAY + 1 replays always reach the stop.
-    int done = 0;
-    for (int c = 0;; c++) {
+    int done = m->force == 2 ? DRIFT : 0;
+    for (int c = 0; !done; c++) {
       if ((e = cudaMemcpyAsync(&done, &m->st->done, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return fail(m, "solve", e);
       if (done || c > m->maxIt / REPLAY + 1) break;
       if ((e = cudaGraphLaunch(m->chunk, s)) != cudaSuccess) return fail(m, "graph launch", e);
     }
     if (!done) return sg_context_fail(m->ctx, SG_ERR_DEVICE, "masked projection: the iterations did not stop");
+    m->route = done == DRIFT ? 2 : done == ZERO ? 0 : 1;
     if (done == DRIFT) {
       // The winds and the first guess are still as they were.
       OrderedState fin{};
@@ -1064,6 +1069,13 @@ int sg_masked_stats(sg_masked* m, int32_t* iterations, double* residual) {
   if (!m) return SG_ERR_INVALID;
   if (iterations) *iterations = m->iterations;
   if (residual) *residual = m->residual;
+  return SG_OK;
+}
+
+int sg_debug_masked_route(sg_masked* m, int force, int32_t* route) {
+  if (!m || force < -1 || force > 2) return SG_ERR_INVALID;
+  if (route) *route = m->route;
+  if (force >= 0) m->force = force;
   return SG_OK;
 }
 

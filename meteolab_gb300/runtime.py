@@ -142,6 +142,7 @@ def load():
             L.sg_masked_stats.argtypes = [vp, C.POINTER(C.c_int32), C.POINTER(C.c_double)]
             L.sg_masked_dropped.argtypes = [vp, _U8]
             L.sg_masked_destroy.argtypes = [vp]
+            L.sg_debug_masked_route.argtypes = [vp, i32, C.POINTER(C.c_int32)]
             _D = C.POINTER(C.c_double)
             L.sg_faces_create.argtypes = [vp, C.POINTER(SgGrid), _D, _FP, C.c_double, i32, C.POINTER(vp)]
             L.sg_faces_set_velocity.argtypes = [vp, _FP, _FP, _FP, _D, _D, _D, _D]
@@ -802,6 +803,13 @@ class MaskedProjection:
         r = C.c_double()
         load().sg_masked_stats(self.h, None, C.byref(r))
         return float(r.value)
+
+    def debug_route(self, force: int = -1) -> int:
+        """The solve the last projection took (1 fast, 2 in a fixed order of operations, 0 none); `force` picks the next
+        ones' (0: as the residuals say)."""
+        route = C.c_int32()
+        self.ctx.check(load().sg_debug_masked_route(self.h, force, C.byref(route)), "masked projection's route")
+        return int(route.value)
 
     @property
     def dropped(self) -> np.ndarray:
