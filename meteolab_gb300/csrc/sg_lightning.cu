@@ -92,8 +92,7 @@ __global__ void k_lgt_rho(const RunDesc R, const LgtDev L) {
   L.rho[i] = dmul(s, lt(L, LT_AIR, i / R.layer));
 }
 // strongest() (:233-246): |E|^2 / Einit^2 of the interior nodes not failed at this step; the largest, first in node order.
-// Each block's best goes to the partials (the conduction's memory, free then), the block that ends last takes the best of
-// those. Multiplying by the levels' reciprocals instead of dividing, and one pass instead of a second one for the node,
+// Each block's best goes to the partials, the block that ends last takes the best of those. Multiplying by the levels' reciprocals instead of dividing, and one pass instead of a second one for the node,
 // took a search of the standard grid from 53 to 8 us.
 SG_D double fieldRatio2(const RunDesc& R, const LgtDev& L, int i) {
   const int nx = R.nx, ny = R.ny, layer = R.layer, z = i / layer, y = (i - z * layer) / nx, x = i - z * layer - y * nx, row = y * nx + z * layer;
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(256) k_lgt_strongest(const RunDesc R, const Lg
   }
   v = blockBest(v);
   unsigned long long* pb = reinterpret_cast<unsigned long long*>(L.part);
-  int* pi = reinterpret_cast<int*>(L.sigma);
+  int* pi = L.partAt;
   if (threadIdx.x == 0) { pb[blockIdx.x] = v.bits; pi[blockIdx.x] = v.at; }
   if (!lastBlock(&L.st->arrived)) return;
   v = Best{0, INT_MAX};
@@ -581,8 +580,8 @@ inline int blocks(int n, int t) { return (n + t - 1) / t; }
 size_t lightning_bytes(int nx, int ny, int nz) {
   const size_t n = (size_t)nx * ny * nz, mh = nx / 2, spec = (size_t)(nz - 2) * (mh + 1) * ny;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  return al(sizeof(LgtState)) + 5 * al(n * 8) + al(n * 4) + 7 * al(n * 4) + 4 * al((size_t)MAX_CHANNEL * 8) +
-         al((size_t)LT_COUNT * nz * 8) + al(((n + 255) / 256 + 1) * 8) + al(spec * 16) + 3 * al(spec * 8) +
+  return al(sizeof(LgtState)) + 4 * al(n * 8) + al(n * 4) + 7 * al(n * 4) + 4 * al((size_t)MAX_CHANNEL * 8) +
+         al((size_t)LT_COUNT * nz * 8) + al(((n + 255) / 256 + 1) * 8) + al(((n + 255) / 256 + 1) * 4) + al(spec * 16) + 3 * al(spec * 8) +
          al((size_t)nx * 16) + al((size_t)ny * 16);
 }
 
@@ -594,7 +593,7 @@ void lightning_bind(char* base, int nx, int ny, int nz, LgtHost& H) {
   auto take = [&](size_t b) { char* p = base + o; o += al(b); return p; };
   L.nz = nz;
   L.st = (LgtState*)take(sizeof(LgtState));
-  L.rho = (double*)take(n * 8); L.phi = (double*)take(n * 8); L.sigma = (double*)take(n * 8);
+  L.rho = (double*)take(n * 8); L.phi = (double*)take(n * 8);
   L.weight = (double*)take(n * 8); L.scale = (double*)take(n * 8);
   L.cloudy = (float*)take(n * 4);
   L.pos = (int*)take(n * 4); L.tag = (unsigned*)take(n * 4);
@@ -602,7 +601,7 @@ void lightning_bind(char* base, int nx, int ny, int nz, LgtHost& H) {
   L.nodes = (int*)take(MAX_CHANNEL * 8); L.parent = (int*)take(MAX_CHANNEL * 8); L.polarity = (int*)take(MAX_CHANNEL * 8);
   L.dep = (double*)take(MAX_CHANNEL * 8);
   L.lv = (double*)take((size_t)LT_COUNT * nz * 8);
-  L.part = (double*)take(((n + 255) / 256 + 1) * 8);
+  L.part = (double*)take(((n + 255) / 256 + 1) * 8); L.partAt = (int*)take(((n + 255) / 256 + 1) * 4);
   H.es.shape(nx, ny, nz - 2);
   H.es.S = (double2*)take(spec * 16);
   H.es.a = (double*)take(spec * 8); H.es.b = (double*)take(spec * 8); H.es.c = (double*)take(spec * 8);
@@ -619,14 +618,12 @@ int lightning_init(cudaStream_t st, const sg_grid* g, const double* rho, LgtHost
   const double dx = g->dx, dy = g->dy;
   for (int z = 0; z < nz; z++) {
     const double h = g->hz[z], e = E_INIT * rho[z] / RHO_STANDARD, Lc = std::cbrt(dx * dy * h);
-    T(LT_EINIT, z, e); T(LT_EINIT2, z, std::pow(e, 2)); T(LT_AIR, z, rho[z]); T(LT_ZS, z, g->zs[z]);
+    T(LT_AIR, z, rho[z]); T(LT_ZS, z, g->zs[z]);
     T(LT_CAP, z, SHIELDING * 2 * 3.14159265358979323846 * EPS0 * Lc / std::log(Lc / CHANNEL_RADIUS));        // :179
-    T(LT_VOLUME, z, dx * dy * h); T(LT_NODEAIR, z, rho[z] * dx * dy * h); T(LT_PERKG, z, 1 / (rho[z] * dx * dy * h));
-    T(LT_SIGMA, z, SIGMA_GROUND * std::exp(g->zs[z] / SIGMA_SCALE));
+    T(LT_NODEAIR, z, rho[z] * dx * dy * h); T(LT_PERKG, z, 1 / (rho[z] * dx * dy * h));
     T(LT_DZS, z, z < nz - 1 ? g->dzs[z] : 0);
-    T(LT_SPAN, z, z > 0 && z < nz - 1 ? g->zs[z + 1] - g->zs[z - 1] : 1);
     T(LT_HZ, z, h);
-    T(LT_ISPAN, z, 1 / lv[(size_t)LT_SPAN * nz + z]); T(LT_IEINIT2, z, 1 / lv[(size_t)LT_EINIT2 * nz + z]);
+    T(LT_ISPAN, z, z > 0 && z < nz - 1 ? 1 / (g->zs[z + 1] - g->zs[z - 1]) : 1); T(LT_IEINIT2, z, 1 / std::pow(e, 2));
     // conductances in series between nodes of clear air or cloud, in the level (clear-clear, clear-cloud, cloud-cloud) and
     // to the next level (bit 1 cloud below, bit 2 cloud above)
     auto series = [](double a, double b) { return 2 * a * b / (a + b); };

@@ -17,14 +17,12 @@ inline int flash_limit(double dt) {                               // flashLimit 
   return v < 1 ? 1 : (int)v;
 }
 
-// Per-level FP64 tables of the lightning (each the reference's expression): the breakdown field and its square, the air
-// density, the height, a channel node's capacitance, the cell's volume and air mass and its inverse, the clear air's
-// conductivity, the level spacing, the centred span zs[z+1] - zs[z-1], the conduction's face factors for dt, the
-// reciprocals of the span and of Einit^2, the faces' conductances by cloud, and the channel links' reaches and their
-// reciprocals (lightning_init).
-enum LgtTable { LT_EINIT, LT_EINIT2, LT_AIR, LT_ZS, LT_CAP, LT_VOLUME, LT_NODEAIR, LT_PERKG, LT_SIGMA, LT_DZS, LT_SPAN, LT_HZ,
-                LT_ACROSS, LT_ALONG, LT_UP, LT_ISPAN, LT_IEINIT2, LT_FLAT, LT_STEP = LT_FLAT + 3, LT_REACH = LT_STEP + 4,
-                LT_IREACH = LT_REACH + 12, LT_COUNT = LT_IREACH + 12 };
+// Per-level FP64 tables of the lightning (each the reference's expression): the air density, the height, a channel node's
+// capacitance, the cell's air mass and its inverse, the level spacing and the volume's height, the conduction's face factors
+// for dt, the reciprocals of the centred span zs[z+1] - zs[z-1] and of the breakdown field's square, the faces' conductances
+// by cloud, and the channel links' reaches and their reciprocals (lightning_init).
+enum LgtTable { LT_AIR, LT_ZS, LT_CAP, LT_NODEAIR, LT_PERKG, LT_DZS, LT_HZ, LT_ACROSS, LT_ALONG, LT_UP, LT_ISPAN, LT_IEINIT2, LT_FLAT,
+                LT_STEP = LT_FLAT + 3, LT_REACH = LT_STEP + 4, LT_IREACH = LT_REACH + 12, LT_COUNT = LT_IREACH + 12 };
 
 // The state a flash's kernels share (device memory; read by the host after each stage).
 struct LgtState {
@@ -41,10 +39,10 @@ struct LgtDev {
   int nz = 0;
   double dx = 0, dy = 0, i2dx = 0, i2dy = 0;
   LgtState* st = nullptr;
-  double *rho = nullptr, *phi = nullptr, *sigma = nullptr, *weight = nullptr, *scale = nullptr, *dep = nullptr, *lv = nullptr, *part = nullptr;
+  double *rho = nullptr, *phi = nullptr, *weight = nullptr, *scale = nullptr, *dep = nullptr, *lv = nullptr, *part = nullptr;
   float* cloudy = nullptr;
   int *mark = nullptr, *seen = nullptr, *link = nullptr, *failed = nullptr, *frontier = nullptr, *nodes = nullptr, *parent = nullptr, *polarity = nullptr,
-      *pos = nullptr;
+      *pos = nullptr, *partAt = nullptr;  // part, partAt: a launch's block results
   unsigned* tag = nullptr;
 };
 
