@@ -53,6 +53,12 @@ SG_D bool below(double v, double bound) { return (bitsOf(v) & 0x7fffffffffffffff
 SG_D bool isZero(double v) { return (bitsOf(v) << 1) == 0; }
 SG_D bool sameSign(double a, double b) { return (bitsOf(a) ^ bitsOf(b)) >= 0; }
 SG_D bool cloudAt(float c) { return c > (float)CLOUDY; }
+// sum / count to the last bit, from 1 / count correctly rounded: the product and one remainder (Markstein, IBM J. Res.
+// Dev. 34, 1990); an FP64 divide's latency is that of 8.6 FMAs, this three.
+SG_D double meanOf(double sum, double count, double icount) {
+  const double m = dmul(sum, icount);
+  return fma(fma(-m, count, sum), icount, m);
+}
 SG_D bool clearOf(double rho, float cloudy) { return below(rho, RHO_MIN) || !cloudAt(cloudy); }  // :343
 
 // Block sum in a fixed order (warps by halves, then the warps), valid in every thread of warp 0; all threads call it.
@@ -215,9 +221,8 @@ SG_D void addNodeWarp(const RunDesc& R, const LgtDev& L, const Front& F, volatil
     L.mark[j] = id; L.nodes[nn] = j; L.parent[nn] = from; V.nnodes = nn + 1;
     if (j < layer) { V.ground = j; V.before = V.potential; V.potential = 0; V.touched = 1; }
     else if (V.ground < 0) {
-      // sum / count, by the correctly rounded reciprocal and one residual step (the divide takes nine times an FMA)
-      const double sum = dadd(V.sum, pj), m = dmul(sum, icount);
-      V.sum = sum; V.potential = fma(fma(-m, count, sum), icount, m);
+      const double sum = dadd(V.sum, pj);
+      V.sum = sum; V.potential = meanOf(sum, count, icount);
     }
   }
   bool fresh = false;
@@ -254,9 +259,10 @@ SG_D void addNodeWarp(const RunDesc& R, const LgtDev& L, const Front& F, volatil
 // A pick: every thread weights a contiguous part of the front (an odd number of links: no bank conflicts); the warps'
 // sums; one random number; the warp that holds the first position where the pick less the weights before it is no longer
 // positive finds it by two scans, removes the link from the front, prunes the clear-air leader's other links (the
-// reference's swap-with-last order) and adds the node; two barriers a node. One block on one SM, bound by its FP64
-// instructions (64 cycles each on a quarter of the SM): three a link and three links a thread at a front of 300, where the
-// weights with their divides took thirty. 8.4 us a node on a front of 400 links before, 3.6 now.
+// reference's swap-with-last order) and adds the node; two barriers a node. One block on one SM, 3.6 us a node on a front
+// of 400 links, bound by the latency of that chain: its FP64 instructions (64 cycles each on a quarter of the SM; three a
+// link and three links a thread at a front of 300) are about a tenth of it, the rest the scans, the pick, the candidates'
+// loads and the barriers.
 __global__ void __launch_bounds__(GROW_THREADS) k_lgt_grow(const RunDesc R, const LgtDev L, int id, int start) {
   extern __shared__ double fsm[];
   constexpr int W = GROW_THREADS / 32;

@@ -1,6 +1,6 @@
 // See sg_masked_ordered.cuh. One iteration is nine launches: the gradient over the node masses and its column fluxes, their
 // divergence with d.Sd, the q/r update with r.r, five of the preconditioner (x and y sums, sweeps, y and x sums with r.z),
-// the new direction. The FP64 pipe bounds it (two operations a clock and SM, a divide some ten of them): the direct sums
+// the new direction. The FP64 pipe bounds it (two operations a clock and SM, a divide costs seven): the direct sums
 // are 770 operations a cell at 127 x 113, 460 at 80 x 64, and are left as they are; what touches no rounding is taken out.
 // A cell's V phi, a node's gradient and a column's fluxes are formed once instead of by every neighbour, divides by dx, dy,
 // the spacings and the pivots are quotients from their reciprocals, and the sums fill their warps over several rows or
@@ -19,8 +19,8 @@ constexpr int TPB = 256, REPLAY_ORDERED = 8;
 using Geo = OrderedSolve;
 
 // x / d to the last bit, from r = 1 / d correctly rounded: x r is within 1.5 units, the first remainder brings it within
-// one, the second gives the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990). Five FP64 operations against a
-// divide's ten; finite operands away from underflow, or a zero, whose sign the remainders would lose.
+// one, the second gives the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990). Five FP64 operations where a divide
+// costs seven; finite operands away from underflow, or a zero, whose sign the remainders would lose.
 __device__ __forceinline__ double quotient(double x, double d, double r) {
   const double q0 = __dmul_rn(x, r), q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0), q2 = __fma_rn(__fma_rn(-q1, d, x), r, q1);
   return (__double_as_longlong(x) << 1) == 0 ? q0 : q2;

@@ -4,7 +4,7 @@
 // complex transform), y forward, one tridiagonal sweep per mode along k, y inverse, x inverse.
 //
 // GB300 issues two FP64 operations a clock and SM (one per FP64 instruction and cell costs 0.4 us on 250,000 cells over
-// the whole chip, and a divide is some twenty of them), so the count of FP64 instructions bounds every kernel here, not
+// the whole chip, and a divide costs seven of them), so the count of FP64 instructions bounds every kernel here, not
 // memory and not index arithmetic: mixed-radix transforms (the direct sums they replace took 80 to 130 multiply-adds a
 // value, these 20 to 30), no divides, the normalisation and the pairing's factor 1/2 folded into the sweep's
 // coefficients, and work split finely enough to reach all 152 SMs. An 80 x 64 x 49 solve took 0.42 ms by direct sums.

@@ -58,3 +58,13 @@ extern "C" int lb_flash(int nx, int ny, int nz, double dx, double dy, const doub
   std::copy(v, v + 7, state);
   return largest;
 }
+
+// how many of sum[i] / (i % MAX_CHANNEL + 1) the mean from the count's reciprocal does not give to the last bit
+extern "C" int lb_means(const double* sum, int n) {
+  int wrong = 0;
+  for (int i = 0; i < n; i++) {
+    const double count = i % MAX_CHANNEL + 1;
+    wrong += emu::bits(meanOf(sum[i], count, 1.0 / count)) != emu::bits(sum[i] / count);
+  }
+  return wrong;
+}

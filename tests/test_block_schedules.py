@@ -127,3 +127,16 @@ def test_a_front_longer_than_shared_memory_grows_the_same_channel(growth, tmp_pa
         for order in (0, 1, 3):
             got = _flash(lib, seed, order)
             assert got[0] == largest and np.array_equal(got[1], nodes) and np.array_equal(got[2], state), (seed, order)
+
+
+def test_the_mean_potential_is_the_division_to_the_last_bit(growth):
+    """Sums of any size over every count a channel may have, and sums next to those whose means are next to a midpoint."""
+    rng = np.random.default_rng(5)
+    n = 900 * MAX_CHANNEL
+    sums = rng.standard_normal(n) * 10.0 ** rng.uniform(-30, 30, n)
+    count = np.arange(n) % MAX_CHANNEL + 1
+    half = n // 2
+    mean = np.ldexp(np.round(np.ldexp(rng.uniform(1, 2, half), 52)) + .5, -52 + rng.integers(-40, 40, half))
+    sums[:half] = np.nextafter(mean * count[:half], np.where(rng.random(half) < .5, np.inf, -np.inf))
+    growth.lb_means.argtypes = [C.POINTER(C.c_double), C.c_int]
+    assert growth.lb_means(sums.ctypes.data_as(C.POINTER(C.c_double)), n) == 0
