@@ -3,9 +3,8 @@
 // at the nodes, phi = 0 on the ground and top levels, periodic in x and y: a 2-D DFT of each interior level's right-hand
 // side, one stretched vertical tridiagonal per horizontal mode with fixed ends (Thomas, the reference's rows and
 // pivots), the inverse DFT. All in FP64: the reference's own tests hold the solution to 1e-9 of the discrete Poisson
-// equation and the plate field to 5e-7, and a solve is small (the standard grid's is 60 thousand nodes). The DFTs are
-// direct sums over exact FP64 twiddle tables, one output a thread: x (real to half-complex) per row, then y per level
-// and x-mode; the inverse in the opposite order.
+// equation and the plate field to 5e-7, and a solve is small (the standard grid's is 60 thousand nodes). Its five launches
+// are sg_spectral64's: mixed-radix transforms along x (two real rows a complex one) and y, the sweeps, y and x back.
 #include <cuda_runtime.h>
 #include <cmath>
 #include <cstring>
@@ -32,7 +31,7 @@ int sg_electric_create(sg_context* ctx, const sg_grid* g, sg_electric** out) {
     return sg_context_fail(ctx, SG_ERR_INVALID, "electric solver: a grid with nx, ny >= 1, dx, dy > 0 and its level arrays");
   if (g->nz < 3) return sg_context_fail(ctx, SG_ERR_INVALID, "the electric solver needs an interior level");
   if (g->nz - 2 > sg::ELEC_MAXNI) return sg_context_fail(ctx, SG_ERR_INVALID, "electric solver: at most 130 levels");
-  // (a row, a column and a half spectrum in shared memory: at most 32 KB)
+  // (the transforms' pairs of rows and columns in shared memory: at most 64 KB)
   if (g->nx > 2048 || g->ny > 2048) return sg_context_fail(ctx, SG_ERR_INVALID, "electric solver: nx and ny at most 2048");
   const int nx = g->nx, ny = g->ny, nz = g->nz;
   for (int k = 0; k < nz; k++)

@@ -89,7 +89,7 @@ void lightning_bind(char* base, int nx, int ny, int nz, LgtHost& H);
 int lightning_init(cudaStream_t st, const sg_grid* g, const double* rho, LgtHost& H);
 // The run's lightning stream and pinned host buffers (once).
 int lightning_host_buffers(LgtHost& H);
-// The discharges of n runs together (lockstep rounds, a stream a run); each job's time is its flashes' model time.
+// The discharges of n runs together (a stream a run, each run's next piece when its last has ended); each job's time is its flashes' model time.
 int lightning_discharge_many(LgtJob* jobs, int n, std::string* err);
 // The discharge after a step at model time `time` (the step's end) with step length dt: at most `limit` flashes, then
 // the conduction and corona over dt, then the vertical field. SG_OK, or SG_ERR_DEVICE with *err set.

@@ -642,8 +642,8 @@ cudaError_t solve_limits() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SPECTRAL64_SMEM);
   return e;
 }
-// Layers a thread of k_mp_flux marches: two layers' work is its start, so as many as leave 152 SMs a block each of 256
-// columns, within 4..16.
+// Layers a thread of k_mp_flux marches: two layers' work is its start, so as many as leave the chip's 152 SMs four blocks
+// of 64 columns each, within 4..16.
 int flux_seg(int layer, int nc) { return std::min(16, std::max(4, (int)((size_t)layer * nc / (152 * (size_t)TPB)))); }
 
 }  // namespace
@@ -885,6 +885,8 @@ int sg_masked_create(sg_context* ctx, const sg_grid* grid, const double* rho, co
   const size_t nparts = std::max({(size_t)blocks(cells), 2 * (size_t)sp.x.groups * nc, (size_t)ny * nc});  // (two sums a group: the watch)
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += al(bytes); return o; };
+  // Some 175 bytes a node, 20 of them the ordered solve's own: its sweep's coefficients and its first spectrum (where the fast
+  // one keeps z0); the two share the rest.
   const size_t oU = take(n * 4), oV = take(n * 4), oW = take(n * 4), oP = take(cells * 8), oB = take(cells * 8), oQ = take(cells * 8), oR = take(cells * 8),
                oZ = take(cells * 8), oD = take(cells * 8), oD2 = take(cells * 8), oSd = take(cells * 8), oFu = take(n * 8), oFv = take(n * 8),
                oFw = take(n * 8), oPart = take(nparts * 8), oLo = take(spec * 8), oPv = take(spec * 8),

@@ -112,6 +112,7 @@ struct Plan {
 };
 enum Family { FAM_NODE, FAM_COLS, FAM_ROWS_FACE, FAM_ROWS_PRES, FAM_MODES, FAM_RUNS, FAM_CELLS, FAM_T_WENO, FAM_T_DYN, FAM_MIX,
               FAM_REFINE, FAM_T_CHG, FAM_T_CHG3, FAM_PHYS, FAM_PHYS_LAST = FAM_PHYS + 5, FAM_FILL, FAM_YCOLS, FAM_LROWS_FACE, FAM_LROWS_PRES, FAM_LMODES, FAM_COUNT };
+static_assert(FAM_COUNT <= sizeof(Plan::off) / sizeof(int), "an offset and a count a family");
 
 }  // namespace
 
@@ -344,11 +345,12 @@ int validate(sg_context* ctx, const sg_grid* g, const sg_base_state* b, const sg
   for (int z = 0; z < g->nz; z++) if (!(b->rho[z] > 0) || !(b->theta[z] > 0) || !(g->hz[z] > 0)) return fail(ctx, SG_ERR_INVALID, "non-positive rho, theta or hz");
   if (!(sw->dt > 0)) return fail(ctx, SG_ERR_INVALID, "dt must be positive");
   if (!sw->pressure_in_stages) return fail(ctx, SG_ERR_UNSUPPORTED, "the device step needs the pressure in the RK3 stages");
-  // the lightning's potential solve holds a row, a column and a half spectrum of a level in shared memory
+  // the lightning's potential solve holds pairs of rows and columns of a level in shared memory (64 KB at most)
   if (sw->lightning && sw->ice && (g->nx > 2048 || g->ny > 2048)) return fail(ctx, SG_ERR_UNSUPPORTED, "lightning: nx and ny at most 2048");
-  // the row path's limit on a wavenumber's slab, (nz + 8) * ny complex values
+  // The limit that grids have always been held to: a wavenumber's slab of (nz + 8) * ny complex values within a block's
+  // shared memory. (No kernel holds that slab any more; the row path's y-transforms take two buffers of about 2048 points.)
   size_t smem = (size_t)(g->nz + 8) * g->ny * 8;
-  if ((int)smem > ctx->maxSmem) return fail(ctx, SG_ERR_UNSUPPORTED, "(nz + 8) * ny too large for one block's shared memory");
+  if ((int)smem > ctx->maxSmem) return fail(ctx, SG_ERR_UNSUPPORTED, "(nz + 8) * ny too large");
   return SG_OK;
 }
 
