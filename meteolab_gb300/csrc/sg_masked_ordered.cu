@@ -20,10 +20,17 @@ using Geo = OrderedSolve;
 
 // x / d to the last bit, from r = 1 / d correctly rounded: x r is within 1.5 units, the first remainder brings it within
 // one, the second gives the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990). Five FP64 operations where a divide
-// costs seven; finite operands away from underflow, or a zero, whose sign the remainders would lose.
+// costs seven; finite operands away from underflow. The remainders are taken with the sign that leaves a zero its own: d > 0
+// (spacings) here, d < 0 (pivots) below.
 __device__ __forceinline__ double quotient(double x, double d, double r) {
-  const double q0 = __dmul_rn(x, r), q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0), q2 = __fma_rn(__fma_rn(-q1, d, x), r, q1);
-  return (__double_as_longlong(x) << 1) == 0 ? q0 : q2;
+  double q = __dmul_rn(x, r);
+  q = __fma_rn(__fma_rn(q, d, -x), -r, q);
+  return __fma_rn(__fma_rn(q, d, -x), -r, q);
+}
+__device__ __forceinline__ double quotient_negative(double x, double d, double r) {
+  double q = __dmul_rn(x, r);
+  q = __fma_rn(__fma_rn(-q, d, x), r, q);
+  return __fma_rn(__fma_rn(-q, d, x), r, q);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -300,7 +307,7 @@ __global__ void k_or_sweep(Geo g, int skip) {
 #pragma unroll
     for (int q = 0; q < AHEAD; q++)
       if (k0 + q < nc) {
-        d = make_double2(quotient(__fma_rn(-a[q], d.x, r[q].x), m[q], w[q]), quotient(__fma_rn(-a[q], d.y, r[q].y), m[q], w[q]));
+        d = make_double2(quotient_negative(__fma_rn(-a[q], d.x, r[q].x), m[q], w[q]), quotient_negative(__fma_rn(-a[q], d.y, r[q].y), m[q], w[q]));
         g.S2[(size_t)(k0 + q) * modes + mode] = d;
       }
   }

@@ -31,10 +31,11 @@ void tc_divergence(int nx, int ny, int nz, double dx, double dy, const float* u,
       });
 }
 
-// how many of x[i] / d[i] the quotient from the reciprocal does not give to the last bit
-int tc_quotients(const double* x, const double* d, int n) {
+// how many of x[i] / d[i] the quotient from the reciprocal does not give to the last bit (the one for divisors below zero
+// with `negative`)
+int tc_quotients(const double* x, const double* d, int n, int negative) {
   int wrong = 0;
-  for (int i = 0; i < n; i++) wrong += emu::bits(quotient(x[i], d[i], 1 / d[i])) != emu::bits(x[i] / d[i]);
+  for (int i = 0; i < n; i++) wrong += emu::bits((negative ? quotient_negative : quotient)(x[i], d[i], 1 / d[i])) != emu::bits(x[i] / d[i]);
   return wrong;
 }
 

@@ -66,4 +66,6 @@ def test_quotients_from_reciprocals_are_the_division_to_the_last_bit(code):
     edge = [(0., 3.), (-0., 3.), (1., 3.), (np.pi, -7.), (1., 2 - 2.0 ** -52), (2 - 2.0 ** -52, 1 + 2.0 ** -52)]
     x[-len(edge):], d[-len(edge):] = zip(*edge)
     dp = lambda a: a.ctypes.data_as(DP)  # noqa: E731
-    assert code.tc_quotients(dp(x), dp(d), n) == 0
+    assert code.tc_quotients(dp(x), dp(d), n, 0) == 0
+    d[d > 0] *= -1
+    assert code.tc_quotients(dp(x), dp(d), n, 1) == 0
