@@ -160,8 +160,8 @@ inline int node_chunk(size_t nodes, size_t sms) {
 
 SG_HD double* fill_part(const RunDesc& R) { return reinterpret_cast<double*>(R.kmkh); }
 SG_HD float lvl(const RunDesc& R, int which, int z) { return R.lv[which * R.nz + z]; }
-// Set s of the 13 base fields is fld[s * 13 n ...]; an electrified run's charge carriers follow the three sets,
-// four fields a set, so the base fields keep their offsets (and the hot kernels their constant strides).
+// Set s of the 13 base fields is fld[s * 13 n ...]; a run with extra fields has theirs after the three sets, NXE fields a set,
+// so the base fields keep their offsets (and the hot kernels their constant strides).
 SG_HD float* field(const RunDesc& R, int set, int f) {
   return f < NF ? R.fld + ((size_t)set * NF + f) * R.n : R.fld + ((size_t)3 * NF + (size_t)set * NXE + (f - NF)) * R.n;
 }
